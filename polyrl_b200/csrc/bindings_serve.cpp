@@ -7,8 +7,8 @@
 
 extern "C" {
 int prl_gemm_bf16(const void*, const void*, void*, const void*, int, int, int, int64_t, int64_t, int64_t, int, cudaStream_t);
-int prl_sample(const void*, int, int64_t, int, int, const float*, const uint64_t*, int, int64_t*, float*, cudaStream_t);
-int prl_sample_topk_topp(const void*, int, int64_t, int, int, const float*, const uint64_t*, int, int, float, int64_t*, float*, cudaStream_t);
+int prl_sample(const void*, int, int64_t, int, int, const float*, int, const uint64_t*, int, int64_t*, float*, cudaStream_t);
+int prl_sample_topk_topp(const void*, int, int64_t, int, int, const float*, int, const uint64_t*, int, int, float, int64_t*, float*, cudaStream_t);
 int prl_attn_fwd(const void*, const void*, const void*, void*, float*, const int32_t*, const int32_t*, int, int, int, int, int, int, int, int64_t, int64_t, int64_t, int64_t, float, int, int, const float*, int, int, long long*, cudaStream_t);
 int prl_paged_decode_workspace_floats(int, int, int, int);
 int prl_paged_decode(const void*, int64_t, const void*, const void*, const int32_t*, int64_t, const int32_t*, int, int, int, int, float, int, int, int, float*, void*, int64_t, cudaStream_t);
@@ -93,8 +93,21 @@ at::Tensor gemm_bf16(const at::Tensor& a, const at::Tensor& b, const c10::option
   return d;
 }
 
-std::vector<at::Tensor> sample(const at::Tensor& logits, const c10::optional<at::Tensor>& inv_temp,
-                               const c10::optional<at::Tensor>& seeds, bool greedy) {
+// What the two samplers take per row: inverse temperatures, or temperatures as the caller holds them.
+const float* row_scales(const at::Tensor& logits, const c10::optional<at::Tensor>& t) {
+  if (!t.has_value()) return nullptr;
+  TORCH_CHECK(t->is_cuda() && t->get_device() == logits.get_device() && t->scalar_type() == at::kFloat && t->is_contiguous() && t->numel() == logits.size(0),
+              "sample: one contiguous fp32 temperature per row, on the logits' device");
+  return t->data_ptr<float>();
+}
+const uint64_t* row_seeds(const at::Tensor& logits, const c10::optional<at::Tensor>& seeds) {
+  if (!seeds.has_value()) return nullptr;
+  TORCH_CHECK(seeds->scalar_type() == at::kLong && seeds->is_cuda() && seeds->is_contiguous() && seeds->numel() >= logits.size(0), "sample: one int64 seed per row");
+  return reinterpret_cast<uint64_t*>(seeds->data_ptr<int64_t>());
+}
+
+std::vector<at::Tensor> sample(const at::Tensor& logits, const c10::optional<at::Tensor>& scales,
+                               const c10::optional<at::Tensor>& seeds, bool greedy, bool inverse) {
   TORCH_CHECK(logits.is_cuda() && logits.dim() == 2 && logits.stride(1) == 1);
   const int dt = logits.scalar_type() == at::kFloat ? 0 : 1;
   TORCH_CHECK(dt == 0 || logits.scalar_type() == at::kBFloat16);
@@ -102,16 +115,13 @@ std::vector<at::Tensor> sample(const at::Tensor& logits, const c10::optional<at:
   c10::cuda::CUDAGuard g(logits.device());
   at::Tensor tok = at::empty({B}, logits.options().dtype(at::kLong));
   at::Tensor lp = at::empty({B}, logits.options().dtype(at::kFloat));
-  const uint64_t* sd = nullptr;
-  if (seeds.has_value()) { TORCH_CHECK(seeds->scalar_type() == at::kLong); sd = reinterpret_cast<const uint64_t*>(seeds->data_ptr<int64_t>()); }
-  check(prl_sample(logits.data_ptr(), dt, logits.stride(0), B, V,
-                   inv_temp.has_value() ? inv_temp->data_ptr<float>() : nullptr, sd, greedy ? 1 : 0,
+  check(prl_sample(logits.data_ptr(), dt, logits.stride(0), B, V, row_scales(logits, scales), inverse ? 1 : 0, row_seeds(logits, seeds), greedy ? 1 : 0,
                    tok.data_ptr<int64_t>(), lp.data_ptr<float>(), cur_stream()), "sample");
   return {tok, lp};
 }
 
-std::vector<at::Tensor> sample_topk_topp(const at::Tensor& logits, const c10::optional<at::Tensor>& inv_temp,
-                                         const c10::optional<at::Tensor>& seeds, bool greedy, int64_t top_k, double top_p) {
+std::vector<at::Tensor> sample_topk_topp(const at::Tensor& logits, const c10::optional<at::Tensor>& scales,
+                                         const c10::optional<at::Tensor>& seeds, bool greedy, int64_t top_k, double top_p, bool inverse) {
   TORCH_CHECK(logits.is_cuda() && logits.dim() == 2 && logits.stride(1) == 1);
   const int dt = logits.scalar_type() == at::kFloat ? 0 : 1;
   TORCH_CHECK(dt == 0 || logits.scalar_type() == at::kBFloat16);
@@ -119,11 +129,8 @@ std::vector<at::Tensor> sample_topk_topp(const at::Tensor& logits, const c10::op
   c10::cuda::CUDAGuard g(logits.device());
   at::Tensor tok = at::empty({B}, logits.options().dtype(at::kLong));
   at::Tensor lp = at::empty({B}, logits.options().dtype(at::kFloat));
-  const uint64_t* sd = nullptr;
-  if (seeds.has_value()) { TORCH_CHECK(seeds->scalar_type() == at::kLong); sd = reinterpret_cast<const uint64_t*>(seeds->data_ptr<int64_t>()); }
-  check(prl_sample_topk_topp(logits.data_ptr(), dt, logits.stride(0), B, V,
-                             inv_temp.has_value() ? inv_temp->data_ptr<float>() : nullptr, sd, greedy ? 1 : 0,
-                             static_cast<int>(top_k), static_cast<float>(top_p), tok.data_ptr<int64_t>(), lp.data_ptr<float>(),
+  check(prl_sample_topk_topp(logits.data_ptr(), dt, logits.stride(0), B, V, row_scales(logits, scales), inverse ? 1 : 0, row_seeds(logits, seeds),
+                             greedy ? 1 : 0, static_cast<int>(top_k), static_cast<float>(top_p), tok.data_ptr<int64_t>(), lp.data_ptr<float>(),
                              cur_stream()), "sample_topk_topp");
   return {tok, lp};
 }
@@ -1024,8 +1031,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("paged_decode", &paged_decode, py::arg("q"), py::arg("k_cache"), py::arg("v_cache"), py::arg("block_table"),
         py::arg("seq_lens"), py::arg("nq"), py::arg("nkv"), py::arg("d"), py::arg("sm_scale"), py::arg("splits") = 1,
         py::arg("out") = py::none(), py::arg("window") = 0, py::arg("keep_first") = 0);
-  m.def("sample", &sample);
-  m.def("sample_topk_topp", &sample_topk_topp);
+  m.def("sample", &sample, py::arg("logits"), py::arg("scales"), py::arg("seeds"), py::arg("greedy"), py::arg("inverse") = true);
+  m.def("sample_topk_topp", &sample_topk_topp, py::arg("logits"), py::arg("scales"), py::arg("seeds"), py::arg("greedy"), py::arg("top_k"), py::arg("top_p"),
+        py::arg("inverse") = true);
   m.def("mix_embed", &mix_embed);
   m.def("mix_norm_add_", &mix_norm_add_);
   m.def("mix_rms", &mix_rms);

@@ -1,307 +1,489 @@
-// polyrl_b200 — token sampling for the rollout engine: temperature + Gumbel-max categorical sampling
-// (exact for top_k=-1/top_p=1, the GRPO default) or greedy, returning the token id AND its
-// log-probability under the temperature-scaled softmax in a single pass over the logits row.
+// polyrl_b200 — token sampling for the rollout engine: temperature + Gumbel-max categorical sampling (exact for top_k=-1 / top_p=1, the
+// GRPO default), top-k / top-p, or greedy, returning the token id AND its log-probability under the distribution that was sampled.
 //
 // Reference capability: SGLang sampler + `return_logprob` (meta_info.output_token_logprobs consumed at
 // rlboost/verl_stream/workers/rollout/sglang_rollout/sglang_rollout_remote.py:318-391).
+//
+// A row belongs to a cluster of 1 to 8 CTAs of 256 threads: as many as keep all rows' CTAs resident at once (row_ctas below).  Rows start
+// at any element; the 16-byte granules that lie inside a row are loaded whole, its two ends element by element.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace prl {
+
+namespace cg = cooperative_groups;
+
+constexpr int kSampleCtas = 8;        // most CTAs per row (cluster)
+constexpr int kSampleThreads = 256;
+constexpr int kSampleWarps = kSampleThreads / 32;
+constexpr float kLog2E = 1.4426950408889634f;
 
 __device__ __forceinline__ uint32_t hash_u32(uint32_t x) {
   x ^= x >> 16; x *= 0x7feb352dU; x ^= x >> 15; x *= 0x846ca68bU; x ^= x >> 16;
   return x;
 }
-__device__ __forceinline__ float gumbel_noise(uint64_t seed, uint32_t row, uint32_t col) {
-  uint32_t h = hash_u32(static_cast<uint32_t>(seed) ^ hash_u32(col + 0x9e3779b9U * (row + 1)));
-  h = hash_u32(h ^ static_cast<uint32_t>(seed >> 32));
-  const float u = (static_cast<float>(h >> 8) + 0.5f) * (1.0f / 16777216.0f);   // (0,1)
+// 32 hashed bits of an element before the mixer's last step (which leaves the upper half as it is), and the Gumbel noise of 24 of them
+__device__ __forceinline__ uint32_t noise_hash(uint64_t seed, uint32_t row, uint32_t col) {
+  const uint32_t h = hash_u32(static_cast<uint32_t>(seed) ^ hash_u32(col + 0x9e3779b9U * (row + 1)));
+  uint32_t x = h ^ static_cast<uint32_t>(seed >> 32);
+  x ^= x >> 16; x *= 0x7feb352dU; x ^= x >> 15; x *= 0x846ca68bU;
+  return x;
+}
+__device__ __forceinline__ float gumbel_of(uint32_t x) {
+  const float u = (static_cast<float>((x ^ (x >> 16)) >> 8) + 0.5f) * (1.0f / 16777216.0f);
   return -__logf(-__logf(u));
 }
-
-struct SampleState {
-  float best;      // max of z + gumbel
-  int best_idx;
-  float best_z;
-  float m;         // running max of z
-  float s;         // running sum exp(z - m)
-};
-__device__ __forceinline__ void merge(SampleState& a, const SampleState& b) {
-  if (b.best > a.best || (b.best == a.best && b.best_idx < a.best_idx)) {
-    a.best = b.best; a.best_idx = b.best_idx; a.best_z = b.best_z;
-  }
-  const float nm = fmaxf(a.m, b.m);
-  if (nm == -INFINITY) return;
-  a.s = a.s * __expf(a.m - nm) + b.s * __expf(b.m - nm);
-  a.m = nm;
+// Hashes below this give noise that is certainly less than `need`.  The 24 bits must reach 2^24 exp(-exp(-need)), less a margin of 256
+// for the errors of the four fast functions (log near 1 is 6 units off at most, the rest under 40); the hash's upper 16 bits decide.
+// A `need` of -inf or NaN lets every element pass.
+__device__ __forceinline__ uint32_t least_hash(float need) {
+  const int bits = static_cast<int>(__expf(-__expf(-need)) * 16777216.0f) - 256;
+  return bits > 0 ? static_cast<uint32_t>(bits) << 8 & 0xffff0000u : 0u;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(1024)
-sample_kernel(const T* __restrict__ logits, int64_t ld, int V, const float* __restrict__ inv_temp,
-              const uint64_t* __restrict__ seeds, int greedy_all, int64_t* __restrict__ out_tok,
-              float* __restrict__ out_lp) {
-  const int row = blockIdx.x;
-  const T* lr = logits + static_cast<int64_t>(row) * ld;
-  const float it = inv_temp ? inv_temp[row] : 1.f;
-  const bool greedy = greedy_all || it <= 0.f;
-  const float scale = greedy ? 1.f : it;
-  const uint64_t seed = seeds ? seeds[row] : 0;
-  SampleState st{-INFINITY, 0x7fffffff, 0.f, -INFINITY, 0.f};
-  auto visit = [&](int c, float raw) {
-    const float z = raw * scale;
-    const float key = greedy ? z : z + gumbel_noise(seed, row, c);
-    if (key > st.best) { st.best = key; st.best_idx = c; st.best_z = z; }
-    const float nm = fmaxf(st.m, z);
-    st.s = st.s * __expf(st.m - nm) + __expf(z - nm);
-    st.m = nm;
-  };
-  int c0 = 0;
-  if constexpr (sizeof(T) == 2) {
-    // 128-bit vector loads (8 bf16) when the row is 16-byte aligned: 8x fewer load instructions (profile: the scalar
-    // version took 131 us per step for [128, 128256] logits)
-    if ((reinterpret_cast<uintptr_t>(lr) & 15) == 0) {
-      const int nvec = V >> 3;
-      for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
-        const int4 q = ld_nc_v4(reinterpret_cast<const __nv_bfloat16*>(lr) + 8 * v);
-        const uint32_t* u = reinterpret_cast<const uint32_t*>(&q);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 f = unpack_bf16(u[j]);
-          visit(8 * v + 2 * j, f.x);
-          visit(8 * v + 2 * j + 1, f.y);
-        }
-      }
-      c0 = nvec << 3;
-    }
-  }
-  for (int c = c0 + threadIdx.x; c < V; c += blockDim.x) visit(c, static_cast<float>(lr[c]));
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    SampleState other;
-    other.best = __shfl_xor_sync(0xffffffffu, st.best, o);
-    other.best_idx = __shfl_xor_sync(0xffffffffu, st.best_idx, o);
-    other.best_z = __shfl_xor_sync(0xffffffffu, st.best_z, o);
-    other.m = __shfl_xor_sync(0xffffffffu, st.m, o);
-    other.s = __shfl_xor_sync(0xffffffffu, st.s, o);
-    merge(st, other);
-  }
-  __shared__ SampleState red[32];
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) red[w] = st;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    SampleState t = red[0];
-    for (int i = 1; i < (blockDim.x >> 5); ++i) merge(t, red[i]);
-    out_tok[row] = t.best_idx;
-    out_lp[row] = t.best_z - (t.m + __logf(t.s));
-  }
-}
-
-// ------------------------------------------------------------------------------------------------------------------
-// top-k / top-p (nucleus) sampling, one CTA per row, no sort: the k-th largest logit and the nucleus cut are found by
-// MSB-first radix selection over order-preserving integer keys of the logits (two 8-bit passes for bf16 rows, four for
-// fp32 rows; count histograms for top-k, FIXED-POINT probability-mass histograms for top-p so that the cut is
-// independent of the order of the shared-memory atomics — tensor-parallel engine ranks must sample identically).
-// Then Gumbel-max over the kept set and the log-prob under the renormalised distribution.  HF / SGLang order:
-// temperature -> top-k -> top-p.  Replaces the eager full-vocabulary sort of round 1 (reference exposes rollout.top_k /
-// rollout.top_p: 3rdparty/verl/verl/trainer/config/rollout/rollout.yaml).
-// ------------------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t order_key(float f) {
   const uint32_t u = __float_as_uint(f);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);      // ascending float order == ascending unsigned order
 }
-
-template <typename T>
-__device__ __forceinline__ float load_logit(const T* p, int i) { return static_cast<float>(p[i]); }
-
-__device__ __forceinline__ float block_reduce_max(float v, float* red) {
-  v = warp_max(v);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) red[w] = v;
-  __syncthreads();
-  float r = red[0];
-  for (int i = 1; i < (blockDim.x >> 5); ++i) r = fmaxf(r, red[i]);
-  return r;
-}
-__device__ __forceinline__ float block_reduce_sum(float v, float* red) {
-  v = warp_sum(v);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) red[w] = v;
-  __syncthreads();
-  float r = 0.f;
-  for (int i = 0; i < (blockDim.x >> 5); ++i) r += red[i];      // fixed order: deterministic
-  return r;
+__device__ __forceinline__ float from_order_key(uint32_t k) { return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k); }
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
 }
 
+// A row in 16-byte granules; granule g holds elements [first(g), first(g) + N), those outside the row read as -inf.
 template <typename T>
-__global__ void __launch_bounds__(1024)
-sample_topk_topp_kernel(const T* __restrict__ logits, int64_t ld, int V, const float* __restrict__ inv_temp,
+struct SampleRow {
+  static constexpr int N = 16 / static_cast<int>(sizeof(T));
+  const T* p;
+  int V, skew;
+  __device__ __forceinline__ SampleRow(const T* row, int v)
+      : p(row), V(v), skew(static_cast<int>((reinterpret_cast<uintptr_t>(row) & 15) / sizeof(T))) {}
+  __device__ __forceinline__ int granules() const { return (skew + V + N - 1) / N; }
+  __device__ __forceinline__ int first(int g) const { return g * N - skew; }
+  __device__ __forceinline__ int4 load(int g) const {
+    const int e = first(g);
+    if (e >= 0 && e + N <= V) return ld_nc_v4(p + e);
+    int4 q;
+    T* t = reinterpret_cast<T*>(&q);
+#pragma unroll
+    for (int j = 0; j < N; ++j) t[j] = (e + j >= 0 && e + j < V) ? p[e + j] : static_cast<T>(-INFINITY);
+    return q;
+  }
+  static __device__ __forceinline__ void unpack(const int4& q, float (&f)[N]) {
+    if constexpr (sizeof(T) == 2) {
+      const uint32_t* u = reinterpret_cast<const uint32_t*>(&q);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 x = unpack_bf16(u[j]);
+        f[2 * j] = x.x; f[2 * j + 1] = x.y;
+      }
+    } else {
+      const float* x = reinterpret_cast<const float*>(&q);
+#pragma unroll
+      for (int j = 0; j < N; ++j) f[j] = x[j];
+    }
+  }
+};
+
+// The best noisy logit so far; the lower index wins a tie.
+struct Pick {
+  float key;
+  int idx;
+  float raw;
+  __device__ __forceinline__ void offer(float k, int i, float r) {
+    if (k > key || (k == key && i < idx)) { key = k; idx = i; raw = r; }
+  }
+};
+
+// Offers a granule's elements (those that are not wanted as -inf).  Most cannot win: the noise is a monotone function of the hash, so a
+// granule computes from the CTA's best key and its own largest logit what a winner's hash must reach, and only elements that reach it pay
+// for two logarithms.
+template <int N>
+__device__ __forceinline__ void offer_granule(Pick& best, float bar, const float (&f)[N], float fmax, int first, float scale, bool greedy,
+                                              uint64_t seed, uint32_t row) {
+  if (greedy) {
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      if (f[j] * scale > best.key) { best.key = f[j] * scale; best.idx = first + j; best.raw = f[j]; }
+    return;
+  }
+  const uint32_t least = least_hash(bar - fmax * scale);
+  uint32_t x[N];
+  bool any = false;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    x[j] = noise_hash(seed, row, first + j);
+    any |= x[j] >= least;
+  }
+  if (any) {
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      if (x[j] >= least) {
+        const float k = f[j] * scale + gumbel_of(x[j]);
+        if (k > best.key) { best.key = k; best.idx = first + j; best.raw = f[j]; }
+      }
+  }
+}
+// The CTA's best key so far (as an order key), which every warp raises; a late read only prunes less.
+__device__ __forceinline__ float raise_bar(uint32_t* bar, const Pick& best) {
+  const uint32_t k = __reduce_max_sync(0xffffffffu, order_key(best.key)), b = *const_cast<volatile uint32_t*>(bar);
+  if (k > b && (threadIdx.x & 31) == 0) atomicMax(bar, k);
+  return from_order_key(k > b ? k : b);
+}
+
+__device__ __forceinline__ Pick warp_pick(Pick p) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float k = __shfl_xor_sync(0xffffffffu, p.key, o);
+    const int i = __shfl_xor_sync(0xffffffffu, p.idx, o);
+    const float r = __shfl_xor_sync(0xffffffffu, p.raw, o);
+    p.offer(k, i, r);
+  }
+  return p;
+}
+// running maximum and sum of 2^((x - max) k2); a part that saw only -inf has the sum 0
+__device__ __forceinline__ void merge_sum(float& m, float& s, float m2, float s2, float k2) {
+  const float nm = fmaxf(m, m2);
+  if (nm == -INFINITY) return;
+  s = (m == -INFINITY ? 0.f : s * ex2((m - nm) * k2)) + (m2 == -INFINITY ? 0.f : s2 * ex2((m2 - nm) * k2));
+  m = nm;
+}
+
+__device__ __forceinline__ float scale_of(const float* temp, int row, bool inverse, bool greedy_all, bool& greedy) {
+  float it = 1.f;
+  if (temp) {
+    const float t = temp[row];
+    it = inverse ? t : (t > 0.f ? __frcp_rn(fmaxf(t, 1e-6f)) : 0.f);
+  }
+  greedy = greedy_all || it <= 0.f;
+  return greedy ? 1.f : it;
+}
+
+// One pass over the row.  Bound by integer instructions: three rounds of the hash are 24 of the 45 that an element takes, on a pipe that
+// takes a warp every other cycle (61% busy).  [128, 128256] bf16: 37 us (two logarithms for every element, one CTA per row: 47); one row
+// of 151936: 9 us (47).
+template <typename T>
+__global__ void __launch_bounds__(kSampleThreads, 4)
+sample_kernel(const T* __restrict__ logits, int64_t ld, int V, const float* __restrict__ temp, int inverse,
+              const uint64_t* __restrict__ seeds, int greedy_all, int64_t* __restrict__ out_tok, float* __restrict__ out_lp) {
+  using Row = SampleRow<T>;
+  constexpr int N = Row::N, AHEAD = 2;
+  struct Part { Pick pick; float m, s; };
+  __shared__ Part part[kSampleWarps];
+  __shared__ Part of_cta[kSampleCtas];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = static_cast<int>(cluster.block_rank()), ctas = static_cast<int>(cluster.num_blocks());
+  const int row = blockIdx.x / ctas;
+  const Row r(logits + static_cast<int64_t>(row) * ld, V);
+  bool greedy;
+  const float scale = scale_of(temp, row, inverse != 0, greedy_all != 0, greedy);
+  const float k2 = scale * kLog2E;
+  const uint64_t seed = seeds ? seeds[row] : 0;
+  __shared__ uint32_t bar;
+  if (threadIdx.x == 0) bar = order_key(-INFINITY);
+  __syncthreads();
+  Pick best{-INFINITY, 0x7fffffff, -INFINITY};
+  float bar_now = -INFINITY, m = -INFINITY, s = 0.f;
+  const int ng = r.granules();
+  const int step = ctas * static_cast<int>(blockDim.x);
+  for (int g0 = rank * static_cast<int>(blockDim.x); g0 < ng; g0 += AHEAD * step) {          // uniform in a CTA
+    int4 q[AHEAD];
+#pragma unroll
+    for (int a = 0; a < AHEAD; ++a) q[a] = r.load(min(g0 + a * step + static_cast<int>(threadIdx.x), ng));   // past the end: -inf
+#pragma unroll
+    for (int a = 0; a < AHEAD; ++a) {
+      if (g0 + a * step >= ng) break;
+      const int first = r.first(g0 + a * step + static_cast<int>(threadIdx.x));
+      float f[N];
+      Row::unpack(q[a], f);
+      float fm = f[0];
+#pragma unroll
+      for (int j = 1; j < N; ++j) fm = fmaxf(fm, f[j]);
+      if (fm > m) { s *= ex2((m - fm) * k2); m = fm; }
+      if (m > -INFINITY) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) s += ex2((f[j] - m) * k2);
+      }
+      if (!greedy && bar_now == -INFINITY) {                    // one element of each lane sets a bar for the rest
+        if (f[0] > -INFINITY) best.offer(f[0] * scale + gumbel_of(noise_hash(seed, row, first)), first, f[0]);
+        bar_now = raise_bar(&bar, best);
+      }
+      offer_granule<N>(best, bar_now, f, fm, first, scale, greedy, seed, row);
+      if (!greedy) bar_now = raise_bar(&bar, best);
+    }
+  }
+  best = warp_pick(best);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) merge_sum(m, s, __shfl_xor_sync(0xffffffffu, m, o), __shfl_xor_sync(0xffffffffu, s, o), k2);
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  if (l == 0) part[w] = Part{best, m, s};
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    Part t = part[0];
+    for (int i = 1; i < static_cast<int>(blockDim.x >> 5); ++i) {
+      t.pick.offer(part[i].pick.key, part[i].pick.idx, part[i].pick.raw);
+      merge_sum(t.m, t.s, part[i].m, part[i].s, k2);
+    }
+    *cluster.map_shared_rank(&of_cta[rank], 0) = t;
+  }
+  cluster.sync();
+  if (rank == 0 && threadIdx.x == 0) {
+    Part t = of_cta[0];
+    for (int i = 1; i < ctas; ++i) {
+      t.pick.offer(of_cta[i].pick.key, of_cta[i].pick.idx, of_cta[i].pick.raw);
+      merge_sum(t.m, t.s, of_cta[i].m, of_cta[i].s, k2);
+    }
+    out_tok[row] = t.pick.idx;
+    out_lp[row] = (t.pick.raw - t.m) * scale - logf(t.s);
+  }
+}
+
+// ------------------------------------------------------------------------------------------------------------------
+// top-k / top-p (nucleus) sampling without a sort: the k-th largest logit and the nucleus cut are found by MSB-first radix selection over
+// order-preserving integer keys of the logits (16 bits of a bf16 logit, 32 of an fp32 one), six bits at a time: counts for top-k,
+// probability mass for top-p.  Then Gumbel-max over the kept set and the log-prob under the renormalised distribution.  HF / SGLang
+// order: temperature -> top-k -> top-p.  (reference exposes rollout.top_k / rollout.top_p:
+// 3rdparty/verl/verl/trainer/config/rollout/rollout.yaml).
+//
+// Logits share a few exponents, so a histogram with shared-memory atomics runs one element after the other.  Here every thread owns a
+// column of 64 bins in shared memory ([bin][thread]: no bank conflict, no atomic), the columns are summed in a fixed order, then the CTAs'
+// sums over the cluster: the cut does not depend on timing (tensor-parallel engine ranks must sample identically).  Every pass reads the
+// row again, from L2: kept in registers (40 a thread at 152 K logits) or shared memory it would cost the third CTA of an SM.
+// [47, 151936] bf16, top_p 0.95: 46 us; with 64-bit atomics on 256 bins, one CTA per row and scalar loads it was 1808.
+// ------------------------------------------------------------------------------------------------------------------
+constexpr int kBins = 64;
+
+template <typename T>
+__global__ void __launch_bounds__(kSampleThreads, 3)
+sample_topk_topp_kernel(const T* __restrict__ logits, int64_t ld, int V, const float* __restrict__ temp, int inverse,
                         const uint64_t* __restrict__ seeds, int greedy_all, int top_k, float top_p,
                         int64_t* __restrict__ out_tok, float* __restrict__ out_lp) {
-  constexpr int NPASS = sizeof(T) == 2 ? 2 : 4;            // bf16 logits are exact in the top 16 key bits
-  constexpr float kL2e = 1.4426950408889634f;
-  __shared__ unsigned long long hist[256];
-  __shared__ float red[32];
-  __shared__ uint32_t s_prefix, s_mask;
-  __shared__ unsigned long long s_remaining;
-  const int row = blockIdx.x;
-  const T* lr = logits + static_cast<int64_t>(row) * ld;
-  const float it = inv_temp ? inv_temp[row] : 1.f;
-  const bool greedy = greedy_all || it <= 0.f;
-  const float scale = greedy ? 1.f : it;
+  using Row = SampleRow<T>;
+  constexpr int N = Row::N;
+  constexpr int KEY_BITS = 8 * static_cast<int>(sizeof(T));
+  extern __shared__ float hist[];                         // [kBins][kSampleThreads]; counts are stored as integers
+  struct Part { Pick pick; float mass; };
+  __shared__ Part part[kSampleWarps];
+  __shared__ Part of_cta[kSampleCtas];
+  __shared__ double sums[2][kSampleCtas][kBins];          // every CTA holds all CTAs' sums; two passes alternate
+  __shared__ float cta_max[kSampleCtas];
+  __shared__ uint32_t s_bin, bar;
+  __shared__ double s_rest;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = static_cast<int>(cluster.block_rank()), ctas = static_cast<int>(cluster.num_blocks());
+  const int row = blockIdx.x / ctas, tid = threadIdx.x, w = tid >> 5, l = tid & 31;
+  const Row r(logits + static_cast<int64_t>(row) * ld, V);
+  bool greedy;
+  const float scale = scale_of(temp, row, inverse != 0, greedy_all != 0, greedy);
+  const float k2 = scale * kLog2E;
   const uint64_t seed = seeds ? seeds[row] : 0;
+  const int ng = r.granules();
+  const int turns = (ng + ctas * kSampleThreads - 1) / (ctas * kSampleThreads);
+  auto granule = [&](int i) { return (i * ctas + rank) * kSampleThreads + tid; };
+  auto key_of = [](float f) { return order_key(f) >> (32 - KEY_BITS); };
+
+  // fn(unpacked granule, granule index) over the thread's granules, in a fixed order; a granule past the end reads as -inf
+  auto each = [&](auto&& fn) {
+    constexpr int AHEAD = 2;
+    for (int i = 0; i < turns; i += AHEAD) {
+      int4 q[AHEAD];
+#pragma unroll
+      for (int a = 0; a < AHEAD; ++a) q[a] = r.load(min(granule(i + a), ng));
+#pragma unroll
+      for (int a = 0; a < AHEAD; ++a) {
+        if (i + a >= turns) break;
+        float f[N];
+        Row::unpack(q[a], f);
+        fn(f, granule(i + a));
+      }
+    }
+  };
 
   float m = -INFINITY;
-  for (int i = threadIdx.x; i < V; i += blockDim.x) m = fmaxf(m, load_logit(lr, i));
-  m = block_reduce_max(m, red);
-
-  // ---- top-k: key of the k-th largest logit (ties at the cut are all kept, like `z < kth` masking)
-  uint32_t k_key = 0;
-  if (top_k > 0 && top_k < V) {
-    if (threadIdx.x == 0) { s_prefix = 0; s_mask = 0; s_remaining = static_cast<unsigned long long>(top_k); }
-    for (int pass = 0; pass < NPASS; ++pass) {
-      const int shift = 24 - 8 * pass;
-      for (int b = threadIdx.x; b < 256; b += blockDim.x) hist[b] = 0;
-      __syncthreads();
-      const uint32_t prefix = s_prefix, mask = s_mask;
-      for (int i = threadIdx.x; i < V; i += blockDim.x) {
-        const uint32_t key = order_key(load_logit(lr, i));
-        if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1ull);
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        unsigned long long cum = 0, rem = s_remaining;
-        int b = 255;
-        for (; b > 0; --b) {
-          if (cum + hist[b] >= rem) break;
-          cum += hist[b];
-        }
-        s_remaining = rem - cum;
-        s_prefix = prefix | (static_cast<uint32_t>(b) << shift);
-        s_mask = mask | (255u << shift);
-      }
-      __syncthreads();
-    }
-    k_key = s_prefix;
+  each([&](const float (&f)[N], int) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) m = fmaxf(m, f[j]);
+  });
+  m = warp_max(m);
+  if (l == 0) part[w].mass = m;
+  if (tid == 0) bar = order_key(-INFINITY);
+  __syncthreads();
+  if (tid < ctas) {
+    float t = part[0].mass;
+    for (int i = 1; i < kSampleWarps; ++i) t = fmaxf(t, part[i].mass);
+    *cluster.map_shared_rank(&cta_max[rank], tid) = t;
   }
+  cluster.sync();
+  m = cta_max[0];
+  for (int i = 1; i < ctas; ++i) m = fmaxf(m, cta_max[i]);
 
-  // ---- softmax mass of the top-k set
-  float sk = 0.f;
-  for (int i = threadIdx.x; i < V; i += blockDim.x) {
-    const float z = load_logit(lr, i);
-    if (order_key(z) >= k_key) sk += exp2f((z - m) * scale * kL2e);
-  }
-  sk = block_reduce_sum(sk, red);
-
-  // ---- top-p inside the top-k set: smallest prefix (by descending logit) whose mass reaches top_p * sk
-  uint32_t p_key = 0;
-  float s_kept = sk;
-  if (!greedy && top_p < 1.f && top_p > 0.f) {
-    const double kFix = 1099511627776.0;                  // 2^40 fixed-point mass units per unit weight (weights are <= 1)
-    if (threadIdx.x == 0) {
-      s_prefix = 0; s_mask = 0;
-      s_remaining = static_cast<unsigned long long>(static_cast<double>(top_p) * static_cast<double>(sk) * kFix);
-    }
-    for (int pass = 0; pass < NPASS; ++pass) {
-      const int shift = 24 - 8 * pass;
-      for (int b = threadIdx.x; b < 256; b += blockDim.x) hist[b] = 0;
+  // Largest key whose elements and all above reach `want` (a share of the whole where `share`), among elements with key >= floor_key.
+  // `mass`: weights instead of counts.
+  int pass_no = 0;
+  auto select = [&](bool mass, double want, bool share, uint32_t floor_key) -> uint32_t {
+    uint32_t prefix = 0;
+    for (int hi = KEY_BITS; hi > 0;) {
+      const int lo = hi > 6 ? hi - 6 : 0;
+      float* col = hist + tid;
+#pragma unroll 16
+      for (int b = 0; b < kBins; ++b) col[b * kSampleThreads] = 0.f;          // also the integer 0
+      each([&](const float (&f)[N], int) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+          const uint32_t key = key_of(f[j]);
+          if (key < floor_key || (hi < KEY_BITS && (key >> hi) != prefix)) continue;
+          float* bin = col + ((key >> lo) & ((1u << (hi - lo)) - 1u)) * kSampleThreads;
+          if (mass) *bin += ex2((f[j] - m) * k2);
+          else *reinterpret_cast<uint32_t*>(bin) += 1u;
+        }
+      });
       __syncthreads();
-      const uint32_t prefix = s_prefix, mask = s_mask;
-      for (int i = threadIdx.x; i < V; i += blockDim.x) {
-        const float z = load_logit(lr, i);
-        const uint32_t key = order_key(z);
-        if (key >= k_key && (key & mask) == prefix) {
-          const float w = exp2f((z - m) * scale * kL2e);
-          atomicAdd(&hist[(key >> shift) & 255u], static_cast<unsigned long long>(static_cast<double>(w) * kFix));
+      double(&all)[kSampleCtas][kBins] = sums[pass_no++ & 1];
+      for (int b = w; b < kBins; b += kSampleWarps) {
+        double t;
+        if (mass) {
+          float x = 0.f;
+#pragma unroll
+          for (int c = 0; c < kSampleWarps; ++c) x += hist[b * kSampleThreads + c * 32 + l];
+          t = warp_sum(x);
+        } else {
+          uint32_t x = 0;
+#pragma unroll
+          for (int c = 0; c < kSampleWarps; ++c) x += reinterpret_cast<const uint32_t*>(hist)[b * kSampleThreads + c * 32 + l];
+          t = __reduce_add_sync(0xffffffffu, x);
+        }
+        if (l < ctas) *cluster.map_shared_rank(&all[rank][b], l) = t;
+      }
+      cluster.sync();
+      if (w == 0) {                                        // lane l: bins 63 - 2 l and 62 - 2 l, from the top down
+        double a = 0., b = 0.;
+        for (int c = 0; c < ctas; ++c) { a += all[c][kBins - 1 - 2 * l]; b += all[c][kBins - 2 - 2 * l]; }
+        double up = a + b;                                 // inclusive sum over the lanes up to this one
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const double t = __shfl_up_sync(0xffffffffu, up, o);
+          if (l >= o) up += t;
+        }
+        if (share) want *= __shfl_sync(0xffffffffu, up, 31);
+        double above = __shfl_up_sync(0xffffffffu, up, 1);
+        if (l == 0) above = 0.;
+        const uint32_t hit = __ballot_sync(0xffffffffu, up >= want);
+        if (hit == 0) {
+          if (l == 0) { s_bin = 0; s_rest = 0.; }          // rounding left the sum short: everything with this prefix
+        } else if (l == __ffs(hit) - 1) {
+          const bool second = above + a < want;
+          s_bin = static_cast<uint32_t>(kBins - 1 - 2 * l - (second ? 1 : 0));
+          s_rest = want - above - (second ? a : 0.);
         }
       }
       __syncthreads();
-      if (threadIdx.x == 0) {
-        unsigned long long cum = 0, rem = s_remaining;
-        int b = 255;
-        for (; b > 0; --b) {
-          if (cum + hist[b] >= rem) break;
-          cum += hist[b];
-        }
-        s_remaining = rem > cum ? rem - cum : 0ull;
-        s_prefix = prefix | (static_cast<uint32_t>(b) << shift);
-        s_mask = mask | (255u << shift);
-      }
-      __syncthreads();
+      prefix = (prefix << (hi - lo)) | s_bin;
+      want = s_rest;
+      share = false;
+      hi = lo;
     }
-    p_key = s_prefix;
-  }
+    return prefix;
+  };
+
+  const uint32_t k_key = top_k > 0 && top_k < V ? select(false, static_cast<double>(top_k), false, 0) : 0;
+  const uint32_t p_key = !greedy && top_p < 1.f && top_p > 0.f ? select(true, static_cast<double>(top_p), true, k_key) : 0;
   const uint32_t cut = k_key > p_key ? k_key : p_key;
 
   // ---- Gumbel-max over the kept set + its mass
-  SampleState st{-INFINITY, 0x7fffffff, 0.f, -INFINITY, 0.f};
-  float mass = 0.f;
-  for (int i = threadIdx.x; i < V; i += blockDim.x) {
-    const float raw = load_logit(lr, i);
-    if (order_key(raw) < cut) continue;
-    const float z = raw * scale;
-    mass += exp2f((raw - m) * scale * kL2e);
-    const float key = greedy ? z : z + gumbel_noise(seed, row, i);
-    if (key > st.best || (key == st.best && i < st.best_idx)) { st.best = key; st.best_idx = i; st.best_z = z; }
-  }
-  if (cut != k_key || p_key != 0) s_kept = 0.f;           // recomputed below when the nucleus cut shrank the set
-  mass = block_reduce_sum(mass, red);
+  Pick best{-INFINITY, 0x7fffffff, -INFINITY};
+  float bar_now = -INFINITY, mass = 0.f;
+  each([&](const float (&raw)[N], int g) {
+    float f[N], fm = -INFINITY;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ob = __shfl_xor_sync(0xffffffffu, st.best, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, st.best_idx, o);
-    const float oz = __shfl_xor_sync(0xffffffffu, st.best_z, o);
-    if (ob > st.best || (ob == st.best && oi < st.best_idx)) { st.best = ob; st.best_idx = oi; st.best_z = oz; }
-  }
-  __shared__ float rb[32], rz[32];
-  __shared__ int ri[32];
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    for (int j = 0; j < N; ++j) {
+      f[j] = key_of(raw[j]) >= cut ? raw[j] : -INFINITY;
+      fm = fmaxf(fm, f[j]);
+    }
+    if (__any_sync(0xffffffffu, fm > -INFINITY)) {
+#pragma unroll
+      for (int j = 0; j < N; ++j) mass += ex2((f[j] - m) * k2);
+      offer_granule<N>(best, bar_now, f, fm, r.first(g), scale, greedy, seed, row);
+      bar_now = raise_bar(&bar, best);
+    }
+  });
+  best = warp_pick(best);
+  mass = warp_sum(mass);
+  if (l == 0) part[w] = Part{best, mass};
   __syncthreads();
-  if (l == 0) { rb[w] = st.best; ri[w] = st.best_idx; rz[w] = st.best_z; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float b = rb[0], z = rz[0];
-    int bi = ri[0];
-    for (int i = 1; i < (blockDim.x >> 5); ++i)
-      if (rb[i] > b || (rb[i] == b && ri[i] < bi)) { b = rb[i]; bi = ri[i]; z = rz[i]; }
-    out_tok[row] = bi;
-    out_lp[row] = (z - m * scale) - __logf(mass);
+  if (tid == 0) {
+    Part t = part[0];
+    for (int i = 1; i < kSampleWarps; ++i) { t.pick.offer(part[i].pick.key, part[i].pick.idx, part[i].pick.raw); t.mass += part[i].mass; }
+    *cluster.map_shared_rank(&of_cta[rank], 0) = t;
   }
-  (void)s_kept;
+  cluster.sync();
+  if (rank == 0 && tid == 0) {
+    Part t = of_cta[0];
+    for (int i = 1; i < ctas; ++i) { t.pick.offer(of_cta[i].pick.key, of_cta[i].pick.idx, of_cta[i].pick.raw); t.mass += of_cta[i].mass; }
+    out_tok[row] = t.pick.idx;
+    out_lp[row] = (t.pick.raw - m) * scale - logf(t.mass);
+  }
+}
+
+// CTAs per row: the most (a power of two, at most 8) that leave the whole batch resident on 148 SMs, `per_sm` CTAs on each.  A second,
+// ragged wave costs more: the plain sampler took 50 us for 128 rows with 8 CTAs a row (1.7 waves) and 37 with 4.
+inline int row_ctas(int B, int per_sm) {
+  int c = kSampleCtas;
+  while (c > 1 && static_cast<int64_t>(B) * c > 148 * per_sm) c >>= 1;
+  return c;
+}
+template <typename K, typename... Args>
+int launch_rows(K kernel, int B, int ctas, int smem, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(B) * ctas);
+  cfg.blockDim = dim3(kSampleThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = ctas;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  PRL_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, args...));
+  return 0;
+}
+
+template <typename T>
+int launch_topk_topp(const void* logits, int64_t ld, int B, int V, const float* temp, int inverse, const uint64_t* seeds, int greedy_all,
+                     int top_k, float top_p, int64_t* out_tok, float* out_lp, cudaStream_t s) {
+  constexpr int smem = kBins * kSampleThreads * static_cast<int>(sizeof(float));
+  PRL_CUDA_CHECK(cudaFuncSetAttribute(sample_topk_topp_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  return launch_rows(sample_topk_topp_kernel<T>, B, row_ctas(B, 3), smem, s, static_cast<const T*>(logits), ld, V, temp, inverse, seeds,
+                     greedy_all, top_k, top_p, out_tok, out_lp);
+}
+template <typename T>
+int launch_sample(const void* logits, int64_t ld, int B, int V, const float* temp, int inverse, const uint64_t* seeds, int greedy_all,
+                  int64_t* out_tok, float* out_lp, cudaStream_t s) {
+  return launch_rows(sample_kernel<T>, B, row_ctas(B, 4), 0, s, static_cast<const T*>(logits), ld, V, temp, inverse, seeds, greedy_all,
+                     out_tok, out_lp);
 }
 
 }  // namespace prl
 
 using namespace prl;
 
+// temp: temperatures of the rows (<= 0: greedy), or their inverses where `inverse`; null: 1.
 // top_k <= 0 disables top-k, top_p >= 1 disables top-p.  dtype: 0 = fp32 logits, 1 = bf16 logits.
-extern "C" int prl_sample_topk_topp(const void* logits, int dtype, int64_t ld, int B, int V, const float* inv_temp,
+extern "C" int prl_sample_topk_topp(const void* logits, int dtype, int64_t ld, int B, int V, const float* temp, int inverse,
                                     const uint64_t* seeds, int greedy_all, int top_k, float top_p, int64_t* out_tok,
                                     float* out_lp, cudaStream_t s) {
   if (B <= 0) return 0;
-  if (dtype == 0)
-    sample_topk_topp_kernel<float><<<B, 1024, 0, s>>>(static_cast<const float*>(logits), ld, V, inv_temp, seeds, greedy_all,
-                                                     top_k, top_p, out_tok, out_lp);
-  else
-    sample_topk_topp_kernel<__nv_bfloat16><<<B, 1024, 0, s>>>(static_cast<const __nv_bfloat16*>(logits), ld, V, inv_temp, seeds,
-                                                             greedy_all, top_k, top_p, out_tok, out_lp);
-  PRL_CUDA_CHECK(cudaGetLastError());
-  return 0;
+  return dtype == 0 ? launch_topk_topp<float>(logits, ld, B, V, temp, inverse, seeds, greedy_all, top_k, top_p, out_tok, out_lp, s)
+                    : launch_topk_topp<__nv_bfloat16>(logits, ld, B, V, temp, inverse, seeds, greedy_all, top_k, top_p, out_tok, out_lp, s);
 }
 
 // dtype: 0 = fp32 logits, 1 = bf16 logits
-extern "C" int prl_sample(const void* logits, int dtype, int64_t ld, int B, int V, const float* inv_temp,
+extern "C" int prl_sample(const void* logits, int dtype, int64_t ld, int B, int V, const float* temp, int inverse,
                           const uint64_t* seeds, int greedy_all, int64_t* out_tok, float* out_lp, cudaStream_t s) {
   if (B <= 0) return 0;
-  if (dtype == 0)
-    sample_kernel<float><<<B, 1024, 0, s>>>(static_cast<const float*>(logits), ld, V, inv_temp, seeds, greedy_all,
-                                           out_tok, out_lp);
-  else
-    sample_kernel<__nv_bfloat16><<<B, 1024, 0, s>>>(static_cast<const __nv_bfloat16*>(logits), ld, V, inv_temp, seeds,
-                                                   greedy_all, out_tok, out_lp);
-  PRL_CUDA_CHECK(cudaGetLastError());
-  return 0;
+  return dtype == 0 ? launch_sample<float>(logits, ld, B, V, temp, inverse, seeds, greedy_all, out_tok, out_lp, s)
+                    : launch_sample<__nv_bfloat16>(logits, ld, B, V, temp, inverse, seeds, greedy_all, out_tok, out_lp, s);
 }

@@ -549,13 +549,17 @@ def sample_tokens(logits: torch.Tensor, temperature: torch.Tensor | float = 1.0,
         temperature = torch.full((b,), float(temperature), device=logits.device, dtype=torch.float32)
     simple = top_k <= 0 and top_p >= 1.0
     if logits.is_cuda and logits.dtype in (torch.bfloat16, torch.float32):
-        inv_t = torch.where(temperature > 0, 1.0 / temperature.clamp_min(1e-6), torch.zeros_like(temperature))
         if seeds is None:
             seeds = torch.randint(0, 2 ** 62, (b,), device=logits.device, dtype=torch.int64)
+        seeds = seeds.contiguous()
+        # temperatures as the engine holds them go to the kernel, which inverts them; any other form becomes inverse temperatures here
+        inverse = temperature.dtype != torch.float32 or temperature.shape != (b,) or not temperature.is_contiguous()
+        scales = torch.where(temperature > 0, 1.0 / temperature.clamp_min(1e-6), torch.zeros_like(temperature)).float().expand(b).contiguous() \
+            if inverse else temperature
         if simple:
-            return tuple(_C().sample(logits, inv_t.float().contiguous(), seeds, bool(greedy)))
+            return tuple(_C().sample(logits, scales, seeds, bool(greedy), inverse))
         # top-k / top-p: radix-select kernel (no sort); log-prob under the renormalised kept set
-        return tuple(_C().sample_topk_topp(logits, inv_t.float().contiguous(), seeds, bool(greedy), int(top_k), float(top_p)))
+        return tuple(_C().sample_topk_topp(logits, scales, seeds, bool(greedy), int(top_k), float(top_p), inverse))
     z = logits.float()
     temperature = temperature.to(z.device)
     row_greedy = torch.ones_like(temperature, dtype=torch.bool) if greedy else temperature <= 0     # per row, like the kernel

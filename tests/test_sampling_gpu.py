@@ -1,0 +1,73 @@
+"""The samplers against a restatement of their noise in torch: every alignment of a row, ends of granules, one element up to several
+rounds of a cluster, masked logits, temperatures or their inverses."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def C():
+    from polyrl_b200 import ops
+
+    return ops.ext()
+
+
+def _hash(x):
+    m = 0xFFFFFFFF
+    x = ((x ^ (x >> 16)) * 0x7FEB352D) & m
+    x = ((x ^ (x >> 15)) * 0x846CA68B) & m
+    return x ^ (x >> 16)
+
+
+def _noise(seed, row, v):
+    n = _hash(_hash((torch.arange(v, device="cuda") + 0x9E3779B9 * (row + 1)) & 0xFFFFFFFF) ^ (seed & 0xFFFFFFFF))
+    u = ((_hash(n ^ (seed >> 32)) >> 8).float() + 0.5) * (1.0 / 16777216.0)
+    return -torch.log(-torch.log(u))
+
+
+def _rows(b, v, dtype, offset):
+    """[b, v] logits whose rows start anywhere: pitch v + 3, first element ``offset``; a tenth of them masked."""
+    base = torch.randn(b * (v + 3) + offset, device="cuda") * 2.5
+    z = base.to(dtype)[offset:].as_strided((b, v), (v + 3, 1))
+    z.masked_fill_(torch.rand(b, v, device="cuda") < 0.1, -math.inf)
+    z[:, v // 2] = 3.0
+    return z
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("b,v,offset", [(1, 1, 0), (3, 7, 1), (2, 255, 3), (5, 2049, 0), (3, 16385, 5), (2, 65543, 2), (2, 151936, 7), (33, 4096, 0)])
+@pytest.mark.parametrize("top_k,top_p", [(-1, 1.0), (17, 1.0), (-1, 0.9), (40, 0.6)])
+def test_choice_and_log_prob(C, dtype, b, v, offset, top_k, top_p):
+    torch.manual_seed(b * 1000 + v)
+    z = _rows(b, v, dtype, offset)
+    t = torch.rand(b, device="cuda") + 0.4
+    t[-1] = 0.0 if b > 2 else t[-1]                                    # one greedy row
+    seeds = torch.randint(0, 2 ** 62, (b,), device="cuda")
+    plain = top_k < 0 and top_p >= 1
+    f = (lambda s, inv: C.sample(z, s, seeds, False, inv)) if plain else (lambda s, inv: C.sample_topk_topp(z, s, seeds, False, top_k, top_p, inv))
+    tok, lp = f(t, False)
+    inv_t = torch.where(t > 0, 1.0 / t.clamp_min(1e-6), torch.zeros_like(t))
+    tok2, lp2 = f(inv_t, True)
+    assert torch.equal(tok, tok2) and torch.equal(lp, lp2)
+    for i in range(b):
+        greedy = float(t[i]) == 0
+        zi = z[i].double() / (1.0 if greedy else float(t[i]))
+        order = zi.sort(descending=True).values
+        if 0 < top_k < v:
+            zi = zi.masked_fill(zi < order[top_k - 1], -math.inf)
+        if top_p < 1 and not greedy:
+            kept = zi.sort(descending=True).values
+            p = kept.softmax(0)
+            zi = zi.masked_fill(zi < kept[(p.cumsum(0) - p) < top_p][-1], -math.inf)
+        want = zi.log_softmax(0)
+        k = int(tok[i])
+        assert 0 <= k < v and math.isfinite(float(want[k])), "a token outside the kept set"
+        # fp32 sums of v positive terms in trees of at most 2^5 sequential additions a level: 1e-5 is over 50 of their units
+        assert abs(float(lp[i]) - float(want[k])) < 1e-5 * max(1.0, abs(float(want[k])))
+        key = zi if greedy else zi + _noise(int(seeds[i]), i, v).double()
+        # the kernel's fast logarithm is 4e-7 off near one, where noise of up to log(2^24) comes from: 4e-7 e^11 relative for the
+        # best of 65 K, so a choice may differ only where two keys are that close
+        assert float(key.max() - key[k]) < 0.05
