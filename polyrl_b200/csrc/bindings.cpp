@@ -18,6 +18,7 @@ int prl_rmsnorm_fwd(const void*, const void*, void*, float*, int, int, float, cu
 int prl_add_rmsnorm(void*, const void*, const void*, void*, int, int, float, cudaStream_t);
 int prl_rmsnorm_bwd(const void*, const void*, const void*, const float*, void*, float*, int, int, cudaStream_t);
 int prl_rope(void*, const int64_t*, const float*, const float*, int, int, int, int, int64_t, float, void*, void*, const int64_t*, int, cudaStream_t);
+int prl_gather_pages(const void*, const void*, const int64_t*, const int64_t*, void*, void*, int, int64_t, int, int, int, cudaStream_t);
 int prl_swiglu_bwd(const void*, const void*, void*, int64_t, int, cudaStream_t);
 int prl_quant_fp8_rowwise(const void*, void*, float*, int, int, cudaStream_t);
 int prl_grad_accum(float*, const void*, int, float, int64_t, float*, cudaStream_t);
@@ -223,6 +224,21 @@ void rope_(at::Tensor qkv, const at::Tensor& pos, const at::Tensor& cos_tab, con
   check(prl_rope(qkv.data_ptr(), pos.data_ptr<int64_t>(), cos_tab.data_ptr<float>(), sin_tab.data_ptr<float>(),
                  qkv.size(0), nq, nkv, d, qkv.stride(0), static_cast<float>(sign), kc, vc, sm, block_size,
                  cur_stream()), "rope");
+}
+
+// (k, v) [T, nkv, d] of the cached positions (blk[t], off[t]) of caches [pages, nkv, page, d]
+std::vector<at::Tensor> gather_pages(const at::Tensor& k_cache, const at::Tensor& v_cache, const at::Tensor& blk, const at::Tensor& off) {
+  CHECK_BF16(k_cache); CHECK_BF16(v_cache);
+  TORCH_CHECK(k_cache.dim() == 4 && k_cache.sizes() == v_cache.sizes() && k_cache.is_contiguous() && v_cache.is_contiguous() && k_cache.size(3) % 8 == 0);
+  TORCH_CHECK(((reinterpret_cast<uintptr_t>(k_cache.data_ptr()) | reinterpret_cast<uintptr_t>(v_cache.data_ptr())) & 15) == 0, "caches must be 16-byte aligned");
+  for (const at::Tensor* t : {&blk, &off})
+    TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kLong && t->dim() == 1 && t->is_contiguous() && t->numel() == blk.numel());
+  c10::cuda::CUDAGuard g(k_cache.device());
+  const int64_t T = blk.numel(), nkv = k_cache.size(1), d = k_cache.size(3);
+  at::Tensor k = at::empty({T, nkv, d}, k_cache.options()), v = at::empty({T, nkv, d}, k_cache.options());
+  check(prl_gather_pages(k_cache.data_ptr(), v_cache.data_ptr(), blk.data_ptr<int64_t>(), off.data_ptr<int64_t>(), k.data_ptr(), v.data_ptr(), T,
+                         k_cache.size(0), nkv, k_cache.size(2), d, cur_stream()), "gather_pages");
+  return {k, v};
 }
 
 at::Tensor swiglu_bwd(const at::Tensor& gu, const at::Tensor& dh) {
@@ -555,6 +571,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("rmsnorm_bwd", &rmsnorm_bwd);
   m.def("add_rmsnorm_", &add_rmsnorm_);
   m.def("rope_", &rope_);
+  m.def("gather_pages", &gather_pages);
   m.def("swiglu_bwd", &swiglu_bwd);
   m.def("quant_fp8_rowwise", &quant_fp8_rowwise);
   m.def("grad_accum_", &grad_accum_);

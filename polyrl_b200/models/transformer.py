@@ -20,7 +20,7 @@ import torch.nn.functional as F
 from .. import ops
 from ..ops import reference as ref
 from ..ops.attention import attention_varlen
-from ..ops.functional import rope_and_cache_
+from ..ops.functional import gather_cached, rope_and_cache_
 from .config import ModelConfig
 
 ParamSpec = list[tuple[str, tuple[int, ...]]]
@@ -466,8 +466,8 @@ def layer_forward(cfg: ModelConfig, w: dict, x: torch.Tensor, inp: PackedInput, 
             from ..ops.attention import attention_varlen_prefix
 
             blk, off, cu_k, max_k = inp.kv_gather            # new tokens were appended to the cache just above
-            a = attention_varlen_prefix(q, kv_sink[0][blk, :, off, :], kv_sink[1][blk, :, off, :], inp.cu_seqlens, cu_k,
-                                        inp.max_seqlen, max_k)
+            keys, values = gather_cached(kv_sink[0], kv_sink[1], blk, off)
+            a = attention_varlen_prefix(q, keys, values, inp.cu_seqlens, cu_k, inp.max_seqlen, max_k)
         elif inp.sp_group is not None:
             from ..parallel.ulysses import ulysses_attention
 

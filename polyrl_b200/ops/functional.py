@@ -357,6 +357,16 @@ def rope_and_cache_(qkv, pos, cos, sin, nq, nkv, d, k_cache, v_cache, slot_mappi
     return qkv
 
 
+def gather_cached(k_cache: torch.Tensor, v_cache: torch.Tensor, blk: torch.Tensor, off: torch.Tensor):
+    """Keys and values [T, nkv, d] at the places (page ``blk[t]``, row ``off[t]``) of caches [pages, nkv, page, d]."""
+    if all(_is_kernel_tensor(c) and c.dim() == 4 and c.is_contiguous() and c.shape[3] % 8 == 0 and c.data_ptr() % 16 == 0 for c in (k_cache, v_cache)) \
+            and k_cache.shape == v_cache.shape and blk.shape == off.shape \
+            and all(i.device == k_cache.device == v_cache.device and i.dtype == torch.int64 and i.dim() == 1 and i.is_contiguous() for i in (blk, off)) \
+            and not (k_cache.requires_grad or v_cache.requires_grad):
+        return tuple(_C().gather_pages(k_cache, v_cache, blk, off))
+    return k_cache[blk, :, off, :], v_cache[blk, :, off, :]
+
+
 # --------------------------------------------------------------------------------------------
 # fused LM head: log-prob + entropy without materialising logits
 # --------------------------------------------------------------------------------------------
