@@ -16,7 +16,8 @@ int prl_linear_ce_fwd(const void*, const void*, const int64_t*, float, int, int,
 int prl_linear_ce_dz(const void*, const void*, const int64_t*, const float*, const float*, const float*, const float*, float, int, int, int, int, int64_t, int64_t, void*, int64_t, cudaStream_t);
 int prl_rmsnorm_fwd(const void*, const void*, void*, float*, int, int, float, cudaStream_t);
 int prl_add_rmsnorm(void*, const void*, const void*, void*, int, int, float, cudaStream_t);
-int prl_rmsnorm_bwd(const void*, const void*, const void*, const float*, void*, float*, int, int, cudaStream_t);
+int prl_rmsnorm_bwd(const void*, const void*, const void*, const float*, const void*, void*, float*, float*, void*, int, int, cudaStream_t);
+int prl_rmsnorm_bwd_parts(int, int);
 int prl_rope(void*, const int64_t*, const float*, const float*, int, int, int, int, int64_t, float, void*, void*, const int64_t*, int, cudaStream_t);
 int prl_gather_pages(const void*, const void*, const int64_t*, const int64_t*, void*, void*, int, int64_t, int, int, int, cudaStream_t);
 int prl_swiglu_bwd(const void*, const void*, void*, int64_t, int, cudaStream_t);
@@ -192,17 +193,26 @@ at::Tensor add_rmsnorm_(at::Tensor x, const at::Tensor& r, const at::Tensor& w, 
   return y;
 }
 
+// dres: gradient that reaches x past the norm, added to dx; the gain's gradient is fp32, or bf16 on request
 std::vector<at::Tensor> rmsnorm_bwd(const at::Tensor& x, const at::Tensor& w, const at::Tensor& dy,
-                                    const at::Tensor& rstd) {
+                                    const at::Tensor& rstd, const c10::optional<at::Tensor>& dres, bool dw_bf16) {
   CHECK_BF16(x); CHECK_BF16(w); CHECK_BF16(dy); CHECK_F32(rstd);
   TORCH_CHECK(x.is_contiguous() && dy.is_contiguous());
   const int H = x.size(-1);
   const int T = x.numel() / H;
+  TORCH_CHECK(H % 8 == 0 && H <= 8192, "rmsnorm_bwd: the row length must be a multiple of 8, at most 8192");
+  const void* r = nullptr;
+  if (dres.has_value()) {
+    CHECK_BF16(*dres);
+    TORCH_CHECK(dres->is_contiguous() && dres->sizes() == x.sizes() && (reinterpret_cast<uintptr_t>(dres->data_ptr()) & 15) == 0);
+    r = dres->data_ptr();
+  }
   c10::cuda::CUDAGuard g(x.device());
   at::Tensor dx = at::empty_like(x);
-  at::Tensor dw = at::zeros({H}, x.options().dtype(at::kFloat));
-  check(prl_rmsnorm_bwd(x.data_ptr(), w.data_ptr(), dy.data_ptr(), rstd.data_ptr<float>(), dx.data_ptr(),
-                        dw.data_ptr<float>(), T, H, cur_stream()), "rmsnorm_bwd");
+  at::Tensor part = at::empty({prl_rmsnorm_bwd_parts(T, H), H}, x.options().dtype(at::kFloat));
+  at::Tensor dw = at::empty({H}, x.options().dtype(dw_bf16 ? at::kBFloat16 : at::kFloat));
+  check(prl_rmsnorm_bwd(x.data_ptr(), w.data_ptr(), dy.data_ptr(), rstd.data_ptr<float>(), r, dx.data_ptr(), part.data_ptr<float>(),
+                        dw_bf16 ? nullptr : dw.data_ptr<float>(), dw_bf16 ? dw.data_ptr() : nullptr, T, H, cur_stream()), "rmsnorm_bwd");
   return {dx, dw};
 }
 
@@ -568,7 +578,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("linear_ce_fwd", &linear_ce_fwd);
   m.def("linear_ce_dz", &linear_ce_dz);
   m.def("rmsnorm_fwd", &rmsnorm_fwd);
-  m.def("rmsnorm_bwd", &rmsnorm_bwd);
+  m.def("rmsnorm_bwd", &rmsnorm_bwd, py::arg("x"), py::arg("w"), py::arg("dy"), py::arg("rstd"), py::arg("dres") = py::none(),
+        py::arg("dw_bf16") = false);
   m.def("add_rmsnorm_", &add_rmsnorm_);
   m.def("rope_", &rope_);
   m.def("gather_pages", &gather_pages);

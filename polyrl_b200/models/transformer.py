@@ -420,7 +420,7 @@ def xielu_mlp(w: dict, h: torch.Tensor, residual: torch.Tensor | None = None) ->
 
 def _mlp_forward(cfg: ModelConfig, w: dict, x: torch.Tensor, aux_out: list | None = None) -> torch.Tensor:
     """Second half of a llama-family block without adapters: x + MLP(norm(x)), dense SwiGLU or mixture of experts."""
-    h = ops.rmsnorm(x, w["ln2"], cfg.rms_norm_eps)
+    h, x = ops.rmsnorm_residual(x, w["ln2"], cfg.rms_norm_eps)
     if "router" in w:
         return x + moe_mlp(cfg, w, h, aux_out)
     if "wup" in w:
@@ -442,7 +442,7 @@ def layer_forward(cfg: ModelConfig, w: dict, x: torch.Tensor, inp: PackedInput, 
         lora = "_lora_scale" in w
         if lora:
             from . import lora as L
-        h = ops.rmsnorm(x, w["ln1"], cfg.rms_norm_eps)
+        h, x = ops.rmsnorm_residual(x, w["ln1"], cfg.rms_norm_eps)
         if cfg.attn_type == "mla":
             from . import mla
 
@@ -486,7 +486,7 @@ def layer_forward(cfg: ModelConfig, w: dict, x: torch.Tensor, inp: PackedInput, 
                 x = x + L.single_delta(w, a, "o_proj")
         if w.get("_skip_mlp"):              # callers that supply their own MLP (expert parallelism, parallel/expert.py)
             return x
-        h = ops.rmsnorm(x, w["ln2"], cfg.rms_norm_eps)
+        h, x = ops.rmsnorm_residual(x, w["ln2"], cfg.rms_norm_eps)
         if "router" in w:
             y = moe_mlp(cfg, w, h, aux_out)
             return x + (ops.rmsnorm(y, w["ln_mlp"], cfg.rms_norm_eps) if cfg.sandwich_norm else y)

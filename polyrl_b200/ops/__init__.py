@@ -91,6 +91,7 @@ from .functional import (  # noqa: E402
     linear,
     linear_swiglu,
     rmsnorm,
+    rmsnorm_residual,
     apply_rope,
     Fp8Weight,
     quantize_weight_fp8,
@@ -108,6 +109,7 @@ __all__ = [
     "linear",
     "linear_swiglu",
     "rmsnorm",
+    "rmsnorm_residual",
     "apply_rope",
     "Fp8Weight",
     "quantize_weight_fp8",

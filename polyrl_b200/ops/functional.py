@@ -298,14 +298,48 @@ class _RmsNormFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, w, rstd = ctx.saved_tensors
-        dx, dw = _C().rmsnorm_bwd(x, w, dy.contiguous(), rstd)
-        return dx, dw.to(w.dtype), None
+        dx, dw = _C().rmsnorm_bwd(x, w, dy.contiguous(), rstd, None, True)
+        return dx, dw, None
 
 
 def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float = 1e-6) -> torch.Tensor:
     if _is_kernel_tensor(x) and w.dtype == torch.bfloat16 and x.shape[-1] % 8 == 0 and x.shape[-1] <= 8192:
         return _RmsNormFn.apply(x, w, eps)
     return ref.rmsnorm(x, w, eps)
+
+
+class _RmsNormResidualFn(torch.autograd.Function):
+    """Norm of a residual stream that goes on past it: the second output is the stream itself, so its gradient arrives here and is
+    added inside the norm's backward kernel instead of in a pass of its own."""
+
+    @staticmethod
+    def forward(ctx, x, w, eps):
+        ctx.set_materialize_grads(False)
+        xc = x.contiguous()
+        y, rstd = _C().rmsnorm_fwd(xc, w, eps)
+        ctx.save_for_backward(xc, w, rstd)
+        return y, x.view_as(x)
+
+    @staticmethod
+    def backward(ctx, dy, dres):
+        x, w, rstd = ctx.saved_tensors
+        if dy is None:
+            return dres, None, None
+        dx, dw = _C().rmsnorm_bwd(x, w, dy.contiguous(), rstd, None if dres is None else _aligned(dres), True)
+        return dx, dw, None
+
+
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+def rmsnorm_residual(x: torch.Tensor, w: torch.Tensor, eps: float = 1e-6) -> tuple[torch.Tensor, torch.Tensor]:
+    """(rmsnorm(x), x): use the returned x for the residual branch, and its gradient is added inside the norm's backward."""
+    if _is_kernel_tensor(x) and w.dtype == torch.bfloat16 and x.shape[-1] % 8 == 0 and x.shape[-1] <= 8192 and torch.is_grad_enabled() \
+            and (x.requires_grad or w.requires_grad):
+        return _RmsNormResidualFn.apply(x, w, eps)
+    return rmsnorm(x, w, eps), x
 
 
 # --------------------------------------------------------------------------------------------

@@ -27,3 +27,21 @@ def test_gather_cached(t, nkv, page, d):
     # a strided cache takes the general path, with the same result
     wide = _randn(pages, nkv, page, 2 * d, seed=3)[..., :d]
     assert torch.equal(OF.gather_cached(wide, wide, blk, off)[0], wide[blk, :, off, :])
+
+
+@pytest.mark.parametrize("t,h", [(1, 64), (3, 896), (301, 1024), (640, 2048), (1187, 4096), (299, 5120), (41, 8192)])
+@pytest.mark.parametrize("res", [False, True])
+def test_rmsnorm_residual(t, h, res):
+    """Norm and residual stream together: one bf16 rounding per result, so 2^-9 of a value; the sums over rows and columns are fp32."""
+    x, w = _randn(t, h, seed=1).requires_grad_(True), _randn(h, seed=2, scale=0.1, shift=1.0).requires_grad_(True)
+    gy, gr = _randn(t, h, seed=3), _randn(t, h, seed=4)
+    y, xr = ops.rmsnorm_residual(x, w, 1e-6)
+    dx, dw = torch.autograd.grad([y, xr] if res else [y], [x, w], [gy, gr] if res else [gy])
+    x64, w64 = x.detach().double().requires_grad_(True), w.detach().double().requires_grad_(True)
+    y64 = x64 * torch.rsqrt(x64.pow(2).mean(-1, keepdim=True) + 1e-6) * w64
+    wx, ww = torch.autograd.grad([y64, x64 * 1.0] if res else [y64], [x64, w64], [gy.double(), gr.double()] if res else [gy.double()])
+    assert torch.equal(xr.detach(), x.detach())
+    for got, want in ((y, y64), (dx, wx), (dw, ww)):
+        err = (got.double() - want).abs()
+        assert (err <= 2.0 ** -8 * want.abs() + 1e-4 * want.abs().max()).all(), err.max()
+    assert torch.equal(torch.autograd.grad(ops.rmsnorm(x, w, 1e-6), w, gy)[0], dw)          # the partial sums have a fixed order
