@@ -25,8 +25,9 @@ constexpr int kAbSmem = 6 * kAbTile + 1024 + 256;
 
 struct AttnBwdParams {
   float* dq_acc;               // [Tq, nq*128] fp32, zero-initialised
-  __nv_bfloat16* dk;           // [Tk, nkv*128]
-  __nv_bfloat16* dv;           // [Tk, nkv*128]
+  __nv_bfloat16* dk;           // [Tk, nkv*128], row pitch lddkv
+  __nv_bfloat16* dv;
+  int64_t lddkv;
   const float* lse;            // [nq, Tq]
   const float* dsum;           // [nq, Tq]   D = rowsum(dO * O)
   const int32_t* cu_q;
@@ -245,8 +246,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       tc_fence_after();
     }
     const int krow = k0 + r;
-    __nv_bfloat16* dkp = p.dk + static_cast<int64_t>(ks + krow) * (static_cast<int64_t>(p.nkv) * 128) + hk * 128 + g * 64;
-    __nv_bfloat16* dvp = p.dv + static_cast<int64_t>(ks + krow) * (static_cast<int64_t>(p.nkv) * 128) + hk * 128 + g * 64;
+    __nv_bfloat16* dkp = p.dk + static_cast<int64_t>(ks + krow) * p.lddkv + hk * 128 + g * 64;
+    __nv_bfloat16* dvp = p.dv + static_cast<int64_t>(ks + krow) * p.lddkv + hk * 128 + g * 64;
 #pragma unroll
     for (int c = 0; c < 64; c += 32) {
       uint32_t a[32], b[32];
@@ -296,11 +297,11 @@ __global__ void attn_dsum_kernel(const __nv_bfloat16* __restrict__ o, const __nv
 
 using namespace prl;
 
-// dq_acc: fp32 [Tq, nq*128] zero-initialised by the caller; dk / dv: bf16 [Tk, nkv*128] (fully overwritten).
+// dq_acc: fp32 [Tq, nq*128] zero-initialised by the caller; dk / dv: bf16 [Tk, nkv*128] with row pitch lddkv (fully overwritten).
 extern "C" int prl_attn_bwd(const void* q, const void* k, const void* v, const void* o, const void* d_o, const float* lse,
                             float* dsum, float* dq_acc, void* dk, void* dv, const int32_t* cu_q, const int32_t* cu_k, int B,
                             int Tq, int Tk, int nq, int nkv, int64_t ldq, int64_t ldk, int64_t ldv, int64_t ldo, int64_t lddo,
-                            float sm_scale, int causal, int max_tiles, cudaStream_t stream) {
+                            int64_t lddkv, float sm_scale, int causal, int max_tiles, cudaStream_t stream) {
   if (Tq <= 0 || Tk <= 0 || B <= 0) return 0;
   if (nq % nkv != 0) return -120;
   {
@@ -317,7 +318,7 @@ extern "C" int prl_attn_bwd(const void* q, const void* k, const void* v, const v
   if (af_tmap(&tmV, v, Tk, static_cast<uint64_t>(nkv) * 128, ldv * 2, 128)) return -123;
   if (af_tmap(&tmdO, d_o, Tq, static_cast<uint64_t>(nq) * 128, lddo * 2, 128)) return -124;
   AttnBwdParams p;
-  p.dq_acc = dq_acc; p.dk = static_cast<__nv_bfloat16*>(dk); p.dv = static_cast<__nv_bfloat16*>(dv);
+  p.dq_acc = dq_acc; p.dk = static_cast<__nv_bfloat16*>(dk); p.dv = static_cast<__nv_bfloat16*>(dv); p.lddkv = lddkv;
   p.lse = lse; p.dsum = dsum; p.cu_q = cu_q; p.cu_k = cu_k;
   p.B = B; p.nq = nq; p.nkv = nkv; p.Tq = Tq;
   p.sm_scale = sm_scale; p.scale_log2 = sm_scale * 1.4426950408889634f; p.causal = causal;

@@ -25,7 +25,11 @@ int prl_quant_fp8_rowwise(const void*, void*, float*, int, int, cudaStream_t);
 int prl_grad_accum(float*, const void*, int, float, int64_t, float*, cudaStream_t);
 int prl_sumsq(const float*, int64_t, float*, cudaStream_t);
 int prl_adamw(float*, float*, float*, float*, void*, int64_t, float, float, float, float, float, int, float, const float*, int*, int, cudaStream_t);
-int prl_attn_bwd(const void*, const void*, const void*, const void*, const void*, const float*, float*, float*, void*, void*, const int32_t*, const int32_t*, int, int, int, int, int, int64_t, int64_t, int64_t, int64_t, int64_t, float, int, int, cudaStream_t);
+int prl_attn_bwd(const void*, const void*, const void*, const void*, const void*, const float*, float*, float*, void*, void*, const int32_t*, const int32_t*, int, int, int, int, int, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, float, int, int, cudaStream_t);
+int prl_qk_rope_width_ok(int);
+int prl_qk_rope(const void*, void*, const int64_t*, const float*, const float*, const void*, const void*, float, int, int, int, int, int64_t, int64_t, float, void*, void*, const int64_t*, int, cudaStream_t);
+int prl_qk_norm_rope_bwd_parts(int, int, int, int);
+int prl_qk_norm_rope_bwd(const void*, int64_t, void*, int64_t, const int64_t*, const float*, const float*, const void*, const void*, float, float*, void*, void*, int, int, int, int, cudaStream_t);
 int prl_ipc_get_handle(void*, void*);
 int prl_ipc_open_handle(const void*, void**);
 int prl_ipc_close_handle(void*);
@@ -231,9 +235,70 @@ void rope_(at::Tensor qkv, const at::Tensor& pos, const at::Tensor& cos_tab, con
     TORCH_CHECK(slot_mapping->scalar_type() == at::kLong);
     sm = slot_mapping->data_ptr<int64_t>();
   }
+  auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  // 16-byte accesses where widths, pitch and addresses allow them; the caches' rows are d wide
+  if (prl_qk_rope_width_ok(d) && qkv.stride(0) % 8 == 0 && aligned(qkv.data_ptr()) && aligned(cos_tab.data_ptr()) && aligned(sin_tab.data_ptr()) &&
+      aligned(kc) && aligned(vc)) {
+    check(prl_qk_rope(qkv.data_ptr(), qkv.data_ptr(), pos.data_ptr<int64_t>(), cos_tab.data_ptr<float>(), sin_tab.data_ptr<float>(), nullptr, nullptr, 0.f,
+                      qkv.size(0), nq, nkv, d, qkv.stride(0), qkv.stride(0), static_cast<float>(sign), kc, vc, sm, block_size, cur_stream()), "rope");
+    return;
+  }
   check(prl_rope(qkv.data_ptr(), pos.data_ptr<int64_t>(), cos_tab.data_ptr<float>(), sin_tab.data_ptr<float>(),
                  qkv.size(0), nq, nkv, d, qkv.stride(0), static_cast<float>(sign), kc, vc, sm, block_size,
                  cur_stream()), "rope");
+}
+
+// RMS norm of every query and key head, then rotation, of packed rows [T, (nq + 2 nkv) * d]: in place, or into `out` [T, (nq + nkv) * d];
+// optionally appends rotated keys and the values to the paged cache.
+void check_qk(const at::Tensor& qkv, const at::Tensor& pos, const at::Tensor& cos_tab, const at::Tensor& sin_tab, const at::Tensor& qn, const at::Tensor& kn,
+              int64_t nq, int64_t nkv, int64_t d) {
+  CHECK_BF16(qkv); CHECK_BF16(qn); CHECK_BF16(kn); CHECK_F32(cos_tab); CHECK_F32(sin_tab);
+  TORCH_CHECK(qkv.dim() == 2 && qkv.stride(1) == 1 && qkv.stride(0) % 8 == 0 && qkv.size(1) >= (nq + 2 * nkv) * d && prl_qk_rope_width_ok(d), "qk_norm_rope: rows");
+  TORCH_CHECK(pos.is_cuda() && pos.scalar_type() == at::kLong && pos.is_contiguous() && pos.numel() == qkv.size(0));
+  TORCH_CHECK(cos_tab.is_contiguous() && sin_tab.is_contiguous() && cos_tab.size(-1) == d / 2 && sin_tab.size(-1) == d / 2);
+  TORCH_CHECK(qn.is_contiguous() && kn.is_contiguous() && qn.numel() == d && kn.numel() == d);
+  for (const at::Tensor* t : {&qkv, &cos_tab, &sin_tab, &qn, &kn})
+    TORCH_CHECK((reinterpret_cast<uintptr_t>(t->data_ptr()) & 15) == 0, "qk_norm_rope: 16-byte aligned operands");
+}
+void qk_norm_rope_(at::Tensor qkv, const at::Tensor& pos, const at::Tensor& cos_tab, const at::Tensor& sin_tab, int64_t nq, int64_t nkv, int64_t d,
+                   const at::Tensor& qn, const at::Tensor& kn, double eps, const c10::optional<at::Tensor>& out, const c10::optional<at::Tensor>& k_cache,
+                   const c10::optional<at::Tensor>& v_cache, const c10::optional<at::Tensor>& slot_mapping, int64_t block_size) {
+  check_qk(qkv, pos, cos_tab, sin_tab, qn, kn, nq, nkv, d);
+  c10::cuda::CUDAGuard g(qkv.device());
+  void* dst = qkv.data_ptr();
+  int64_t ldo = qkv.stride(0);
+  if (out.has_value()) {
+    CHECK_BF16(*out);
+    TORCH_CHECK(out->dim() == 2 && out->is_contiguous() && out->size(0) == qkv.size(0) && out->size(1) == (nq + nkv) * d &&
+                (reinterpret_cast<uintptr_t>(out->data_ptr()) & 15) == 0);
+    dst = out->data_ptr();
+    ldo = out->stride(0);
+  }
+  void* kc = nullptr; void* vc = nullptr; const int64_t* sm = nullptr;
+  if (slot_mapping.has_value()) {
+    TORCH_CHECK(k_cache.has_value() && v_cache.has_value() && slot_mapping->scalar_type() == at::kLong && slot_mapping->is_contiguous());
+    CHECK_BF16(*k_cache); CHECK_BF16(*v_cache);
+    kc = k_cache->data_ptr(); vc = v_cache->data_ptr(); sm = slot_mapping->data_ptr<int64_t>();
+    TORCH_CHECK(((reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 15) == 0);
+  }
+  check(prl_qk_rope(qkv.data_ptr(), dst, pos.data_ptr<int64_t>(), cos_tab.data_ptr<float>(), sin_tab.data_ptr<float>(), qn.data_ptr(), kn.data_ptr(),
+                    static_cast<float>(eps), qkv.size(0), nq, nkv, d, qkv.stride(0), ldo, 1.f, kc, vc, sm, block_size, cur_stream()), "qk_norm_rope");
+}
+// gradient of the above, in place on the query and key columns of g; x: the rows before the norm.  Returns the gains' gradients.
+std::vector<at::Tensor> qk_norm_rope_bwd_(at::Tensor g, const at::Tensor& x, const at::Tensor& pos, const at::Tensor& cos_tab, const at::Tensor& sin_tab,
+                                          int64_t nq, int64_t nkv, int64_t d, const at::Tensor& qn, const at::Tensor& kn, double eps) {
+  check_qk(x, pos, cos_tab, sin_tab, qn, kn, nq, nkv, d);
+  CHECK_BF16(g);
+  TORCH_CHECK(g.dim() == 2 && g.stride(1) == 1 && g.stride(0) % 8 == 0 && g.size(0) == x.size(0) && g.size(1) >= (nq + nkv) * d &&
+              (reinterpret_cast<uintptr_t>(g.data_ptr()) & 15) == 0, "qk_norm_rope_bwd: gradient rows");
+  c10::cuda::CUDAGuard dg(x.device());
+  const int T = x.size(0);
+  at::Tensor part = at::empty({prl_qk_norm_rope_bwd_parts(T, nq, nkv, d), d}, x.options().dtype(at::kFloat));
+  at::Tensor dqn = at::empty({d}, qn.options()), dkn = at::empty({d}, kn.options());
+  check(prl_qk_norm_rope_bwd(x.data_ptr(), x.stride(0), g.data_ptr(), g.stride(0), pos.data_ptr<int64_t>(), cos_tab.data_ptr<float>(),
+                             sin_tab.data_ptr<float>(), qn.data_ptr(), kn.data_ptr(), static_cast<float>(eps), part.data_ptr<float>(), dqn.data_ptr(),
+                             dkn.data_ptr(), T, nq, nkv, d, cur_stream()), "qk_norm_rope_bwd");
+  return {dqn, dkn};
 }
 
 // (k, v) [T, nkv, d] of the cached positions (blk[t], off[t]) of caches [pages, nkv, page, d]
@@ -302,10 +367,11 @@ void adamw_(at::Tensor master, at::Tensor m, at::Tensor v, at::Tensor grad, cons
 }
 
 // varlen causal flash-attention forward on tcgen05 (csrc/attn_fwd.cu).  q:[Tq,nq,128] k,v:[Tk,nkv,128] (row-strided views allowed)
-// flash-attention backward (csrc/attn_bwd.cu): returns (dq, dk, dv) in bf16, shapes of q / k / v (contiguous)
+// flash-attention backward (csrc/attn_bwd.cu): (dq, dk, dv) in bf16, shapes of q / k / v; contiguous, or views of the columns of `out`
+// [T, (nq + 2 nkv) * 128] (the gradient of a fused projection: query, key and value heads side by side)
 std::vector<at::Tensor> attn_bwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& o,
                                  const at::Tensor& d_o, const at::Tensor& lse, const at::Tensor& cu_q, const at::Tensor& cu_k,
-                                 double sm_scale, bool causal) {
+                                 double sm_scale, bool causal, const c10::optional<at::Tensor>& out) {
   CHECK_BF16(q); CHECK_BF16(k); CHECK_BF16(v); CHECK_BF16(o); CHECK_BF16(d_o); CHECK_F32(lse);
   for (const at::Tensor* t : {&q, &k, &v, &o, &d_o}) {
     TORCH_CHECK(t->dim() == 3 && t->size(2) == 128 && t->stride(2) == 1 && t->stride(1) == 128 && t->stride(0) % 8 == 0 &&
@@ -314,15 +380,26 @@ std::vector<at::Tensor> attn_bwd(const at::Tensor& q, const at::Tensor& k, const
   const int Tq = q.size(0), Tk = k.size(0), nq = q.size(1), nkv = k.size(1), B = cu_q.numel() - 1;
   TORCH_CHECK(lse.is_contiguous() && lse.size(0) == nq && lse.size(1) == Tq);
   c10::cuda::CUDAGuard g(q.device());
+  at::Tensor dq, dk, dv;
+  if (out.has_value()) {
+    CHECK_BF16(*out);
+    TORCH_CHECK(Tq == Tk && out->dim() == 2 && out->is_contiguous() && out->size(0) == Tq && out->size(1) == (nq + 2 * nkv) * 128 &&
+                (reinterpret_cast<uintptr_t>(out->data_ptr()) & 15) == 0, "attn_bwd: out is [T, (nq + 2 nkv) * 128]");
+    const at::Tensor heads = out->view({Tq, nq + 2 * nkv, 128});
+    dq = heads.narrow(1, 0, nq); dk = heads.narrow(1, nq, nkv); dv = heads.narrow(1, nq + nkv, nkv);
+  } else {
+    dk = at::empty({Tk, nkv, 128}, q.options());
+    dv = at::empty({Tk, nkv, 128}, q.options());
+  }
   at::Tensor dq_acc = at::zeros({Tq, nq, 128}, q.options().dtype(at::kFloat));
-  at::Tensor dk = at::empty({Tk, nkv, 128}, q.options());
-  at::Tensor dv = at::empty({Tk, nkv, 128}, q.options());
   at::Tensor dsum = at::empty({nq, Tq}, q.options().dtype(at::kFloat));
   check(prl_attn_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), d_o.data_ptr(), lse.data_ptr<float>(),
                      dsum.data_ptr<float>(), dq_acc.data_ptr<float>(), dk.data_ptr(), dv.data_ptr(), cu_q.data_ptr<int>(),
-                     cu_k.data_ptr<int>(), B, Tq, Tk, nq, nkv, q.stride(0), k.stride(0), v.stride(0), o.stride(0), d_o.stride(0),
+                     cu_k.data_ptr<int>(), B, Tq, Tk, nq, nkv, q.stride(0), k.stride(0), v.stride(0), o.stride(0), d_o.stride(0), dk.stride(0),
                      static_cast<float>(sm_scale), causal ? 1 : 0, Tk / 128 + B, cur_stream()), "attn_bwd");
-  return {dq_acc.to(at::kBFloat16), dk, dv};
+  if (out.has_value()) dq.copy_(dq_acc);
+  else dq = dq_acc.to(at::kBFloat16);
+  return {dq, dk, dv};
 }
 
 // Decode-shape GEMM (swap-AB + split-K).  mode 0: out = x @ w.T (+bias)(+residual); mode 1: SwiGLU on interleaved W.
@@ -583,12 +660,17 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("add_rmsnorm_", &add_rmsnorm_);
   m.def("rope_", &rope_);
   m.def("gather_pages", &gather_pages);
+  m.def("qk_norm_rope_", &qk_norm_rope_, py::arg("qkv"), py::arg("pos"), py::arg("cos"), py::arg("sin"), py::arg("nq"), py::arg("nkv"), py::arg("d"),
+        py::arg("q_norm"), py::arg("k_norm"), py::arg("eps"), py::arg("out") = py::none(), py::arg("k_cache") = py::none(), py::arg("v_cache") = py::none(),
+        py::arg("slot_mapping") = py::none(), py::arg("block_size") = 16);
+  m.def("qk_norm_rope_bwd_", &qk_norm_rope_bwd_);
   m.def("swiglu_bwd", &swiglu_bwd);
   m.def("quant_fp8_rowwise", &quant_fp8_rowwise);
   m.def("grad_accum_", &grad_accum_);
   m.def("sumsq_", &sumsq_);
   m.def("adamw_", &adamw_);
-  m.def("attn_bwd", &attn_bwd);
+  m.def("attn_bwd", &attn_bwd, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("o"), py::arg("d_o"), py::arg("lse"), py::arg("cu_q"), py::arg("cu_k"),
+        py::arg("sm_scale"), py::arg("causal"), py::arg("out") = py::none());
   m.def("sym_malloc", &sym_malloc);
   m.def("sym_free", &sym_free);
   m.def("ipc_get_handle", &ipc_get_handle);

@@ -19,8 +19,8 @@ import torch.nn.functional as F
 
 from .. import ops
 from ..ops import reference as ref
-from ..ops.attention import attention_varlen
-from ..ops.functional import gather_cached, rope_and_cache_
+from ..ops.attention import attention_varlen, rope_attention
+from ..ops.functional import gather_cached, head_norm_ok, head_norm_rope_and_cache_, rope_and_cache_
 from .config import ModelConfig
 
 ParamSpec = list[tuple[str, tuple[int, ...]]]
@@ -228,8 +228,8 @@ def rope_tables(cfg: ModelConfig, device) -> tuple[torch.Tensor, torch.Tensor]:
 
 
 def qk_norm_(cfg: ModelConfig, w: dict, qkv: torch.Tensor) -> torch.Tensor:
-    """Qwen3: RMS-normalise every q and k head (over head_dim) with learned gains, before RoPE.  Library ops on purpose (rows of
-    128 elements are a poor fit for the row-per-CTA norm kernel); returns a new fused qkv tensor."""
+    """Qwen3: RMS-normalise every q and k head (over head_dim) with learned gains, before RoPE: the general form, in library
+    ops, where the kernel that norms and rotates in one pass does not apply; returns a new fused qkv tensor."""
     if "q_norm" not in w:
         return qkv
     t = qkv.shape[0]
@@ -237,6 +237,17 @@ def qk_norm_(cfg: ModelConfig, w: dict, qkv: torch.Tensor) -> torch.Tensor:
     q = ref.rmsnorm(qkv[:, : nq * d].reshape(t, nq, d), w["q_norm"], cfg.rms_norm_eps)
     k = ref.rmsnorm(qkv[:, nq * d:(nq + nkv) * d].reshape(t, nkv, d), w["k_norm"], cfg.rms_norm_eps)
     return torch.cat([q.reshape(t, nq * d), k.reshape(t, nkv * d), qkv[:, (nq + nkv) * d:]], dim=-1)
+
+
+def qk_norm_rope_and_cache_(cfg: ModelConfig, w: dict, qkv: torch.Tensor, pos, cos, sin, k_cache, v_cache, slots, page: int | None = None) -> torch.Tensor:
+    """Inference: head norms (if the model has them), rotation and append to the paged cache; one kernel where its operands fit."""
+    nq, nkv, d = cfg.num_heads, cfg.num_kv_heads, cfg.head_dim
+    page = k_cache.shape[2] if page is None else page
+    if "q_norm" in w and head_norm_ok(qkv, cos, sin, d, w["q_norm"], w["k_norm"]) and not (torch.is_grad_enabled() and qkv.requires_grad) \
+            and all(c.dtype == torch.bfloat16 and c.is_contiguous() and c.data_ptr() % 16 == 0 for c in (k_cache, v_cache)) \
+            and all(i.is_cuda and i.dtype == torch.int64 and i.is_contiguous() and i.numel() == qkv.shape[0] for i in (pos, slots)):
+        return head_norm_rope_and_cache_(qkv, pos, cos, sin, nq, nkv, d, w["q_norm"], w["k_norm"], cfg.rms_norm_eps, k_cache, v_cache, slots, page)
+    return rope_and_cache_(qk_norm_(cfg, w, qkv), pos, cos, sin, nq, nkv, d, k_cache, v_cache, slots, page)
 
 
 def _MOE_STATIC_DECODE() -> bool:
@@ -453,15 +464,19 @@ def layer_forward(cfg: ModelConfig, w: dict, x: torch.Tensor, inp: PackedInput, 
         qkv = ops.linear(h, w["wqkv"], bias=w.get("bqkv"))
         if lora and L.has_lora(w, "q_proj", "k_proj", "v_proj"):
             qkv = qkv + L.qkv_delta(cfg, w, h)
-        qkv = qk_norm_(cfg, w, qkv)
         pos, cos, sin = inp.rope_inputs(cfg, x.device)
+        a = None
         if kv_sink is not None:
-            qkv = rope_and_cache_(qkv, pos, cos, sin, nq, nkv, d, *kv_sink)
+            qkv = qk_norm_rope_and_cache_(cfg, w, qkv, pos, cos, sin, *kv_sink[:3], page=kv_sink[3] if len(kv_sink) > 3 else 16)
         else:
-            qkv = ops.apply_rope(qkv, pos, cos, sin, nq, nkv, d)
-        q = qkv[:, : nq * d].view(t, nq, d)
-        k = qkv[:, nq * d:(nq + nkv) * d].view(t, nkv, d)
-        v = qkv[:, (nq + nkv) * d:].view(t, nkv, d)
+            if inp.sp_group is None:
+                a = rope_attention(qkv, pos, cos, sin, nq, nkv, d, inp.cu_seqlens, w.get("q_norm"), w.get("k_norm"), cfg.rms_norm_eps)
+            if a is None:
+                qkv = ops.apply_rope(qk_norm_(cfg, w, qkv), pos, cos, sin, nq, nkv, d)
+        if a is None:
+            q = qkv[:, : nq * d].view(t, nq, d)
+            k = qkv[:, nq * d:(nq + nkv) * d].view(t, nkv, d)
+            v = qkv[:, (nq + nkv) * d:].view(t, nkv, d)
         if inp.kv_gather is not None and kv_sink is not None:
             from ..ops.attention import attention_varlen_prefix
 
@@ -472,7 +487,7 @@ def layer_forward(cfg: ModelConfig, w: dict, x: torch.Tensor, inp: PackedInput, 
             from ..parallel.ulysses import ulysses_attention
 
             a = ulysses_attention(q, k, v, inp.cu_seqlens, inp.max_seqlen, inp.sp_group, inp.total_tokens, causal=True)
-        else:
+        elif a is None:
             a = attention_varlen(q, k, v, inp.cu_seqlens, inp.max_seqlen, causal=True)
         a = a.reshape(t, nq * d)
         if cfg.sandwich_norm:
@@ -575,10 +590,9 @@ def layer_decode(cfg: ModelConfig, w: dict, x: torch.Tensor, inp: DecodeInput, k
         return ops.linear(ops.linear_swiglu(h, w["wgu"]), w["wd"], residual=x)
     if cfg.family == "llama":
         h = ops.rmsnorm(x, w["ln1"], cfg.rms_norm_eps)
-        qkv = qk_norm_(cfg, w, ops.linear(h, w["wqkv"], bias=w.get("bqkv")))
         cos, sin = rope_tables(cfg, x.device)
-        rope_and_cache_(qkv, inp.position_ids, cos, sin, nq, nkv, d, k_cache, v_cache, inp.slot_mapping,
-                        k_cache.shape[2])
+        qkv = qk_norm_rope_and_cache_(cfg, w, ops.linear(h, w["wqkv"], bias=w.get("bqkv")), inp.position_ids, cos, sin, k_cache, v_cache,
+                                      inp.slot_mapping)
         a = ops.paged_decode_attention(qkv[:, : nq * d], k_cache, v_cache, inp.block_table, inp.seq_lens, nq, nkv, d,
                                        scale, max_len=inp.max_len)
         if cfg.sandwich_norm:
@@ -618,9 +632,8 @@ def layer_decode_fused(cfg: ModelConfig, w: dict, x: torch.Tensor, delta: torch.
     C = ext()
     nq, nkv, d = cfg.num_heads, cfg.num_kv_heads, cfg.head_dim
     h = ops.rmsnorm(x, w["ln1"], cfg.rms_norm_eps) if delta is None else C.add_rmsnorm_(x, delta, w["ln1"], cfg.rms_norm_eps)
-    qkv = qk_norm_(cfg, w, ops.linear(h, w["wqkv"], bias=w.get("bqkv")))
     cos, sin = rope_tables(cfg, x.device)
-    rope_and_cache_(qkv, inp.position_ids, cos, sin, nq, nkv, d, k_cache, v_cache, inp.slot_mapping, k_cache.shape[2])
+    qkv = qk_norm_rope_and_cache_(cfg, w, ops.linear(h, w["wqkv"], bias=w.get("bqkv")), inp.position_ids, cos, sin, k_cache, v_cache, inp.slot_mapping)
     a = ops.paged_decode_attention(qkv[:, : nq * d], k_cache, v_cache, inp.block_table, inp.seq_lens, nq, nkv, d, d ** -0.5,
                                    max_len=inp.max_len)
     o = ops.linear(a, w["wo"])

@@ -61,6 +61,80 @@ def _own_attention(q, k, v, cu_q, cu_k, scale, causal=True):
     return ext().attn_fwd(_rows(q), _rows(k), _rows(v), cu_q.contiguous(), cu_k.contiguous(), float(scale), bool(causal), False)[0]
 
 
+class _RopeAttnFn(torch.autograd.Function):
+    """Optional norm of the query and key heads, rotation and causal attention over packed rows of a fused projection.  One function,
+    so that the backward kernels write query, key and value gradients side by side into the gradient of the projection: as separate
+    functions, autograd filled, copied and added three tensors of the projection's size to put them together."""
+
+    @staticmethod
+    def forward(ctx, qkv, pos, cos, sin, q_norm, k_norm, eps, cu, nq, nkv, d, scale):
+        from . import ext
+
+        C, t = ext(), qkv.shape[0]
+        if q_norm is not None:
+            rot = torch.empty(t, (nq + nkv) * d, device=qkv.device, dtype=qkv.dtype)
+            C.qk_norm_rope_(qkv, pos, cos, sin, nq, nkv, d, q_norm, k_norm, eps, rot)
+        else:
+            C.rope_(qkv, pos, cos, sin, nq, nkv, d, 1.0, None, None, None, 16)
+            rot = None
+        q, k, v = _heads(qkv if rot is None else rot, qkv, nq, nkv, d)
+        o, lse = C.attn_fwd(q, k, v, cu, cu, scale, True, True)
+        ctx.save_for_backward(qkv, rot, o, lse, pos, cos, sin, q_norm, k_norm, cu)
+        ctx.dims = (nq, nkv, d, scale, eps)
+        return o
+
+    @staticmethod
+    def backward(ctx, do):
+        from . import ext
+
+        C = ext()
+        qkv, rot, o, lse, pos, cos, sin, q_norm, k_norm, cu = ctx.saved_tensors
+        nq, nkv, d, scale, eps = ctx.dims
+        q, k, v = _heads(qkv if rot is None else rot, qkv, nq, nkv, d)
+        g = torch.empty(qkv.shape, device=qkv.device, dtype=qkv.dtype)
+        C.attn_bwd(q, k, v, o, _rows(do), lse, cu, cu, scale, True, g)
+        dqn = dkn = None
+        if rot is not None:
+            dqn, dkn = C.qk_norm_rope_bwd_(g, qkv, pos, cos, sin, nq, nkv, d, q_norm, k_norm, eps)
+        else:
+            C.rope_(g, pos, cos, sin, nq, nkv, d, -1.0, None, None, None, 16)
+        return g, None, None, None, dqn, dkn, None, None, None, None, None, None
+
+
+def _heads(qk: torch.Tensor, qkv: torch.Tensor, nq: int, nkv: int, d: int):
+    """Views [T, heads, d] of the query and key columns of ``qk`` and the value columns of ``qkv``."""
+    t = qkv.shape[0]
+    return (qk[:, : nq * d].view(t, nq, d), qk[:, nq * d:(nq + nkv) * d].view(t, nkv, d),
+            qkv[:, (nq + nkv) * d:].view(t, nkv, d))
+
+
+def rope_attention(qkv: torch.Tensor, pos: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, nq: int, nkv: int, d: int,
+                   cu_seqlens: torch.Tensor, q_norm: torch.Tensor | None = None, k_norm: torch.Tensor | None = None,
+                   eps: float = 1e-6) -> torch.Tensor | None:
+    """Causal attention [T, nq, d] over packed rows ``qkv`` [T, (nq + 2 nkv) * d] of a projection, its query and key heads normed (if
+    gains are given) and rotated first.  ``qkv`` is consumed: its contents afterwards are undefined.  None: these operands need the
+    general path (``apply_rope`` and ``attention_varlen``)."""
+    from .functional import head_norm_ok
+
+    if not (qkv.dim() == 2 and qkv.is_contiguous() and qkv.shape[1] == (nq + 2 * nkv) * d and qkv.data_ptr() % 16 == 0 and cu_seqlens.is_cuda
+            and pos.is_cuda and pos.dtype == torch.int64 and pos.is_contiguous() and pos.dim() == 1 and pos.shape[0] == qkv.shape[0]
+            and not any(t.requires_grad for t in (cos, sin))):
+        return None
+    q, k, v = _heads(qkv.detach(), qkv.detach(), nq, nkv, d)
+    if not _own_ok(q, k, v) or (q_norm is not None and not head_norm_ok(qkv, cos, sin, d, q_norm, k_norm)):
+        return None
+    cu, scale = cu_seqlens.to(torch.int32).contiguous(), d ** -0.5
+    if torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (qkv, q_norm, k_norm)):
+        return _RopeAttnFn.apply(qkv, pos, cos, sin, q_norm, k_norm, eps, cu, nq, nkv, d, scale)
+    from . import ext
+
+    if q_norm is not None:
+        ext().qk_norm_rope_(qkv, pos, cos, sin, nq, nkv, d, q_norm, k_norm, eps)
+    else:
+        ext().rope_(qkv, pos, cos, sin, nq, nkv, d, 1.0, None, None, None, 16)
+    return ext().attn_fwd(q, k, v, cu, cu, scale, True, False)[0]
+
+
 def _flash():
     global _FLASH
     if _FLASH is None:

@@ -391,6 +391,21 @@ def rope_and_cache_(qkv, pos, cos, sin, nq, nkv, d, k_cache, v_cache, slot_mappi
     return qkv
 
 
+def head_norm_ok(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, d: int, q_norm: torch.Tensor, k_norm: torch.Tensor) -> bool:
+    """The fused norm + rotation kernel takes these operands: bf16 rows and gains, a head width it is built for, 16-byte alignment."""
+    return (_is_kernel_tensor(qkv) and d in (32, 64, 128, 256) and qkv.dim() == 2 and qkv.stride(1) == 1 and qkv.stride(0) % 8 == 0
+            and all(g.dtype == torch.bfloat16 and g.is_contiguous() and g.numel() == d for g in (q_norm, k_norm))
+            and all(t.is_contiguous() and t.dtype == torch.float32 and t.shape[-1] == d // 2 for t in (cos, sin))
+            and all(t.is_cuda and t.data_ptr() % 16 == 0 for t in (qkv, cos, sin, q_norm, k_norm)))
+
+
+def head_norm_rope_and_cache_(qkv, pos, cos, sin, nq, nkv, d, q_norm, k_norm, eps, k_cache, v_cache, slot_mapping, page: int = 16):
+    """Inference: RMS norm of every query and key head, rotation and append to the paged cache in one kernel, in place on ``qkv``
+    (operands as ``head_norm_ok`` says)."""
+    _C().qk_norm_rope_(qkv, pos, cos, sin, nq, nkv, d, q_norm, k_norm, eps, None, k_cache, v_cache, slot_mapping, page)
+    return qkv
+
+
 def gather_cached(k_cache: torch.Tensor, v_cache: torch.Tensor, blk: torch.Tensor, off: torch.Tensor):
     """Keys and values [T, nkv, d] at the places (page ``blk[t]``, row ``off[t]``) of caches [pages, nkv, page, d]."""
     if all(_is_kernel_tensor(c) and c.dim() == 4 and c.is_contiguous() and c.shape[3] % 8 == 0 and c.data_ptr() % 16 == 0 for c in (k_cache, v_cache)) \

@@ -45,3 +45,79 @@ def test_rmsnorm_residual(t, h, res):
         err = (got.double() - want).abs()
         assert (err <= 2.0 ** -8 * want.abs() + 1e-4 * want.abs().max()).all(), err.max()
     assert torch.equal(torch.autograd.grad(ops.rmsnorm(x, w, 1e-6), w, gy)[0], dw)          # the partial sums have a fixed order
+
+
+def _rope64(x, pos, cos, sin):
+    c, s = cos[pos].double()[:, None], sin[pos].double()[:, None]
+    lo, hi = x.chunk(2, -1)
+    return torch.cat([lo * c - hi * s, hi * c + lo * s], -1)
+
+
+def _heads64(qkv, pos, cos, sin, nq, nkv, d, qn, kn, eps):
+    p = qkv.double().view(-1, nq + 2 * nkv, d)
+    q, k, v = p[:, :nq], p[:, nq:nq + nkv], p[:, nq + nkv:]
+    if qn is not None:
+        q = q * torch.rsqrt(q.pow(2).mean(-1, keepdim=True) + eps) * qn.double()
+        k = k * torch.rsqrt(k.pow(2).mean(-1, keepdim=True) + eps) * kn.double()
+    return _rope64(q, pos, cos, sin), _rope64(k, pos, cos, sin), v
+
+
+@pytest.mark.parametrize("d,nq,nkv", [(32, 3, 1), (64, 14, 2), (128, 8, 2), (256, 2, 2), (48, 2, 1)])
+@pytest.mark.parametrize("norm", [False, True])
+def test_norm_rope_and_cache(d, nq, nkv, norm):
+    """One rounding to bf16 of a value computed in fp32; places without a slot leave the cache as it is.  Widths other than the kernel's
+    (48 here) keep the general rotation."""
+    if norm and d == 48:
+        pytest.skip("the norm kernel is not built for this width")
+    t, page, pages = 37, 16, 6
+    qkv = _randn(t, (nq + 2 * nkv) * d, seed=1)
+    cos, sin = (f.cuda() for f in OF.ref.rope_tables(64, d, 1e4))
+    pos = (torch.arange(t) * 7 % 64).cuda()
+    slots = torch.randperm(page * pages, generator=torch.Generator().manual_seed(0))[:t].cuda()
+    slots[5] = -1
+    kc, vc = _randn(pages, nkv, page, d, seed=2), _randn(pages, nkv, page, d, seed=3)
+    qn, kn = (_randn(d, seed=4, scale=0.1, shift=1.0), _randn(d, seed=5, scale=0.1, shift=1.0)) if norm else (None, None)
+    q, k, v = _heads64(qkv, pos, cos, sin, nq, nkv, d, qn, kn, 1e-6)
+    wk, wv, ok = kc.double(), vc.double(), slots >= 0
+    wk[slots[ok] // page, :, slots[ok] % page], wv[slots[ok] // page, :, slots[ok] % page] = k[ok], v[ok]
+    if norm:
+        OF.head_norm_rope_and_cache_(qkv, pos, cos, sin, nq, nkv, d, qn, kn, 1e-6, kc, vc, slots, page)
+    else:
+        OF.rope_and_cache_(qkv, pos, cos, sin, nq, nkv, d, kc, vc, slots, page)
+    for got, want in ((qkv.view(t, -1, d), torch.cat([q, k, v], 1)), (kc, wk), (vc, wv)):
+        assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()
+
+
+@pytest.mark.parametrize("nq,nkv,lens", [(4, 4, [1]), (8, 2, [128, 1, 129]), (6, 2, [77, 300, 5])])
+@pytest.mark.parametrize("norm", [False, True])
+def test_rope_attention(nq, nkv, lens, norm):
+    """Norm, rotation and attention as one function against autograd in 64 bits: probabilities and their gradients pass through bf16 on
+    their way into the products, so 2e-2 of the norm.  A lone token has no gradient but the difference of two fp32 sums of 128 products,
+    128 * 2^-24 * 128^-0.5 < 7e-7 an element of the 512 that a gain sums: 2e-5."""
+    from polyrl_b200.ops.attention import rope_attention
+
+    d, t = 128, sum(lens)
+    qkv = _randn(t, (nq + 2 * nkv) * d, seed=1)
+    cos, sin = (f.cuda() for f in OF.ref.rope_tables(512, d, 1e4))
+    pos = torch.cat([torch.arange(n) for n in lens]).cuda()
+    cu = torch.tensor([0] + lens, dtype=torch.int32).cumsum(0).to(torch.int32).cuda()
+    qn, kn = (_randn(d, seed=4, scale=0.1, shift=1.0), _randn(d, seed=5, scale=0.1, shift=1.0)) if norm else (None, None)
+    go = _randn(t, nq, d, seed=6)
+    leaves = [qkv.double().requires_grad_(True)] + ([g.double().requires_grad_(True) for g in (qn, kn)] if norm else [])
+    q, k, v = _heads64(leaves[0], pos, cos, sin, nq, nkv, d, *(leaves[1:] if norm else (None, None)), 1e-6)
+    outs = []
+    for a, b, c in zip(q.split(lens), k.split(lens), v.split(lens)):
+        b, c = b.repeat_interleave(nq // nkv, 1), c.repeat_interleave(nq // nkv, 1)
+        z = torch.einsum("qhd,khd->hqk", a, b) * d ** -0.5
+        z = z.masked_fill(torch.ones(z.shape[-2:], dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+        outs.append(torch.einsum("hqk,khd->qhd", z.softmax(-1), c))
+    want = torch.cat(outs)
+    wants = [want, *torch.autograd.grad(want, leaves, go.double())]
+    with torch.no_grad():
+        plain = rope_attention(qkv.clone(), pos, cos, sin, nq, nkv, d, cu, qn, kn)
+    mine = [qkv.clone().requires_grad_(True)] + ([g.clone().requires_grad_(True) for g in (qn, kn)] if norm else [])
+    got = rope_attention(mine[0] * 1.0, pos, cos, sin, nq, nkv, d, cu, *(mine[1:] if norm else (None, None)))
+    assert torch.equal(plain, got)
+    for a, b in zip([got, *torch.autograd.grad(got, mine, go)], wants):
+        assert (a.double() - b).norm() <= 2e-2 * b.norm() + 2e-5
+    assert rope_attention(qkv[:, : (nq + 2 * nkv) * d - 8], pos, cos, sin, nq, nkv, d, cu) is None        # not the rows it is made for
