@@ -17,11 +17,11 @@
 // receives its 128 accumulator rows.  Halving the per-SM B traffic is what lifts the kernel off
 // the shared-memory bandwidth limit of the 1-CTA 128x256 tile (gemm_sm100.cuh).
 //
-// Warp roles per CTA (192 threads): warp 0 TMA producer (both CTAs, completion bytes counted on the
-// LEADER's full barrier), warp 1 TMEM allocator + (leader only) MMA issuer, warps 2..5 epilogue.
+// Warp roles per CTA (192 threads with one epilogue group): warp 0 TMA producer (both CTAs, completion bytes counted on the
+// LEADER's full barrier), warp 1 TMEM allocator + (leader only) MMA issuer, warps 2..5 (2..9) epilogue.
 // Barriers: full[s] leader-only (count 1, expect 2 x stage bytes); empty[s] and tmem_full[a] per
-// CTA, signalled by multicast `tcgen05.commit`; tmem_empty[a] on the leader, 8 remote arrivals
-// (one elected lane per epilogue warp of both CTAs).
+// CTA, signalled by multicast `tcgen05.commit`; tmem_empty[a] on the leader, one remote arrival per epilogue warp
+// (an elected lane per epilogue warp of both CTAs).
 //
 // Epilogues: (a) functor mode — same `Epi` interface as gemm_sm100.cuh (SwiGLU, linear-CE, ...);
 // (b) TMA-store mode — accumulators -> bf16 -> 128B-swizzled shared staging -> `cp.async.bulk.tensor`
@@ -34,8 +34,13 @@ namespace prl {
 
 constexpr int kSmemMax = 232448;   // 227 KB opt-in limit per CTA
 
-template <int BN, bool A_MN_, bool B_MN_, bool TMA_STORE_>
+// EPI_GROUPS: warpgroups that share a tile's columns in the epilogue.  One is enough where the epilogue converts and stores; an epilogue
+// that takes an exponential per element gets two, because a warp per scheduler cannot hide its latencies and short reductions
+// (K of about a thousand) leave it no time: the figures are beside its users.
+template <int BN, bool A_MN_, bool B_MN_, bool TMA_STORE_, int EPI_GROUPS_ = 1>
 struct Gemm2Cfg {
+  static constexpr int EPI_GROUPS = EPI_GROUPS_, EPI_WARPS = 4 * EPI_GROUPS, THREADS = 64 + 32 * EPI_WARPS;
+  static constexpr int GROUP_N = BN / EPI_GROUPS;     // columns of a group
   static constexpr bool A_MN = A_MN_, B_MN = B_MN_, TMA_STORE = TMA_STORE_;
   static constexpr int BLOCK_M = 256;                 // per CTA pair
   static constexpr int CTA_M = 128;
@@ -45,7 +50,7 @@ struct Gemm2Cfg {
   static constexpr int A_BYTES = CTA_M * 128;
   static constexpr int B_BYTES = CTA_N * 128;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int EPI_BYTES = TMA_STORE ? 4 * 2 * 4096 : 0;
+  static constexpr int EPI_BYTES = TMA_STORE ? EPI_WARPS * 2 * 4096 : 0;
   static constexpr int STAGES_RAW = (kSmemMax - 1024 - 512 - EPI_BYTES) / STAGE_BYTES;
   static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
   static constexpr int TMEM_COLS = 2 * BN;            // 256 or 512
@@ -61,15 +66,18 @@ struct TmaStoreParams {
 };
 struct EpiTmaStore {
   using Params = TmaStoreParams;
+  static constexpr bool kRow = false;   // true: a functor with per-row state, begin(params, row, M) and apply(params, r[64], column)
   static constexpr int kAct = 0;
 };
 // same with gelu (tanh form) on the accumulators, in the exactly equivalent shape z * sigmoid(2 u)
 struct EpiTmaStoreGelu {
   using Params = TmaStoreParams;
+  static constexpr bool kRow = false;
   static constexpr int kAct = 1;
 };
 struct EpiTmaStoreSilu {
   using Params = TmaStoreParams;
+  static constexpr bool kRow = false;
   static constexpr int kAct = 2;
 };
 __device__ __forceinline__ float gelu_fast(float z) {
@@ -78,7 +86,7 @@ __device__ __forceinline__ float gelu_fast(float z) {
 __device__ __forceinline__ float silu_fast(float z) { return __fdividef(z, 1.0f + __expf(fminf(-z, 80.f))); }
 
 template <class Cfg, class Epi>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Cfg::THREADS, 1)
 gemm2_sm100_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const __grid_constant__ CUtensorMap tmD, typename Epi::Params ep, int M, int N, int K,
                    int num_m_blocks, int num_n_blocks, int n_splits, int nb_per_split, Sched sc) {
@@ -114,7 +122,7 @@ gemm2_sm100_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tmem_full[i], 1);
-      mbar_init(&tmem_empty[i], 8);
+      mbar_init(&tmem_empty[i], 2 * Cfg::EPI_WARPS);
     }
     fence_barrier_init();
   }
@@ -201,24 +209,27 @@ gemm2_sm100_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   } else {
     // ================================ epilogue (both CTAs) ====================================
     const int quad = warp & 3;                       // TMEM lane quadrant this warp may read
+    const int group = (warp - 2) >> 2;               // which columns of the tile are its own
     const int row_in_tile = static_cast<int>(rank) * Cfg::CTA_M + quad * 32 + lane;
     uint32_t tile_iter = 0;
     if constexpr (Cfg::TMA_STORE) {
       uint8_t* ebuf = smem_epi + (warp - 2) * 8192;
+      [[maybe_unused]] Epi epi;
       uint32_t chunk_ctr = 0;
       for (int w = cluster_id; w < total_work; w += num_clusters) {
         const WorkInfo wi = decode_work(w, num_m_blocks, num_n_blocks, n_splits, nb_per_split, sc);
         const int row = wi.m_blk * Cfg::BLOCK_M + row_in_tile;
         const int row0 = row - lane;
+        if constexpr (Epi::kRow) epi.begin(ep, row, M);
         for (int nb = wi.n_begin; nb < wi.n_end; ++nb, ++tile_iter) {
           const uint32_t as = tile_iter & 1;
           const uint32_t aphase = (tile_iter >> 1) & 1;
-          const int n0 = rot_n(nb, num_n_blocks, sc) * BN;
+          const int n0 = rot_n(nb, num_n_blocks, sc) * BN + group * Cfg::GROUP_N;
           mbar_wait(&tmem_full[as], aphase);
           tc_fence_after();
-          const uint32_t taddr = tmem_base + as * BN + (static_cast<uint32_t>(quad * 32) << 16);
+          const uint32_t taddr = tmem_base + as * BN + group * Cfg::GROUP_N + (static_cast<uint32_t>(quad * 32) << 16);
 #pragma unroll 1
-          for (int c = 0; c < BN / 64; ++c, ++chunk_ctr) {
+          for (int c = 0; c < Cfg::GROUP_N / 64; ++c, ++chunk_ctr) {
             uint8_t* buf = ebuf + (chunk_ctr & 1) * 4096;
             if (lane == 0) tma_store_wait_read<1>();   // the store that last read `buf` has drained it
             __syncwarp();
@@ -226,12 +237,15 @@ gemm2_sm100_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
             tmem_ld_32x32(taddr + c * 64, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
             tmem_ld_32x32(taddr + c * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
             tmem_ld_wait();
-            if (c == BN / 64 - 1) {                     // accumulator fully read: hand TMEM back early
+            if (c == Cfg::GROUP_N / 64 - 1) {                     // accumulator fully read: hand TMEM back early
               tc_fence_before();
               __syncwarp();
               if (lane == 0) mbar_arrive_cluster(&tmem_empty[as], 0);
             }
             const int col0 = n0 + c * 64;
+            if constexpr (Epi::kRow) {
+              epi.apply(ep, r, col0);
+            } else {
             if (ep.R != nullptr && row < M) {
               const __nv_bfloat16* rp = ep.R + static_cast<int64_t>(row) * ep.ldr + col0;
 #pragma unroll
@@ -254,6 +268,7 @@ gemm2_sm100_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 #pragma unroll
               for (int j = 0; j < 64; ++j)
                 r[j] = __float_as_uint(Epi::kAct == 1 ? gelu_fast(__uint_as_float(r[j])) : silu_fast(__uint_as_float(r[j])));
+            }
             }
             // row `lane` of the 32 x 64 box: 8 x 16 B chunks, chunk j lands at (j ^ (lane & 7)) (128B swizzle)
             const uint32_t row_base = smem_u32(buf) + lane * 128;
@@ -280,16 +295,17 @@ gemm2_sm100_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     } else {
       Epi epi;
       for (int w = cluster_id; w < total_work; w += num_clusters) {
-        const WorkInfo wi = decode_work(w, num_m_blocks, num_n_blocks, n_splits, nb_per_split, sc);
+        WorkInfo wi = decode_work(w, num_m_blocks, num_n_blocks, n_splits, nb_per_split, sc);
         const int row = wi.m_blk * Cfg::BLOCK_M + row_in_tile;
+        wi.split = wi.split * Cfg::EPI_GROUPS + group;       // each group carries running state of its own
         epi.begin(ep, row, M, wi);
         for (int nb = wi.n_begin; nb < wi.n_end; ++nb, ++tile_iter) {
           const uint32_t as = tile_iter & 1;
           const uint32_t aphase = (tile_iter >> 1) & 1;
           mbar_wait(&tmem_full[as], aphase);
           tc_fence_after();
-          AccReader acc{tmem_base + as * BN + (static_cast<uint32_t>(quad * 32) << 16)};
-          epi.template tile<BN>(ep, acc, row, M, rot_n(nb, num_n_blocks, sc) * BN, N);
+          AccReader acc{tmem_base + as * BN + group * Cfg::GROUP_N + (static_cast<uint32_t>(quad * 32) << 16)};
+          epi.template tile<Cfg::GROUP_N>(ep, acc, row, M, rot_n(nb, num_n_blocks, sc) * BN + group * Cfg::GROUP_N, N);
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster(&tmem_empty[as], 0);
@@ -340,7 +356,7 @@ int launch_gemm2(const void* A, const void* B, void* D, int M, int N, int K, int
   int clusters = sm_count() / 2;
   const int total = num_m_blocks * n_splits;
   if (total < clusters) clusters = total;
-  kern<<<2 * clusters, kNumThreads, Cfg::SMEM_BYTES, stream>>>(tmA, tmB, tmD, ep, M, N, K, num_m_blocks, num_n_blocks,
+  kern<<<2 * clusters, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(tmA, tmB, tmD, ep, M, N, K, num_m_blocks, num_n_blocks,
                                                                n_splits, nb_per_split, sc);
   PRL_CUDA_CHECK(cudaGetLastError());
   return 0;

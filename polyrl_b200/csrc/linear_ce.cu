@@ -43,18 +43,30 @@ struct EpiCeFwd {
       if (valid <= 0) continue;
       float cmax = -INFINITY;
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        v[i] = (i < valid) ? v[i] * scale2 : -INFINITY;   // base-2 scaled logits
-        cmax = fmaxf(cmax, v[i]);
-      }
-      const float nm = fmaxf(m2, cmax);
-      const float resc = exp2f(m2 - nm);                  // m2 = -inf -> 0
-      float ls = 0.f, lb = 0.f;
+      for (int i = 0; i < 32; ++i) v[i] *= scale2;        // base-2 scaled logits
+      if (valid < 32) {
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const float e = exp2f(v[i] - nm);                 // masked cols: 2^-inf = 0
-        ls += e;
-        lb += (i < valid) ? v[i] * e : 0.f;
+        for (int i = 0; i < 32; ++i) v[i] = (i < valid) ? v[i] : -INFINITY;
+      }
+#pragma unroll
+      for (int i = 0; i < 32; ++i) cmax = fmaxf(cmax, v[i]);
+      const float nm = fmaxf(m2, cmax);
+      const float resc = fast_exp2(m2 - nm);              // m2 = -inf -> 0
+      float ls = 0.f, lb = 0.f;
+      if (valid < 32) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          const float e = fast_exp2(v[i] - nm);           // masked cols: 2^-inf = 0
+          ls += e;
+          lb += (i < valid) ? v[i] * e : 0.f;
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          const float e = fast_exp2(v[i] - nm);
+          ls += e;
+          lb += v[i] * e;
+        }
       }
       s = s * resc + ls;
       b = b * resc + lb;
@@ -118,18 +130,51 @@ struct CeBwdParams {
   __nv_bfloat16* DZ;     // [T, lddz]
   int64_t lddz;
 };
-struct EpiCeBwd {
-  using Params = CeBwdParams;
-  float lse2, ezv, glp, gent;
+// With t = z log2 e - lse2 and p = 2^t the slice is  -p (A + B z)  and, at the label, + inv_tau g_lp:  A = inv_tau (g_lp - g_ent E[z]),
+// B = inv_tau g_ent.  Two multiply-adds, an exponential and a product an element; the bf16 rows leave through shared memory and TMA.
+struct CeBwdRow {
+  float lse2, a, b, hot;
   int64_t label;
-  __device__ __forceinline__ void begin(const Params& p, int row, int M, const WorkInfo&) {
+  __device__ __forceinline__ void begin(const CeBwdParams& p, int row, int M) {
     const bool ok = row < M;
+    const float glp = (ok && p.g_lp) ? p.g_lp[row] : 0.f, gent = (ok && p.g_ent) ? p.g_ent[row] : 0.f;
     lse2 = ok ? p.lse[row] * kLog2e : 0.f;
-    ezv = ok ? p.ez[row] : 0.f;
-    glp = (ok && p.g_lp) ? p.g_lp[row] : 0.f;
-    gent = (ok && p.g_ent) ? p.g_ent[row] : 0.f;
+    a = p.inv_tau * (glp - gent * (ok ? p.ez[row] : 0.f));
+    b = p.inv_tau * (gent * p.inv_tau);            // on the accumulator, z = acc inv_tau
+    hot = p.inv_tau * glp;
     label = ok ? p.labels[row] - p.v0 : -1;
   }
+  template <int NV>
+  __device__ __forceinline__ void values(const CeBwdParams& p, float (&v)[NV], int col) const {
+    const float scale2 = p.inv_tau * kLog2e;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) v[i] = -fast_exp2(v[i] * scale2 - lse2) * (a + b * v[i]);
+    const int64_t rel = label - col;
+    if (rel >= 0 && rel < NV) {
+#pragma unroll
+      for (int i = 0; i < NV; ++i) v[i] += i == rel ? hot : 0.f;
+    }
+  }
+};
+// CTA-pair kernel: 64 columns at a time, staged for TMA
+struct EpiCeBwdStore : CeBwdRow {
+  using Params = CeBwdParams;
+  static constexpr bool kRow = true;
+  static constexpr int kAct = 0;
+  __device__ __forceinline__ void apply(const Params& p, uint32_t (&r)[64], int col) const {
+    float v[64];
+#pragma unroll
+    for (int i = 0; i < 64; ++i) v[i] = __uint_as_float(r[i]);
+    values(p, v, col);
+#pragma unroll
+    for (int i = 0; i < 64; ++i) r[i] = __float_as_uint(v[i]);
+  }
+};
+// one-CTA kernel (up to 128 rows): direct stores
+struct EpiCeBwd {
+  using Params = CeBwdParams;
+  CeBwdRow r;
+  __device__ __forceinline__ void begin(const Params& p, int row, int M, const WorkInfo&) { r.begin(p, row, M); }
   __device__ __forceinline__ void end(const Params&, int, int, const WorkInfo&) {}
   template <int BN>
   __device__ __forceinline__ void tile(const Params& p, const AccReader& acc, int row, int M, int n0, int N) {
@@ -140,13 +185,7 @@ struct EpiCeBwd {
       const int col = n0 + c;
       const int valid = min(32, N - col);
       if (row >= M || valid <= 0) continue;
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const float z = v[i] * p.inv_tau;
-        const float pr = exp2f(z * kLog2e - lse2);
-        const float onehot = (static_cast<int64_t>(col + i) == label) ? 1.f : 0.f;
-        v[i] = p.inv_tau * (glp * (onehot - pr) - gent * pr * (z - ezv));
-      }
+      r.values(p, v, col);
       __nv_bfloat16* dst = p.DZ + static_cast<int64_t>(row) * p.lddz + col;
       if (valid >= 32) {
 #pragma unroll
@@ -159,7 +198,9 @@ struct EpiCeBwd {
           st_v4(dst + 8 * i, o);
         }
       } else {
-        for (int i = 0; i < valid; ++i) dst[i] = __float2bfloat16(v[i]);
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+          if (i < valid) dst[i] = __float2bfloat16(v[i]);
       }
     }
   }
@@ -169,17 +210,26 @@ struct EpiCeBwd {
 
 using namespace prl;
 
-extern "C" int prl_linear_ce_num_splits(int T, int V) {
-  // T > 128 runs on the CTA-pair kernel: 256-row m-blocks, one work item per SM PAIR
-  const int mb = T > kBlockM ? (T + 255) / 256 : 1;
-  const int nb = (V + 255) / 256;
+// How many runs of n-blocks a row's vocabulary is cut into: a run is one work item of an SM (pair), so with mb m-blocks the pass takes
+// ceil(mb runs / workers) rounds of ceil(nb / runs) tiles.  The cut with the fewest tiles in a row wins, the smaller one if equal.
+// (About two items a worker, whatever the remainder, left the last round nearly empty: 168 items on 74 pairs at 6005 x 128256, K 4096, 5540 us; now 144, 4170 us.)
+static int ce_runs(int T, int V) {
+  const int mb = T > kBlockM ? (T + 255) / 256 : 1, nb = (V + 255) / 256;
   const int workers = T > kBlockM ? sm_count() / 2 : sm_count();
-  int s = (2 * workers + mb - 1) / mb;   // ~2 waves of work items
-  if (s < 1) s = 1;
-  if (s > nb) s = nb;
-  const int per = (nb + s - 1) / s;
-  return (nb + per - 1) / per;
+  int best = 1;
+  int64_t best_cost = INT64_MAX;
+  for (int s = 1; s <= nb && (s == 1 || static_cast<int64_t>(mb) * s <= 16ll * workers); ++s) {
+    const int per = (nb + s - 1) / s, runs = (nb + per - 1) / per;
+    const int64_t cost = (static_cast<int64_t>(mb) * runs + workers - 1) / workers * per;
+    if (cost < best_cost) { best_cost = cost; best = runs; }
+  }
+  return best;
 }
+// Epilogue groups of the pair kernel, each with statistics of its own.  At K = 896 a tile's products take 7200 cycles and one group's
+// exponentials longer: with two, 2503 x 151936 forward 891 -> 454 us (the cut above is part of it), gradients of the logits 951 -> 575 us.
+constexpr int kCeGroups = 2;
+// partial statistics a row
+extern "C" int prl_linear_ce_num_splits(int T, int V) { return ce_runs(T, V) * (T > kBlockM ? kCeGroups : 1); }
 
 // hidden:[T,H] bf16, W:[V,H] bf16, labels:[T] int64 -> logprob/entropy/lse/ez:[T] fp32.
 // scratch: 3*T*S + T floats.
@@ -196,9 +246,9 @@ extern "C" int prl_linear_ce_fwd(const void* hidden, const void* W, const int64_
   p.label_logit = scratch + 3 * static_cast<int64_t>(T) * S;
   p.S = S;
   using Cfg = GemmCfg<256, 2>;
-  using Cfg2 = Gemm2Cfg<256, false, false, false>;
+  using Cfg2 = Gemm2Cfg<256, false, false, false, kCeGroups>;
   int rc = T > kBlockM
-               ? launch_gemm2<Cfg2, EpiCeFwd>(hidden, W, nullptr, T, V, H, ldh * 2, ldw * 2, 0, p, S, stream)
+               ? launch_gemm2<Cfg2, EpiCeFwd>(hidden, W, nullptr, T, V, H, ldh * 2, ldw * 2, 0, p, S / kCeGroups, stream)
                : launch_gemm<Cfg, EpiCeFwd, NoGate, false>(hidden, W, T, V, H, ldh * 2, ldw * 2, p, NoGate::Params{}, S, 0,
                                                            stream);
   if (rc) return rc;
@@ -214,8 +264,8 @@ extern "C" int prl_linear_ce_dz(const void* hidden, const void* W_slice, const i
                                 int H, int v0, int64_t ldh, int64_t ldw, void* DZ, int64_t lddz, cudaStream_t stream) {
   CeBwdParams p{labels, lse, ez, g_lp, g_ent, inv_tau, v0, static_cast<__nv_bfloat16*>(DZ), lddz};
   using Cfg = GemmCfg<256, 2>;
-  using Cfg2 = Gemm2Cfg<256, false, false, false>;
-  if (T > kBlockM) return launch_gemm2<Cfg2, EpiCeBwd>(hidden, W_slice, nullptr, T, Vc, H, ldh * 2, ldw * 2, 0, p, 0, stream);
+  using Cfg2 = Gemm2Cfg<256, false, false, true, kCeGroups>;
+  if (T > kBlockM) return launch_gemm2<Cfg2, EpiCeBwdStore>(hidden, W_slice, DZ, T, Vc, H, ldh * 2, ldw * 2, lddz * 2, p, 0, stream);
   return launch_gemm<Cfg, EpiCeBwd, NoGate, false>(hidden, W_slice, T, Vc, H, ldh * 2, ldw * 2, p, NoGate::Params{}, 0,
                                                    0, stream);
 }

@@ -121,3 +121,22 @@ def test_rope_attention(nq, nkv, lens, norm):
     for a, b in zip([got, *torch.autograd.grad(got, mine, go)], wants):
         assert (a.double() - b).norm() <= 2e-2 * b.norm() + 2e-5
     assert rope_attention(qkv[:, : (nq + 2 * nkv) * d - 8], pos, cos, sin, nq, nkv, d, cu) is None        # not the rows it is made for
+
+
+@pytest.mark.parametrize("t,v,h", [(1, 264, 64), (128, 392, 64), (129, 392, 128), (300, 640, 64), (515, 5000, 896)])
+@pytest.mark.parametrize("tau", [1.0, 0.7])
+def test_linear_ce_edges(t, v, h, tau):
+    """Labels at the edges of tiles and of the epilogue groups' halves, vocabularies that end in either half.  Statistics are fp32 sums over
+    at most 5000 columns and products over 896 (1e-5); the gradient of the logits is rounded to bf16 on its way into the products (1e-2)."""
+    x, w = _randn(t, h, seed=1).requires_grad_(True), _randn(v, h, seed=2, scale=0.1).requires_grad_(True)
+    edges = [e for e in (0, 31, 32, 63, 64, 127, 128, 191, 255, 256, 383, 384, v - 1) if e < v]
+    lab = torch.tensor([edges[i % len(edges)] for i in range(t)]).cuda()
+    glp, gent = _randn(t, seed=3, dtype=torch.float32), _randn(t, seed=4, dtype=torch.float32)
+    lp, ent = ops.linear_cross_entropy(x, w, lab, tau)
+    got = [lp, ent, *torch.autograd.grad([lp, ent], [x, w], [glp, gent])]
+    x64, w64 = x.detach().double().requires_grad_(True), w.detach().double().requires_grad_(True)
+    logp = (x64 @ w64.t() / tau).log_softmax(-1)
+    lp64, ent64 = logp.gather(1, lab[:, None])[:, 0], -(logp.exp() * logp).sum(-1)
+    want = [lp64, ent64, *torch.autograd.grad([lp64, ent64], [x64, w64], [glp.double(), gent.double()])]
+    for a, b, tol in zip(got, want, (1e-5, 1e-5, 1e-2, 1e-2)):
+        assert (a.double() - b).norm() <= tol * b.norm()
