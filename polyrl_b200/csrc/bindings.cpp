@@ -8,8 +8,9 @@
 #include <vector>
 
 extern "C" {
-int prl_gemm2_bf16(const void*, const void*, void*, const void*, int, int, int, int64_t, int64_t, int64_t, int, int, int, cudaStream_t);
-int prl_gemm2_bf16_accum_f32(const void*, const void*, float*, float, int, int, int, int64_t, int64_t, int64_t, int, int, cudaStream_t);
+int prl_gemm2_bf16(const void*, const void*, void*, const void*, int, int, int, int64_t, int64_t, int64_t, int64_t, int, int, int, float*, cudaStream_t);
+int64_t prl_gemm2_ws_floats(int, int, int);
+int prl_gemm2_bf16_accum_f32(const void*, const void*, float*, float, int, int, int, int64_t, int64_t, int64_t, int, int, float*, cudaStream_t);
 int prl_gemm_fp8(const void*, const void*, void*, const float*, const float*, int, int, int, int64_t, int64_t, int64_t, int, cudaStream_t);
 int prl_linear_ce_num_splits(int, int);
 int prl_linear_ce_fwd(const void*, const void*, const int64_t*, float, int, int, int, int64_t, int64_t, float*, int, float*, float*, float*, float*, cudaStream_t);
@@ -102,8 +103,9 @@ at::Tensor gemm2_bf16(const at::Tensor& a, const at::Tensor& b, bool a_mn, bool 
     r = residual->data_ptr();
   }
   TORCH_CHECK(a.stride(0) >= a.size(1) && b.stride(0) >= b.size(1), "gemm2_bf16: row pitch shorter than the row");
-  const int rc = prl_gemm2_bf16(a.data_ptr(), b.data_ptr(), d.data_ptr(), r, M, N, K, a.stride(0), b.stride(0), d.stride(0),
-                                a_mn ? 1 : 0, b_mn ? 1 : 0, static_cast<int>(force_bn), cur_stream());
+  const at::Tensor ws = split_scratch(prl_gemm2_ws_floats(M, N, K), a);
+  const int rc = prl_gemm2_bf16(a.data_ptr(), b.data_ptr(), d.data_ptr(), r, M, N, K, a.stride(0), b.stride(0), d.stride(0), d.stride(0),
+                                a_mn ? 1 : 0, b_mn ? 1 : 0, static_cast<int>(force_bn), split_ptr(ws), cur_stream());
   TORCH_CHECK(rc == 0, "polyrl_b200 kernel 'gemm2_bf16' failed with code ", rc, " (M=", M, " N=", N, " K=", K, " a_mn=", a_mn,
               " b_mn=", b_mn, " lda=", a.stride(0), " ldb=", b.stride(0), " ldd=", d.stride(0), " a=", a.data_ptr(), " b=",
               b.data_ptr(), " dev=", a.get_device(), ")");
@@ -118,8 +120,9 @@ void gemm2_accum_f32_(at::Tensor out32, const at::Tensor& a, const at::Tensor& b
   TORCH_CHECK(K == Kb && out32.dim() == 2 && out32.size(0) == M && out32.size(1) == N);
   TORCH_CHECK(a.size(1) % 8 == 0 && b.size(1) % 8 == 0 && a.stride(0) % 8 == 0 && b.stride(0) % 8 == 0 && out32.stride(0) % 4 == 0);
   c10::cuda::CUDAGuard g(a.device());
+  const at::Tensor ws = split_scratch(N % 4 == 0 ? prl_gemm2_ws_floats(M, N, K) : 0, a);       // (slots are finished four columns at a time)
   check(prl_gemm2_bf16_accum_f32(a.data_ptr(), b.data_ptr(), out32.data_ptr<float>(), static_cast<float>(beta), M, N, K,
-                                 a.stride(0), b.stride(0), out32.stride(0), a_mn ? 1 : 0, b_mn ? 1 : 0, cur_stream()),
+                                 a.stride(0), b.stride(0), out32.stride(0), a_mn ? 1 : 0, b_mn ? 1 : 0, split_ptr(ws), cur_stream()),
         "gemm2_accum_f32");
 }
 

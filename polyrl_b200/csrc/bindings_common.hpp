@@ -19,4 +19,10 @@ inline void check(int rc, const char* what) {
 #define CHECK_F32(t) TORCH_CHECK((t).is_cuda() && (t).scalar_type() == at::kFloat, #t " must be a CUDA fp32 tensor")
 #define CHECK_LASTDIM(t) TORCH_CHECK((t).stride(-1) == 1, #t " must be contiguous in the last dim")
 
+// scratch of a product whose last round of tiles is cut along the reduction (gemm2_sm100.cuh); nothing when it is not
+inline at::Tensor split_scratch(int64_t floats, const at::Tensor& like) {
+  return floats > 0 ? at::empty({floats}, like.options().dtype(at::kFloat)) : at::Tensor();
+}
+inline float* split_ptr(const at::Tensor& ws) { return ws.defined() ? ws.data_ptr<float>() : nullptr; }
+
 }  // namespace

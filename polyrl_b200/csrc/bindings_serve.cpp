@@ -6,14 +6,15 @@
 #include "scheduler.hpp"
 
 extern "C" {
-int prl_gemm_bf16(const void*, const void*, void*, const void*, int, int, int, int64_t, int64_t, int64_t, int, cudaStream_t);
+int prl_gemm_bf16(const void*, const void*, void*, const void*, int, int, int, int64_t, int64_t, int64_t, int64_t, int, float*, cudaStream_t);
+int64_t prl_gemm2_ws_floats(int, int, int);
 int prl_sample(const void*, int, int64_t, int, int, const float*, int, const uint64_t*, int, int64_t*, float*, cudaStream_t);
 int prl_sample_topk_topp(const void*, int, int64_t, int, int, const float*, int, const uint64_t*, int, int, float, int64_t*, float*, cudaStream_t);
 int prl_attn_fwd(const void*, const void*, const void*, void*, float*, const int32_t*, const int32_t*, int, int, int, int, int, int, int, int64_t, int64_t, int64_t, int64_t, float, int, int, const float*, int, int, long long*, cudaStream_t);
 int prl_paged_decode_workspace_floats(int, int, int, int);
 int prl_paged_decode(const void*, int64_t, const void*, const void*, const int32_t*, int64_t, const int32_t*, int, int, int, int, float, int, int, int, float*, void*, int64_t, cudaStream_t);
 int prl_gemm_clamped_glu_bf16(const void*, const void*, void*, int, int, int, int64_t, int64_t, int64_t, float, float, cudaStream_t);
-int prl_gemm_swiglu_bf16(const void*, const void*, void*, void*, int, int, int, int64_t, int64_t, int64_t, int64_t, cudaStream_t);
+int prl_gemm_swiglu_bf16(const void*, const void*, void*, void*, int, int, int, int64_t, int64_t, int64_t, int64_t, float*, cudaStream_t);
 int prl_gemm_experts_bf16(const void*, const void*, void*, const int32_t*, int, int, int, int, int, float, float, cudaStream_t);
 int prl_sink_decode(const void*, const void*, const void*, const int32_t*, int64_t, const int32_t*, int, int, int, int, int, float, int, const float*, float*, void*, cudaStream_t);
 int prl_map_attn_fwd(const void*, const void*, const void*, void*, const int32_t*, const int32_t*, int, int, int, int, int, int, int, int, int, float, int, const float*, float, float, int, cudaStream_t);
@@ -88,8 +89,9 @@ at::Tensor gemm_bf16(const at::Tensor& a, const at::Tensor& b, const c10::option
     TORCH_CHECK(residual->sizes() == d.sizes() && residual->stride(0) == d.stride(0) && residual->stride(1) == 1);
     r = residual->data_ptr();
   }
-  check(prl_gemm_bf16(a.data_ptr(), b.data_ptr(), d.data_ptr(), r, M, N, K, a.stride(0), b.stride(0), d.stride(0),
-                      static_cast<int>(force_bn), cur_stream()), "gemm_bf16");
+  const at::Tensor ws = split_scratch(M > 128 && force_bn == 0 ? prl_gemm2_ws_floats(M, N, K) : 0, a);
+  check(prl_gemm_bf16(a.data_ptr(), b.data_ptr(), d.data_ptr(), r, M, N, K, a.stride(0), b.stride(0), d.stride(0), d.stride(0),
+                      static_cast<int>(force_bn), split_ptr(ws), cur_stream()), "gemm_bf16");
   return d;
 }
 
@@ -542,8 +544,9 @@ std::vector<at::Tensor> gemm_swiglu(const at::Tensor& a, const at::Tensor& wgu, 
   c10::cuda::CUDAGuard g(a.device());
   at::Tensor h = at::empty({M, N2 / 2}, a.options());
   at::Tensor gu = save_gu ? at::empty({M, N2}, a.options()) : at::Tensor();
+  const at::Tensor ws = split_scratch(M > 128 ? prl_gemm2_ws_floats(M, N2, K) : 0, a);
   check(prl_gemm_swiglu_bf16(a.data_ptr(), wgu.data_ptr(), h.data_ptr(), save_gu ? gu.data_ptr() : nullptr, M, N2, K,
-                             a.stride(0), wgu.stride(0), h.stride(0), save_gu ? gu.stride(0) : 0, cur_stream()),
+                             a.stride(0), wgu.stride(0), h.stride(0), save_gu ? gu.stride(0) : 0, split_ptr(ws), cur_stream()),
         "gemm_swiglu");
   if (save_gu) return {h, gu};
   return {h};

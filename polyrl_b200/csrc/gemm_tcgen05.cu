@@ -84,6 +84,20 @@ struct SwigluParams {
 };
 struct EpiSwiglu {
   using Params = SwigluParams;
+  static constexpr bool kFinish = true;
+  template <class Sum>
+  __device__ __forceinline__ static void finish(const Params& p, const Sum& sum, int row, int n0, int c, int N) {
+    if (c >= 128 || n0 + 128 + c >= N) return;
+    const float4 g = sum(c), u = sum(128 + c);
+    if (p.GU) {
+      __nv_bfloat16* o = p.GU + static_cast<int64_t>(row) * p.ldgu + n0 + c;
+      *reinterpret_cast<uint2*>(o) = make_uint2(pack_bf16(g.x, g.y), pack_bf16(g.z, g.w));
+      *reinterpret_cast<uint2*>(o + 128) = make_uint2(pack_bf16(u.x, u.y), pack_bf16(u.z, u.w));
+    }
+    const float a = g.x / (1.0f + __expf(-g.x)) * u.x, b = g.y / (1.0f + __expf(-g.y)) * u.y, d = g.z / (1.0f + __expf(-g.z)) * u.z,
+                e = g.w / (1.0f + __expf(-g.w)) * u.w;
+    *reinterpret_cast<uint2*>(p.H + static_cast<int64_t>(row) * p.ldh + (n0 >> 1) + c) = make_uint2(pack_bf16(a, b), pack_bf16(d, e));
+  }
   __device__ __forceinline__ void begin(const Params&, int, int, const WorkInfo&) {}
   __device__ __forceinline__ void end(const Params&, int, int, const WorkInfo&) {}
   template <int BN>
@@ -119,6 +133,7 @@ struct ClampedGluParams {
 };
 struct EpiClampedGlu {
   using Params = ClampedGluParams;
+  static constexpr bool kFinish = false;
   __device__ __forceinline__ void begin(const Params&, int, int, const WorkInfo&) {}
   __device__ __forceinline__ void end(const Params&, int, int, const WorkInfo&) {}
   template <int BN>
@@ -212,13 +227,14 @@ static int pick_bn(int M, int N) {
 using namespace prl;
 
 // D = A·B^T (+R).  A:[M,K] B:[N,K] bf16 row-major with pitches lda/ldb/ldd in ELEMENTS.
-extern "C" int prl_gemm2_bf16(const void*, const void*, void*, const void*, int, int, int, int64_t, int64_t, int64_t, int, int,
-                              int, cudaStream_t);
+extern "C" int prl_gemm2_bf16(const void*, const void*, void*, const void*, int, int, int, int64_t, int64_t, int64_t, int64_t, int, int,
+                              int, float*, cudaStream_t);
 
 extern "C" int prl_gemm_bf16(const void* A, const void* B, void* D, const void* R, int M, int N, int K, int64_t lda,
-                             int64_t ldb, int64_t ldd, int force_bn, cudaStream_t stream) {
+                             int64_t ldb, int64_t ldd, int64_t ldr, int force_bn, float* ws, cudaStream_t stream) {
   // more than one 128-row block of tokens: the CTA-pair kernel (256-row tiles, cta_group::2) is the faster mainloop
-  if (M > kBlockM && N > 128 && force_bn == 0) return prl_gemm2_bf16(A, B, D, R, M, N, K, lda, ldb, ldd, 0, 0, 0, stream);
+  if (M > kBlockM && N > 128 && force_bn == 0) return prl_gemm2_bf16(A, B, D, R, M, N, K, lda, ldb, ldd, ldr, 0, 0, 0, ws, stream);
+  if (R != nullptr && ldr != ldd) return -14;          // a bias is the pair kernel's
   StoreParams sp{static_cast<__nv_bfloat16*>(D), static_cast<const __nv_bfloat16*>(R), ldd, nullptr, nullptr};
   const int bn = force_bn > 0 ? force_bn : pick_bn(M, N);
   switch (bn) {
@@ -245,12 +261,12 @@ extern "C" int prl_gemm_fp8(const void* A, const void* B, void* D, const float* 
 
 // H = silu(A·Wg^T) * (A·Wu^T) with W_gu block-interleaved ([128 gate | 128 up] per 256 rows).
 extern "C" int prl_gemm_swiglu_bf16(const void* A, const void* Wgu, void* H, void* GU, int M, int N2, int K,
-                                    int64_t lda, int64_t ldw, int64_t ldh, int64_t ldgu, cudaStream_t stream) {
+                                    int64_t lda, int64_t ldw, int64_t ldh, int64_t ldgu, float* ws, cudaStream_t stream) {
   if (N2 % 256 != 0) return -11;
   SwigluParams sp{static_cast<__nv_bfloat16*>(H), static_cast<__nv_bfloat16*>(GU), ldh, ldgu};
   if (M > kBlockM) {
     using Cfg2 = Gemm2Cfg<256, false, false, false>;
-    return launch_gemm2<Cfg2, EpiSwiglu>(A, Wgu, nullptr, M, N2, K, lda * 2, ldw * 2, 0, sp, 0, stream);
+    return launch_gemm2<Cfg2, EpiSwiglu>(A, Wgu, nullptr, M, N2, K, lda * 2, ldw * 2, 0, sp, 0, stream, Sched{0, 1, 0}, ws);
   }
   using Cfg = GemmCfg<256, 2>;
   return launch_gemm<Cfg, EpiSwiglu, NoGate, false>(A, Wgu, M, N2, K, lda * 2, ldw * 2, sp, NoGate::Params{}, 0, 0,

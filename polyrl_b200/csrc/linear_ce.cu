@@ -25,6 +25,7 @@ struct CeFwdParams {
 
 struct EpiCeFwd {
   using Params = CeFwdParams;
+  static constexpr bool kFinish = false;
   float m2, s, b;
   int64_t label;
   __device__ __forceinline__ void begin(const Params& p, int row, int M, const WorkInfo&) {
@@ -159,7 +160,7 @@ struct CeBwdRow {
 // CTA-pair kernel: 64 columns at a time, staged for TMA
 struct EpiCeBwdStore : CeBwdRow {
   using Params = CeBwdParams;
-  static constexpr bool kRow = true;
+  static constexpr bool kRow = true, kFinish = false;
   static constexpr int kAct = 0;
   __device__ __forceinline__ void apply(const Params& p, uint32_t (&r)[64], int col) const {
     float v[64];

@@ -140,3 +140,35 @@ def test_linear_ce_edges(t, v, h, tau):
     want = [lp64, ent64, *torch.autograd.grad([lp64, ent64], [x64, w64], [glp.double(), gent.double()])]
     for a, b, tol in zip(got, want, (1e-5, 1e-5, 1e-2, 1e-2)):
         assert (a.double() - b).norm() <= tol * b.norm()
+
+
+@pytest.mark.parametrize("m,n,k", [(300, 520, 8200), (257, 264, 4104), (2048, 2560, 16384), (129, 2816, 6000)])
+def test_gemm_cut_along_the_reduction(m, n, k):
+    """Products whose last round of tiles is cut: all layouts, residual, fp32 accumulation, gate / up.  One rounding to bf16; the fp32 sums
+    are k / 16 additions, each at most 2^-23 off."""
+    from polyrl_b200.ops import ext
+
+    C = ext()
+    a, b = _randn(m, k, seed=1), _randn(n, k, seed=2, scale=0.05)
+    m8 = m // 8 * 8
+    want = a.double() @ b.double().t()
+
+    def close(got, ref):
+        assert ((got.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4 * ref.abs().max()).all()
+
+    close(C.gemm2_bf16(a, b, False, False, None, None, 0), want)
+    close(C.gemm2_bf16(a, b.t().contiguous(), False, True, None, None, 0), want)
+    at = a[:m8].t().contiguous()
+    close(C.gemm2_bf16(at, b.t().contiguous(), True, True, None, None, 0), want[:m8])
+    close(C.gemm2_bf16(at, b, True, False, None, None, 0), want[:m8])
+    r = _randn(m, n, seed=3)
+    close(C.gemm_bf16(a, b, r, None, 0), want + r.double())
+    acc = _randn(m, n, seed=4, dtype=torch.float32)
+    ref = want + 0.5 * acc.double()
+    C.gemm2_accum_f32_(acc, a, b, False, False, 0.5)
+    assert (acc.double() - ref).norm() <= k * 2.0 ** -27 * ref.norm()
+    n2 = n // 256 * 256
+    gu = want[:, :n2].view(m, -1, 2, 128)
+    h, saved = C.gemm_swiglu(a, b[:n2], True)
+    close(saved, want[:, :n2])
+    close(h, (torch.nn.functional.silu(gu[:, :, 0]) * gu[:, :, 1]).flatten(1))
