@@ -394,6 +394,252 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
 }
 
+// ---- one softmax map, widths up to 128: two persistent CTAs an SM -------------------------------------------------------------------
+// The kernel above holds an SM alone and works on one tile: of a short sequence's (three or four key tiles) it spent more time on its
+// launch, first loads, the masked diagonal and its stores than on products.  Here a CTA takes half of the SM (96 KB of operands, 256 TMEM
+// columns, 192 threads), the other one fills its gaps, and both walk (query tile, head) items, so the loads of an item run under the end of
+// the one before:
+//   warp 0  TMA producer: Q, then one K and one V stage; K_(n+1) arrives while the softmax of tile n runs, V_(n+1) after PV_n
+//   warp 1  MMA issuer: S_n = Q K_n^T, then O += P_n V_n with P_n in TMEM, over the columns of S_n
+//   warps 2-5  softmax: thread = query row, so the row maximum and sum need no exchange; the 128 scores are read once and stay in
+//           registers; P goes back to TMEM as bf16
+// O stays in TMEM (fp32).  It is rescaled only when a row's maximum has grown by more than 2^8 since the last time: the probabilities
+// are relative to that older maximum, at most 256, and lose nothing as bf16 and fp32 have the same exponent range.
+// A mask is one comparison an element with a place inside the tile, under a test that is the same for the whole tile (written as conditions
+// on keys and sequence lengths it took 4000 cycles a tile, twice the rest of the softmax).  Rows leave through shared memory, 64 bytes of
+// eight rows a store, where 16 bytes of 32 rows took 3300 cycles.
+// 32 query heads, 8 KV heads of 128, causal: 19 sequences of 647 on average 473 -> 222 us; 24 of 512: 194 (one-tile CTAs) -> 110 us;
+// 3 of 4096: 603 -> 494 us.
+constexpr int kArThreads = 192;
+template <int DK, int DV>
+struct ArCfg {
+  static constexpr int QKT = 128 * DK * 2, VT = 128 * DV * 2;
+  static constexpr int SMEM = 2 * QKT + VT + 4 * 2048 + 1024 + 256;
+};
+template <int DK, int DV>
+__global__ void __launch_bounds__(kArThreads, 2)
+attn_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
+                 AttnFwdParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  using Cfg = ArCfg<DK, DV>;
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* sQ = smem;
+  uint8_t* sK = smem + Cfg::QKT;
+  uint8_t* sV = smem + 2 * Cfg::QKT;
+  uint8_t* sOut = smem + 2 * Cfg::QKT + Cfg::VT;       // a warp's 32 rows x 32 columns, bf16
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sOut + 4 * 2048);
+  uint64_t* q_full = bars;           // TMA
+  uint64_t* k_full = bars + 1;       // TMA
+  uint64_t* v_full = bars + 2;       // TMA
+  uint64_t* s_full = bars + 3;       // MMA commit: S_n is there, K_n (and behind an item's last, Q) may be overwritten
+  uint64_t* p_full = bars + 4;       // 128 arrivals: P_n is in TMEM, O is rescaled
+  uint64_t* pv_done = bars + 5;      // MMA commit: O is up to date, V_n and P_n may be overwritten
+  uint64_t* o_free = bars + 6;       // 128 arrivals: the item's O has been read
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 7);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
+    mbar_init(q_full, 1); mbar_init(k_full, 1); mbar_init(v_full, 1); mbar_init(s_full, 1); mbar_init(p_full, 128); mbar_init(pv_done, 1);
+    mbar_init(o_free, 128);
+    fence_barrier_init();
+  }
+  if (warp == 1) { tmem_alloc(tmem_slot, 256); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tS = tmem_base, tO = tmem_base + 128;
+
+  struct Item {
+    int h, q0, qs, lq, ks, lk, off, nt, kept_tiles, gap;
+    __device__ __forceinline__ int tile_of(int j) const { return j < kept_tiles ? j : j + gap; }
+  };
+  // item w (all of a warp asks): false behind the last one.  Heads of a tile are neighbours; tiles are numbered sequence by sequence.
+  auto item = [&](int w, Item& it) {
+    int q0 = 0;
+    const int seq = find_row_tile(p.cu_q, p.B, w / p.nq, &q0);
+    if (seq < 0) return false;
+    it.h = w % p.nq; it.q0 = q0;
+    it.qs = p.cu_q[seq]; it.lq = p.cu_q[seq + 1] - it.qs;
+    it.ks = p.cu_k[seq]; it.lk = p.cu_k[seq + 1] - it.ks;
+    it.off = it.lk - it.lq;                            // bottom-right aligned causal mask (prefix-cached prefill: lk > lq)
+    const int kv_end = p.causal ? min(it.lk, q0 + kAfBM + it.off) : it.lk;       // keys beyond the last row's diagonal are never needed
+    // key tiles in use: those of the kept first keys, then those from the window of this tile's first query on
+    const int w_tile = max(0, q0 + it.off - p.window + 1) / kAfBN;
+    it.kept_tiles = min((p.keep_first + kAfBN - 1) / kAfBN, w_tile);
+    it.gap = w_tile - it.kept_tiles;
+    it.nt = max(1, (kv_end + kAfBN - 1) / kAfBN - it.gap);
+    return true;
+  };
+
+  int n = 0, i = 0;                                    // tiles and items so far: the barriers' phases
+  Item it;
+  if (warp == 0) {
+    for (int w = blockIdx.x; item(w, it); w += gridDim.x, ++i) {
+      if (lane == 0) {
+        const int hk = it.h / (p.nq / p.nkv);
+        for (int j = 0; j < it.nt; ++j, ++n) {
+          const int key0 = it.ks + it.tile_of(j) * kAfBN;
+          if (n > 0) mbar_wait(s_full, (n - 1) & 1);
+          if (j == 0) {
+            mbar_expect_tx(q_full, Cfg::QKT);
+#pragma unroll
+            for (int c = 0; c < DK / 64; ++c) tma_load_2d(&tmQ, q_full, sQ + c * 16384, it.h * DK + c * 64, it.qs + it.q0);
+          }
+          mbar_expect_tx(k_full, Cfg::QKT);
+#pragma unroll
+          for (int c = 0; c < DK / 64; ++c) tma_load_2d(&tmK, k_full, sK + c * 16384, hk * DK + c * 64, key0);
+          if (n > 0) mbar_wait(pv_done, (n - 1) & 1);
+          mbar_expect_tx(v_full, Cfg::VT);
+#pragma unroll
+          for (int c = 0; c < DV / 64; ++c) tma_load_2d(&tmV, v_full, sV + c * 16384, hk * DV + c * 64, key0);
+        }
+      }
+      __syncwarp();
+    }
+  } else if (warp == 1) {
+    constexpr uint32_t idS = umma_idesc(128, 128, 1, 1);
+    constexpr uint32_t idO = umma_idesc_major(128, DV, 1, 1, 0, 1);         // B = V consumed MN-major
+    for (int w = blockIdx.x; item(w, it); w += gridDim.x, ++i) {
+      if (lane == 0) {
+        mbar_wait(q_full, i & 1);
+        for (int j = 0; j < it.nt; ++j, ++n) {
+          mbar_wait(k_full, n & 1);
+          if (n > 0) mbar_wait(pv_done, (n - 1) & 1);
+          tc_fence_after();
+#pragma unroll
+          for (int kk = 0; kk < DK / 16; ++kk) {
+            const uint64_t da = umma_desc_sw128_kmajor(sQ + (kk >> 2) * 16384) + 2 * (kk & 3);
+            const uint64_t db = umma_desc_sw128_kmajor(sK + (kk >> 2) * 16384) + 2 * (kk & 3);
+            umma_bf16_ss(tS, da, db, idS, kk != 0);
+          }
+          umma_commit(s_full);
+          mbar_wait(v_full, n & 1);
+          mbar_wait(p_full, n & 1);
+          if (j == 0 && i > 0) mbar_wait(o_free, (i - 1) & 1);
+          tc_fence_after();
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)               // 16 keys: 8 columns of P
+            umma_bf16_ts(tO, tS + 8 * kk, umma_desc_sw128_mnmajor(sV, 16384) + kk * 128, idO, (j | kk) != 0);
+          umma_commit(pv_done);
+        }
+      }
+      __syncwarp();
+    }
+  } else {
+    const int quad = warp & 3;
+    const int r = quad * 32 + lane;                       // query row inside the tile == TMEM lane
+    const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
+    const uint32_t stage = smem_u32(sOut) + (warp - 2) * 2048;
+    for (int w = blockIdx.x; item(w, it); w += gridDim.x, ++i) {
+      const int qrow = it.q0 + r;
+      const int last = p.causal ? min(qrow + it.off, it.lk - 1) : it.lk - 1;      // last key this row may attend to
+      const int klo = qrow + it.off - p.window;           // keys up to here are behind the window (unless kept)
+      float m_ref = -INFINITY, l_run = 0.f;
+      for (int j = 0; j < it.nt; ++j, ++n) {
+        mbar_wait(s_full, n & 1);
+        tc_fence_after();
+        const int base = it.tile_of(j) * kAfBN;
+        uint32_t v[128];
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < 128; c += 32) tmem_ld_32x32(tS + lane_base + c, *reinterpret_cast<uint32_t(*)[32]>(&v[c]));
+        tmem_ld_wait();
+        if (base + kAfBN > it.lk || (p.causal && base + kAfBN - 1 > it.q0 + it.off)) {
+          const int in = last - base;                     // place of the last key in this tile
+#pragma unroll
+          for (int e = 0; e < 128; ++e) v[e] = e <= in ? v[e] : 0xff800000u;      // -inf
+        }
+        if (base <= it.q0 + kAfBM - 1 + it.off - p.window) {
+          const int lo = klo - base, kept = p.keep_first - base;
+#pragma unroll
+          for (int e = 0; e < 128; ++e) v[e] = static_cast<int>(e > lo) | static_cast<int>(e < kept) ? v[e] : 0xff800000u;
+        }
+        float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+        for (int e = 0; e < 128; ++e) mx[e & 3] = fmaxf(mx[e & 3], __uint_as_float(v[e]));
+        const float m_new = fmaxf(m_ref, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])));
+        // raise this row's reference? (the first time it sees a key, and when probabilities would pass 2^8)
+        const bool raise = m_new > m_ref && (m_ref == -INFINITY || (m_new - m_ref) * p.scale_log2 > 8.f);
+        if (__any_sync(0xffffffffu, raise)) {
+          const float alpha = !raise ? 1.f : m_ref == -INFINITY ? 0.f : fast_exp2((m_ref - m_new) * p.scale_log2);
+          if (raise) m_ref = m_new;
+          l_run *= alpha;
+          if (j > 0) {                                    // (S_n was issued after PV_(n-1) had finished)
+#pragma unroll 1
+            for (int c = 0; c < DV; c += 16) {
+              uint32_t o[16];
+              tmem_ld_32x16(tO + lane_base + c, o);
+              tmem_ld_wait();
+#pragma unroll
+              for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
+              tmem_st_32x16(tO + lane_base + c, o);
+            }
+          }
+        }
+        const float mb = m_ref == -INFINITY ? 0.f : m_ref * p.scale_log2;
+        float ls[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int c = 0; c < 128; c += 32) {
+          uint32_t pk[16];
+#pragma unroll
+          for (int e = 0; e < 32; e += 2) {
+            const float a = fast_exp2(__uint_as_float(v[c + e]) * p.scale_log2 - mb);
+            const float b = fast_exp2(__uint_as_float(v[c + e + 1]) * p.scale_log2 - mb);
+            ls[e & 2] += a;
+            ls[(e & 2) + 1] += b;
+            pk[e >> 1] = pack_bf16(a, b);
+          }
+          tmem_st_32x16(tS + lane_base + (c >> 1), pk);
+        }
+        l_run += (ls[0] + ls[1]) + (ls[2] + ls[3]);
+        tmem_st_wait();
+        tc_fence_before();
+        mbar_arrive(p_full);
+      }
+      if (p.sink != nullptr && m_ref != -INFINITY) l_run += fast_exp2(p.sink[it.h] * 1.4426950408889634f - m_ref * p.scale_log2);
+      const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
+      if (p.lse && qrow < it.lq)
+        p.lse[static_cast<int64_t>(it.h) * p.Tq + it.qs + qrow] = m_ref == -INFINITY ? -INFINITY : m_ref * p.sm_scale + __logf(l_run);
+      mbar_wait(pv_done, (n - 1) & 1);
+      tc_fence_after();
+      // 16-byte unit u of row r lies at u ^ (r >> 1 & 3): eight rows' units, written or read, fall on all banks
+      const int row_in = it.q0 + quad * 32 + (lane >> 2);
+      __nv_bfloat16* dst = p.o + static_cast<int64_t>(it.qs + row_in) * p.ldo + it.h * DV + (lane & 3) * 8;
+#pragma unroll 1
+      for (int c = 0; c < DV; c += 32) {
+        uint32_t o[32];
+        __syncwarp();
+        tmem_ld_32x32(tO + lane_base + c, o);
+        tmem_ld_wait();
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          uint32_t q[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) q[e] = pack_bf16(__uint_as_float(o[8 * u + 2 * e]) * inv, __uint_as_float(o[8 * u + 2 * e + 1]) * inv);
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stage + lane * 64 + ((u ^ (lane >> 1 & 3)) << 4)), "r"(q[0]), "r"(q[1]), "r"(q[2]), "r"(q[3])
+                       : "memory");
+        }
+        __syncwarp();
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {                     // rows 8 g + lane / 4
+          const int row = 8 * g + (lane >> 2);
+          int4 q;
+          asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(q.x), "=r"(q.y), "=r"(q.z), "=r"(q.w)
+                       : "r"(stage + row * 64 + (((lane & 3) ^ (row >> 1 & 3)) << 4)) : "memory");
+          if (row_in + 8 * g < it.lq) st_v4(dst + 8 * g * p.ldo + c, q);
+        }
+      }
+      tc_fence_before();
+      mbar_arrive(o_free);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, 256); }
+}
+
 using EncodeTiledFn4 = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                     const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                     CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -444,6 +690,31 @@ static int run_attn_fwd(const void* q, const void* k, const void* v, const AttnF
   return 0;
 }
 
+template <int DK, int DV>
+static int run_attn_rows(const void* q, const void* k, const void* v, const AttnFwdParams& p, int Tk, int64_t ldq, int64_t ldk, int64_t ldv,
+                         int max_tiles, cudaStream_t stream) {
+  CUtensorMap tmQ, tmK, tmV;
+  if (af_tmap(&tmQ, q, p.Tq, static_cast<uint64_t>(p.nq) * DK, ldq * 2, kAfBM)) return -111;
+  if (af_tmap(&tmK, k, Tk, static_cast<uint64_t>(p.nkv) * DK, ldk * 2, kAfBN)) return -112;
+  if (af_tmap(&tmV, v, Tk, static_cast<uint64_t>(p.nkv) * DV, ldv * 2, kAfBN)) return -113;
+  static bool attr = false;
+  if (!attr) {
+    PRL_CUDA_CHECK(cudaFuncSetAttribute(attn_rows_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, ArCfg<DK, DV>::SMEM));
+    attr = true;
+  }
+  static int sms = 0;
+  if (!sms) {
+    int dev = 0;
+    PRL_CUDA_CHECK(cudaGetDevice(&dev));
+    PRL_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  }
+  const int64_t items = static_cast<int64_t>(max_tiles) * p.nq;       // (an upper bound: a CTA without an item returns)
+  const int grid = static_cast<int>(items < 2 * sms ? items : 2 * sms);
+  attn_rows_kernel<DK, DV><<<grid, kArThreads, ArCfg<DK, DV>::SMEM, stream>>>(tmQ, tmK, tmV, p);
+  PRL_CUDA_CHECK(cudaGetLastError());
+  return 0;
+}
+
 // q:[Tq, nq*dk] (pitch ldq), k:[Tk, nkv*dk], v:[Tk, nkv*dv] (pitches ldk/ldv), o:[Tq, nq*dv] (pitch ldo); pitches in ELEMENTS;
 // dk, dv = 64 or 128; dk = 192 (dv = 128).  window > 0 (causal only): query i sees keys j <= i with i - j < window or j < keep_first.  cu_q / cu_k: int32 [B+1] device arrays.  max_tiles: upper bound on sum_b ceil(lq_b / 128) (e.g. Tq/128 + B).
 // sink: fp32 [nq] or null.
@@ -466,10 +737,10 @@ extern "C" int prl_attn_fwd(const void* q, const void* k, const void* v, void* o
   p.keep_first = window > 0 ? keep_first : 0;
   p.sink = sink;
   p.dbg = dbg;
-  if (dk == 64 && dv == 64) return run_attn_fwd<64, 64, 1>(q, k, v, p, Tk, ldq, ldk, ldv, max_tiles, stream);
-  if (dk == 64 && dv == 128) return run_attn_fwd<64, 128, 1>(q, k, v, p, Tk, ldq, ldk, ldv, max_tiles, stream);
-  if (dk == 128 && dv == 64) return run_attn_fwd<128, 64, 1>(q, k, v, p, Tk, ldq, ldk, ldv, max_tiles, stream);
-  if (dk == 128 && dv == 128) return run_attn_fwd<128, 128, 1>(q, k, v, p, Tk, ldq, ldk, ldv, max_tiles, stream);
+  if (dk == 64 && dv == 64) return run_attn_rows<64, 64>(q, k, v, p, Tk, ldq, ldk, ldv, max_tiles, stream);
+  if (dk == 64 && dv == 128) return run_attn_rows<64, 128>(q, k, v, p, Tk, ldq, ldk, ldv, max_tiles, stream);
+  if (dk == 128 && dv == 64) return run_attn_rows<128, 64>(q, k, v, p, Tk, ldq, ldk, ldv, max_tiles, stream);
+  if (dk == 128 && dv == 128) return run_attn_rows<128, 128>(q, k, v, p, Tk, ldq, ldk, ldv, max_tiles, stream);
   if (dk == 192 && dv == 128) return run_attn_fwd<192, 128, 1>(q, k, v, p, Tk, ldq, ldk, ldv, max_tiles, stream);
   return -114;
 }

@@ -390,6 +390,30 @@ __device__ __forceinline__ float2 unpack_bf16(uint32_t u) {
   return __bfloat1622float2(h);
 }
 
+// Which 128-row tile of a packed batch is number `t`?  Tiles are counted sequence by sequence.  Called by one whole warp, which looks at
+// 32 sequences at a time.  Returns the sequence (-1: fewer tiles than t + 1) and the tile's first row.
+__device__ __forceinline__ int find_row_tile(const int32_t* __restrict__ cu, int B, int t, int* row0) {
+  const int lane = threadIdx.x & 31;
+  for (int b0 = 0; b0 < B; b0 += 32) {
+    const int b = b0 + lane;
+    const int nt = b < B ? (cu[b + 1] - cu[b] + 127) >> 7 : 0;
+    int incl = nt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    const unsigned hit = __ballot_sync(0xffffffffu, t < incl);
+    if (hit) {
+      const int l = __ffs(hit) - 1;
+      *row0 = (t - __shfl_sync(0xffffffffu, incl - nt, l)) * 128;
+      return b0 + l;
+    }
+    t -= __shfl_sync(0xffffffffu, incl, 31);
+  }
+  return -1;
+}
+
 }  // namespace prl
 
 // cuTensorMapEncodeTiled is a driver call and needs a context bound to the calling thread.  A fresh thread (an autograd worker

@@ -172,3 +172,42 @@ def test_gemm_cut_along_the_reduction(m, n, k):
     h, saved = C.gemm_swiglu(a, b[:n2], True)
     close(saved, want[:, :n2])
     close(h, (torch.nn.functional.silu(gu[:, :, 0]) * gu[:, :, 1]).flatten(1))
+
+
+def _attend64(q, k, v, lq, lk, causal):
+    """Packed attention in 64 bits: (output, log-sum-exp [heads, T])."""
+    outs, lses = [], []
+    g, scale = q.shape[1] // k.shape[1], q.shape[2] ** -0.5
+    for a, b, c in zip(q.split(lq), k.split(lk), v.split(lk)):
+        z = torch.einsum("qhd,khd->hqk", a, b.repeat_interleave(g, 1)) * scale
+        if causal:
+            z = z.masked_fill(torch.ones(z.shape[-2:], dtype=torch.bool, device=q.device).triu(z.shape[2] - z.shape[1] + 1), float("-inf"))
+        lses.append(z.logsumexp(-1))
+        outs.append(torch.einsum("hqk,khd->qhd", z.softmax(-1), c.repeat_interleave(g, 1)))
+    return torch.cat(outs), torch.cat(lses, 1)
+
+
+def _packed(d, lq, lk, growth, nq=4, nkv=2):
+    q, k, v = _randn(sum(lq), nq, d, seed=1), _randn(sum(lk), nkv, d, seed=2), _randn(sum(lk), nkv, d, seed=3)
+    k = (k.float() * torch.cat([1 + growth * torch.arange(n, device="cuda") / 128 for n in lk])[:, None, None]).bfloat16()
+    cu_q, cu_k = (torch.tensor([0] + x, dtype=torch.int32).cumsum(0).to(torch.int32).cuda() for x in (lq, lk))
+    return q, k, v, cu_q, cu_k
+
+
+_LENGTHS = [([1], [1], True), ([130], [130], True), ([3, 128, 257], [3, 128, 257], True), ([5, 200], [700, 333], True), ([64, 1], [640, 129], False),
+            ([7] * 100, [7] * 100, True)]
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("lq,lk,causal", _LENGTHS)
+@pytest.mark.parametrize("growth", [0.0, 3.0])
+def test_attention_forward_tiles(d, lq, lk, causal, growth):
+    """Packed sequences, prompts behind a prefix among them.  ``growth`` makes later keys longer, so that row maxima rise by more than 2^8
+    from tile to tile and the output is rescaled.  Probabilities and the output are bf16: each value within 2^-8, 1e-2 of the norm."""
+    from polyrl_b200.ops import ext
+
+    q, k, v, cu_q, cu_k = _packed(d, lq, lk, growth)
+    o, lse = ext().attn_fwd(q, k, v, cu_q, cu_k, d ** -0.5, causal, True)
+    want, lse64 = _attend64(q.double(), k.double(), v.double(), lq, lk, causal)
+    assert (o.double() - want).norm() <= 1e-2 * want.norm()
+    assert (lse.double() - lse64).abs().max() <= 1e-5 * (1 + lse64.abs().max()) + 1e-4
