@@ -31,6 +31,7 @@
 
 namespace prl {
 
+constexpr int kNoWindow = 0x40000000;    // wider than any sequence; distances from queries before the first key stay within 32 bits
 constexpr int kAfThreads = 320;          // warp0 TMA, warp1 MMA, warps 2-5 + 6-9: two softmax warpgroups
 constexpr int kAfBM = 128, kAfBN = 128;
 constexpr int kAfTile = 128 * 128 * 2;              // 32 KB: one 128 x 128 bf16 operand tile (2 chunks of 64 columns)
@@ -54,7 +55,7 @@ struct AttnFwdParams {
   float scale_log2;            // sm_scale * log2(e)
   float sm_scale;
   int causal;
-  int window, keep_first;      // window: 0x7fffffff when every earlier key is seen
+  int window, keep_first;      // window: kNoWindow when every earlier key is seen
   const float* sink;           // [nq] or null: natural-log sink of the softmax denominator
   const float* lam;            // two maps: [1] weight of the second
   float keep, eps;             // two maps: factor behind the norm, and what is added under its root
@@ -733,7 +734,7 @@ extern "C" int prl_attn_fwd(const void* q, const void* k, const void* v, void* o
   p.scale_log2 = sm_scale * 1.4426950408889634f;
   p.causal = causal;
   if (window > 0 && !causal) return -115;
-  p.window = window > 0 ? window : 0x7fffffff;
+  p.window = window > 0 ? min(window, kNoWindow) : kNoWindow;
   p.keep_first = window > 0 ? keep_first : 0;
   p.sink = sink;
   p.dbg = dbg;
@@ -759,7 +760,7 @@ extern "C" int prl_map_attn_fwd(const void* q, const void* k, const void* v, voi
   p.sm_scale = sm_scale;
   p.scale_log2 = sm_scale * 1.4426950408889634f;
   p.causal = 1;
-  p.window = window;
+  p.window = min(window, kNoWindow);
   p.lam = lam; p.keep = keep; p.eps = eps; p.dv_out = dv_out; p.shared_row = shared_row;
   const int64_t ldq = static_cast<int64_t>(nq) * 2 * dk, ldk = static_cast<int64_t>(nkv) * (shared_row ? 1 : 2) * dk, ldv = static_cast<int64_t>(nkv) * dv;
   if (dk == 64 && dv == 64) return run_attn_fwd<64, 64, 2>(q, k, v, p, Tk, ldq, ldk, ldv, max_tiles, stream);

@@ -26,7 +26,7 @@ int prl_quant_fp8_rowwise(const void*, void*, float*, int, int, cudaStream_t);
 int prl_grad_accum(float*, const void*, int, float, int64_t, float*, cudaStream_t);
 int prl_sumsq(const float*, int64_t, float*, cudaStream_t);
 int prl_adamw(float*, float*, float*, float*, void*, int64_t, float, float, float, float, float, int, float, const float*, int*, int, cudaStream_t);
-int prl_attn_bwd(const void*, const void*, const void*, const void*, const void*, const float*, float*, float*, void*, void*, const int32_t*, const int32_t*, int, int, int, int, int, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, float, int, int, cudaStream_t);
+int prl_attn_bwd(const void*, const void*, const void*, const void*, const void*, const float*, float*, void*, void*, void*, const int32_t*, const int32_t*, int, int, int, int, int, int, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, float, int, int, int, cudaStream_t);
 int prl_qk_rope_width_ok(int);
 int prl_qk_rope(const void*, void*, const int64_t*, const float*, const float*, const void*, const void*, float, int, int, int, int, int64_t, int64_t, float, void*, void*, const int64_t*, int, cudaStream_t);
 int prl_qk_norm_rope_bwd_parts(int, int, int, int);
@@ -371,14 +371,16 @@ void adamw_(at::Tensor master, at::Tensor m, at::Tensor v, at::Tensor grad, cons
 
 // varlen causal flash-attention forward on tcgen05 (csrc/attn_fwd.cu).  q:[Tq,nq,128] k,v:[Tk,nkv,128] (row-strided views allowed)
 // flash-attention backward (csrc/attn_bwd.cu): (dq, dk, dv) in bf16, shapes of q / k / v; contiguous, or views of the columns of `out`
-// [T, (nq + 2 nkv) * 128] (the gradient of a fused projection: query, key and value heads side by side)
+// [T, (nq + 2 nkv) * d] (the gradient of a fused projection: query, key and value heads side by side)
 std::vector<at::Tensor> attn_bwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& o,
                                  const at::Tensor& d_o, const at::Tensor& lse, const at::Tensor& cu_q, const at::Tensor& cu_k,
                                  double sm_scale, bool causal, const c10::optional<at::Tensor>& out) {
   CHECK_BF16(q); CHECK_BF16(k); CHECK_BF16(v); CHECK_BF16(o); CHECK_BF16(d_o); CHECK_F32(lse);
+  const int64_t d = q.size(-1);
+  TORCH_CHECK(d == 64 || d == 128, "attn_bwd: head width 64 or 128");
   for (const at::Tensor* t : {&q, &k, &v, &o, &d_o}) {
-    TORCH_CHECK(t->dim() == 3 && t->size(2) == 128 && t->stride(2) == 1 && t->stride(1) == 128 && t->stride(0) % 8 == 0 &&
-                (reinterpret_cast<uintptr_t>(t->data_ptr()) & 15) == 0, "attn_bwd: [T, heads, 128] row-strided bf16 operands");
+    TORCH_CHECK(t->dim() == 3 && t->size(2) == d && t->stride(2) == 1 && t->stride(1) == d && t->stride(0) % 8 == 0 &&
+                (reinterpret_cast<uintptr_t>(t->data_ptr()) & 15) == 0, "attn_bwd: [T, heads, d] row-strided bf16 operands");
   }
   const int Tq = q.size(0), Tk = k.size(0), nq = q.size(1), nkv = k.size(1), B = cu_q.numel() - 1;
   TORCH_CHECK(lse.is_contiguous() && lse.size(0) == nq && lse.size(1) == Tq);
@@ -386,22 +388,20 @@ std::vector<at::Tensor> attn_bwd(const at::Tensor& q, const at::Tensor& k, const
   at::Tensor dq, dk, dv;
   if (out.has_value()) {
     CHECK_BF16(*out);
-    TORCH_CHECK(Tq == Tk && out->dim() == 2 && out->is_contiguous() && out->size(0) == Tq && out->size(1) == (nq + 2 * nkv) * 128 &&
-                (reinterpret_cast<uintptr_t>(out->data_ptr()) & 15) == 0, "attn_bwd: out is [T, (nq + 2 nkv) * 128]");
-    const at::Tensor heads = out->view({Tq, nq + 2 * nkv, 128});
+    TORCH_CHECK(Tq == Tk && out->dim() == 2 && out->is_contiguous() && out->size(0) == Tq && out->size(1) == (nq + 2 * nkv) * d &&
+                (reinterpret_cast<uintptr_t>(out->data_ptr()) & 15) == 0, "attn_bwd: out is [T, (nq + 2 nkv) * d]");
+    const at::Tensor heads = out->view({Tq, nq + 2 * nkv, d});
     dq = heads.narrow(1, 0, nq); dk = heads.narrow(1, nq, nkv); dv = heads.narrow(1, nq + nkv, nkv);
   } else {
-    dk = at::empty({Tk, nkv, 128}, q.options());
-    dv = at::empty({Tk, nkv, 128}, q.options());
+    dq = at::empty({Tq, nq, d}, q.options());
+    dk = at::empty({Tk, nkv, d}, q.options());
+    dv = at::empty({Tk, nkv, d}, q.options());
   }
-  at::Tensor dq_acc = at::zeros({Tq, nq, 128}, q.options().dtype(at::kFloat));
-  at::Tensor dsum = at::empty({nq, Tq}, q.options().dtype(at::kFloat));
+  at::Tensor stats = at::empty({nq, Tq, 2}, q.options().dtype(at::kFloat));
   check(prl_attn_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), d_o.data_ptr(), lse.data_ptr<float>(),
-                     dsum.data_ptr<float>(), dq_acc.data_ptr<float>(), dk.data_ptr(), dv.data_ptr(), cu_q.data_ptr<int>(),
-                     cu_k.data_ptr<int>(), B, Tq, Tk, nq, nkv, q.stride(0), k.stride(0), v.stride(0), o.stride(0), d_o.stride(0), dk.stride(0),
-                     static_cast<float>(sm_scale), causal ? 1 : 0, Tk / 128 + B, cur_stream()), "attn_bwd");
-  if (out.has_value()) dq.copy_(dq_acc);
-  else dq = dq_acc.to(at::kBFloat16);
+                     stats.data_ptr<float>(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), cu_q.data_ptr<int>(),
+                     cu_k.data_ptr<int>(), B, Tq, Tk, nq, nkv, d, q.stride(0), k.stride(0), v.stride(0), o.stride(0), d_o.stride(0), dq.stride(0), dk.stride(0),
+                     static_cast<float>(sm_scale), causal ? 1 : 0, Tq / 128 + B, Tk / 128 + B, cur_stream()), "attn_bwd");
   return {dq, dk, dv};
 }
 

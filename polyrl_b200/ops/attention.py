@@ -1,6 +1,6 @@
 """Packed (varlen) causal self-attention for training / prefill.
 
-Backends, in order: the own tcgen05 / TMEM flash-attention kernels (csrc/attn_fwd.cu, csrc/attn_bwd.cu: head_dim 128, bf16,
+Backends, in order: the own tcgen05 / TMEM flash-attention kernels (csrc/attn_fwd.cu, csrc/attn_bwd.cu: head_dim 64 or 128, bf16,
 GQA, bottom-right aligned causal mask for prefill behind a cached prefix) on CUDA; the flash-attn varlen library (what the
 reference calls, 3rdparty/verl/verl/models/transformers/monkey_patch.py:108) for other head sizes / dtypes or when
 ``POLYRL_ATTN_BACKEND=flash``; PyTorch SDPA over a padded [B, S] view otherwise (CPU tests).  Decode-time attention is NOT
@@ -18,12 +18,12 @@ _FLASH = None
 
 def _own_ok(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> bool:
     return (q.is_cuda and q.dtype == torch.bfloat16 and k.dtype == torch.bfloat16 and v.dtype == torch.bfloat16
-            and q.shape[-1] == 128 and k.shape[-1] == 128 and q.shape[1] % k.shape[1] == 0
+            and q.shape[-1] in (64, 128) and k.shape[-1] == v.shape[-1] == q.shape[-1] and q.shape[1] % k.shape[1] == 0
             and os.environ.get("POLYRL_ATTN_BACKEND", "own") == "own" and os.environ.get("POLYRL_GEMM_BACKEND", "tcgen05") != "cublas")
 
 
 def _rows(t: torch.Tensor) -> torch.Tensor:
-    """[T, heads, 128] view whose heads are contiguous inside a token row (row pitch free): what the kernels' TMA maps need."""
+    """[T, heads, d] view whose heads are contiguous inside a token row (row pitch free): what the kernels' TMA maps need."""
     if t.stride(2) != 1 or t.stride(1) != t.shape[2] or t.stride(0) % 8 != 0 or t.data_ptr() % 16 != 0:
         t = t.contiguous()
     return t

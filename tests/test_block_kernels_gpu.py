@@ -88,17 +88,18 @@ def test_norm_rope_and_cache(d, nq, nkv, norm):
         assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()
 
 
-@pytest.mark.parametrize("nq,nkv,lens", [(4, 4, [1]), (8, 2, [128, 1, 129]), (6, 2, [77, 300, 5])])
+@pytest.mark.parametrize("d,nq,nkv,lens", [(128, 4, 4, [1]), (128, 8, 2, [128, 1, 129]), (128, 6, 2, [77, 300, 5]), (64, 14, 2, [127, 600, 1, 256]),
+                                           (128, 2, 1, [5] * 40)])
 @pytest.mark.parametrize("norm", [False, True])
-def test_rope_attention(nq, nkv, lens, norm):
+def test_rope_attention(d, nq, nkv, lens, norm):
     """Norm, rotation and attention as one function against autograd in 64 bits: probabilities and their gradients pass through bf16 on
     their way into the products, so 2e-2 of the norm.  A lone token has no gradient but the difference of two fp32 sums of 128 products,
     128 * 2^-24 * 128^-0.5 < 7e-7 an element of the 512 that a gain sums: 2e-5."""
     from polyrl_b200.ops.attention import rope_attention
 
-    d, t = 128, sum(lens)
+    t = sum(lens)
     qkv = _randn(t, (nq + 2 * nkv) * d, seed=1)
-    cos, sin = (f.cuda() for f in OF.ref.rope_tables(512, d, 1e4))
+    cos, sin = (f.cuda() for f in OF.ref.rope_tables(640, d, 1e4))
     pos = torch.cat([torch.arange(n) for n in lens]).cuda()
     cu = torch.tensor([0] + lens, dtype=torch.int32).cumsum(0).to(torch.int32).cuda()
     qn, kn = (_randn(d, seed=4, scale=0.1, shift=1.0), _randn(d, seed=5, scale=0.1, shift=1.0)) if norm else (None, None)
@@ -211,3 +212,23 @@ def test_attention_forward_tiles(d, lq, lk, causal, growth):
     want, lse64 = _attend64(q.double(), k.double(), v.double(), lq, lk, causal)
     assert (o.double() - want).norm() <= 1e-2 * want.norm()
     assert (lse.double() - lse64).abs().max() <= 1e-5 * (1 + lse64.abs().max()) + 1e-4
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("lq,lk,causal", _LENGTHS + [([300], [100], True)])
+def test_attention_backward_tiles(d, lq, lk, causal):
+    """Gradients of packed sequences, of prompts behind a prefix, and of queries before the first key, which see none.  Probabilities and
+    their gradients enter the products as bf16: 2e-2 of the norm; with one key the gradients of the scores are differences of equal sums."""
+    from polyrl_b200.ops import ext
+
+    q, k, v, cu_q, cu_k = _packed(d, lq, lk, 0.0)
+    go = _randn(*q.shape, seed=4)
+    o, lse = ext().attn_fwd(q, k, v, cu_q, cu_k, d ** -0.5, causal, True)
+    got = ext().attn_bwd(q, k, v, o, go, lse, cu_q, cu_k, d ** -0.5, causal)
+    blind = max(0, lq[0] - lk[0]) if causal else 0                        # queries of the first sequence that see no key
+    leaves = [x.double().requires_grad_(True) for x in (q[blind:], k, v)]
+    out, _ = _attend64(*leaves, [lq[0] - blind] + lq[1:], lk, causal)
+    want = torch.autograd.grad(out, leaves, go[blind:].double())
+    assert not got[0][:blind].any()
+    for a, b in zip((got[0][blind:], got[1], got[2]), want):
+        assert (a.double() - b).norm() <= 2e-2 * b.norm() + 1e-3
