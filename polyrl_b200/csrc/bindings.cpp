@@ -10,6 +10,8 @@
 extern "C" {
 int prl_gemm2_bf16(const void*, const void*, void*, const void*, int, int, int, int64_t, int64_t, int64_t, int64_t, int, int, int, float*, cudaStream_t);
 int64_t prl_gemm2_ws_floats(int, int, int);
+int prl_gemm2_grads_joint(int, int, int);
+int prl_gemm2_grads(const void*, const void*, const void*, void*, float*, float, void*, int, int, int, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, cudaStream_t);
 int prl_gemm2_bf16_accum_f32(const void*, const void*, float*, float, int, int, int, int64_t, int64_t, int64_t, int, int, float*, cudaStream_t);
 int prl_gemm_fp8(const void*, const void*, void*, const float*, const float*, int, int, int, int64_t, int64_t, int64_t, int, cudaStream_t);
 int prl_linear_ce_num_splits(int, int);
@@ -124,6 +126,41 @@ void gemm2_accum_f32_(at::Tensor out32, const at::Tensor& a, const at::Tensor& b
   check(prl_gemm2_bf16_accum_f32(a.data_ptr(), b.data_ptr(), out32.data_ptr<float>(), static_cast<float>(beta), M, N, K,
                                  a.stride(0), b.stride(0), out32.stride(0), a_mn ? 1 : 0, b_mn ? 1 : 0, split_ptr(ws), cur_stream()),
         "gemm2_accum_f32");
+}
+
+// Both gradients of y = x w^T: (dx, dw) = (dy w, dy^T x) from dy [T, N], w [N, K], x [T, K].  dx32: accumulate into this fp32 matrix
+// (beta * dx32 + dy w) instead of returning a bf16 one.  One launch for both where that is the faster way.
+std::vector<at::Tensor> gemm2_grads(const at::Tensor& dy, const at::Tensor& w, const at::Tensor& x, const c10::optional<at::Tensor>& dw_out,
+                                    const c10::optional<at::Tensor>& dx32, double beta) {
+  for (const at::Tensor* t : {&dy, &w, &x}) {
+    CHECK_BF16(*t);
+    TORCH_CHECK(t->dim() == 2 && t->stride(1) == 1 && t->stride(0) % 8 == 0 && t->stride(0) >= t->size(1) && t->size(1) % 8 == 0 &&
+                (reinterpret_cast<uintptr_t>(t->data_ptr()) & 15) == 0 && t->get_device() == dy.get_device(), "gemm2_grads: operands");
+  }
+  const int64_t T = dy.size(0), N = dy.size(1), K = w.size(1);
+  TORCH_CHECK(w.size(0) == N && x.size(0) == T && x.size(1) == K, "gemm2_grads: shapes");
+  c10::cuda::CUDAGuard g(dy.device());
+  at::Tensor dw = dw_out.has_value() ? *dw_out : at::empty({N, K}, w.options()), dx;
+  CHECK_BF16(dw);
+  TORCH_CHECK(dw.dim() == 2 && dw.size(0) == N && dw.size(1) == K && dw.stride(1) == 1 && dw.stride(0) % 8 == 0 &&
+              (reinterpret_cast<uintptr_t>(dw.data_ptr()) & 15) == 0, "gemm2_grads: dw");
+  if (dx32.has_value()) {
+    CHECK_F32(*dx32);
+    TORCH_CHECK(dx32->dim() == 2 && dx32->size(0) == T && dx32->size(1) == K && dx32->stride(1) == 1 && dx32->stride(0) % 4 == 0 &&
+                (reinterpret_cast<uintptr_t>(dx32->data_ptr()) & 15) == 0, "gemm2_grads: dx32");
+  } else {
+    dx = at::empty({T, K}, x.options());
+  }
+  if (T == 0 || N == 0 || K == 0 || !prl_gemm2_grads_joint(T, N, K)) {
+    if (dx32.has_value()) gemm2_accum_f32_(*dx32, dy, w, false, true, beta);
+    else dx = gemm2_bf16(dy, w, false, true, c10::nullopt, dx, 0);
+    gemm2_bf16(dy, x, true, true, c10::nullopt, dw, 0);
+    return {dx32.has_value() ? *dx32 : dx, dw};
+  }
+  check(prl_gemm2_grads(dy.data_ptr(), w.data_ptr(), x.data_ptr(), dx32.has_value() ? nullptr : dx.data_ptr(),
+                        dx32.has_value() ? dx32->data_ptr<float>() : nullptr, static_cast<float>(beta), dw.data_ptr(), T, N, K, dy.stride(0), w.stride(0),
+                        x.stride(0), dx32.has_value() ? 0 : dx.stride(0), dx32.has_value() ? dx32->stride(0) : 0, dw.stride(0), cur_stream()), "gemm2_grads");
+  return {dx32.has_value() ? *dx32 : dx, dw};
 }
 
 at::Tensor gemm_fp8(const at::Tensor& a, const at::Tensor& b, const at::Tensor& row_scale, const at::Tensor& col_scale,
@@ -645,6 +682,8 @@ void nvls_bcast_store(const at::Tensor& src, int64_t mc_dst, int64_t ctas) {
 }
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.def("gemm2_grads", &gemm2_grads, py::arg("dy"), py::arg("w"), py::arg("x"), py::arg("dw") = py::none(), py::arg("dx32") = py::none(),
+        py::arg("beta") = 0.0);
   m.def("gemm2_bf16", &gemm2_bf16, py::arg("a"), py::arg("b"), py::arg("a_mn") = false, py::arg("b_mn") = false,
         py::arg("residual") = py::none(), py::arg("out") = py::none(), py::arg("force_bn") = 0);
   m.def("gemm2_accum_f32_", &gemm2_accum_f32_);

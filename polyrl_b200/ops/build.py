@@ -28,7 +28,7 @@ MODULES: dict[str, dict] = {
                "cu": ["gemm_tcgen05.cu", "gemm2.cu", "attn_fwd.cu", "decode_attn.cu", "sampling.cu", "mix_elem.cu", "mix_scan.cu", "mix_chunk.cu", "mix_chunk_tc.cu", "mix_delta.cu", "mix_latent.cu",
                       "mix_window.cu", "mix_maps.cu", "mix_block.cu", "mix_experts.cu", "mix_streams.cu", "mix_selective.cu", "mix_gla.cu"]},
     "_C": {"bindings": "bindings.cpp",
-           "cu": ["gemm_tcgen05.cu", "gemm2.cu", "skinny_gemm.cu", "decode_gemm.cu", "vmm.cu", "linear_ce.cu", "ag_gemm.cu", "elementwise.cu", "qk_rope.cu",
+           "cu": ["gemm_tcgen05.cu", "gemm2.cu", "gemm2_grads.cu", "skinny_gemm.cu", "decode_gemm.cu", "vmm.cu", "linear_ce.cu", "ag_gemm.cu", "elementwise.cu", "qk_rope.cu",
                   "optim.cu", "attn_bwd.cu", "attn_fwd.cu", "p2p.cu", "nvls.cu"]},
 }
 HEADERS = ["common.cuh", "gemm_sm100.cuh", "gemm2_sm100.cuh", "mixers.cuh", "mix_tc.cuh", "mix_params.hpp"]

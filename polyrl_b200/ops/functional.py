@@ -75,6 +75,13 @@ def mm_tn(dy: torch.Tensor, x: torch.Tensor, out: torch.Tensor | None = None) ->
     return _C().gemm2_bf16(_g2_operand(dy), _g2_operand(x), True, True, None, out, 0)
 
 
+def mm_grads(dy: torch.Tensor, w: torch.Tensor, x: torch.Tensor, dw_out: torch.Tensor | None = None) -> tuple[torch.Tensor, torch.Tensor]:
+    """(dgrad, wgrad) of ``y = x @ w.T``: ``mm_nn(dy, w)`` and ``mm_tn(dy, x)``, in one launch where the kernels take the operands."""
+    if _cublas() or not (_is_kernel_tensor(dy) and w.dtype == x.dtype == torch.bfloat16 and _g2_ok(dy.shape[1], w.shape[1])):
+        return mm_nn(dy, w), mm_tn(dy, x, out=dw_out)
+    return tuple(_C().gemm2_grads(_g2_operand(dy), _g2_operand(w), _g2_operand(x), dw_out))
+
+
 # ---- decode-shape ("skinny") GEMM: swap-AB + split-K tcgen05 kernel for <= 256 rows, inference only ----
 _SKINNY_WS: dict = {}
 _SKINNY_MAX_ROWS = int(os.environ.get("POLYRL_SKINNY_MAX_ROWS", "256"))
@@ -206,9 +213,12 @@ class _LinearFn(torch.autograd.Function):
         x2, w = ctx.saved_tensors
         dy2 = dy.reshape(-1, dy.shape[-1])
         dx = dw = dres = None
-        if ctx.needs_input_grad[0]:
+        if ctx.needs_input_grad[0] and ctx.needs_input_grad[1]:
+            dx, dw = mm_grads(dy2, w, x2, _sink_for(w))
+            dx = dx.reshape(ctx.x_shape)
+        elif ctx.needs_input_grad[0]:
             dx = mm_nn(dy2, w).reshape(ctx.x_shape)
-        if ctx.needs_input_grad[1]:
+        elif ctx.needs_input_grad[1]:
             dw = mm_tn(dy2, x2, out=_sink_for(w))
         if ctx.has_res and ctx.needs_input_grad[2]:
             dres = dy
@@ -263,6 +273,9 @@ class _LinearSwigluFn(torch.autograd.Function):
         x2, wgu, gu = ctx.saved_tensors
         dh2 = dh.reshape(-1, dh.shape[-1]).contiguous()
         dgu = _C().swiglu_bwd(gu, dh2)
+        if ctx.needs_input_grad[0] and ctx.needs_input_grad[1]:
+            dx, dw = mm_grads(dgu, wgu, x2, _sink_for(wgu))
+            return dx.reshape(ctx.x_shape), dw
         dx = mm_nn(dgu, wgu).reshape(ctx.x_shape) if ctx.needs_input_grad[0] else None
         dw = mm_tn(dgu, x2, out=_sink_for(wgu)) if ctx.needs_input_grad[1] else None
         return dx, dw
@@ -450,6 +463,9 @@ class _LinearCEFn(torch.autograd.Function):
             v1 = min(V, v0 + _CE_CHUNK)
             ws = w[v0:v1]
             dz = C.linear_ce_dz(h2, ws, lab, lse, ez, g_lp, g_ent, ctx.inv_tau, v0)
+            if need_h and need_w and own and w.stride(1) == 1 and w.stride(0) % 8 == 0 and ws.data_ptr() % 16 == 0 and h2.data_ptr() % 16 == 0:
+                C.gemm2_grads(dz, ws, h2, dw[v0:v1], dh, 0.0 if v0 == 0 else 1.0)
+                continue
             if need_h:
                 if own:      # dH (fp32) += dz @ W_slice inside the GEMM epilogue
                     C.gemm2_accum_f32_(dh, dz, ws, False, True, 0.0 if v0 == 0 else 1.0)

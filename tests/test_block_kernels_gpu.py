@@ -232,3 +232,23 @@ def test_attention_backward_tiles(d, lq, lk, causal):
     assert not got[0][:blind].any()
     for a, b in zip((got[0][blind:], got[1], got[2]), want):
         assert (a.double() - b).norm() <= 2e-2 * b.norm() + 1e-3
+
+
+@pytest.mark.parametrize("t,n,k", [(8, 136, 136), (387, 1152, 896), (300, 4096, 520), (2503, 2048, 896), (520, 200, 2056), (1030, 6144, 1000)])
+def test_gemm2_grads(t, n, k):
+    """Input and weight gradient of a linear layer in one launch: bf16 and accumulating fp32 input gradient, results of the separate
+    products bit for bit where those sum whole tiles, ragged edges in every dimension."""
+    from polyrl_b200.ops import ext
+
+    C = ext()
+    dy, w, x = _randn(t, n, seed=1), _randn(n, k, seed=2, scale=0.05), _randn(t, k, seed=3)
+    dx, dw = C.gemm2_grads(dy, w, x)
+    for got, want in ((dx, dy.double() @ w.double()), (dw, dy.double().t() @ x.double())):
+        assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4 * want.abs().max()).all()
+    acc = _randn(t, k, seed=4, dtype=torch.float32)
+    ref = acc.double() + dy.double() @ w.double()
+    out = torch.empty(n + 8, k + 8, device="cuda", dtype=torch.bfloat16)[8:, 8:]
+    if out.data_ptr() % 16 == 0 and out.stride(0) % 8 == 0:
+        C.gemm2_grads(dy, w, x, out, acc, 1.0)
+        assert torch.equal(out, dw)
+        assert (acc.double() - ref).norm() <= n * 2.0 ** -27 * ref.norm() + 1e-6 * ref.norm()
