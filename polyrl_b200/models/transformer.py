@@ -20,6 +20,7 @@ import torch.nn.functional as F
 from .. import ops
 from ..ops import reference as ref
 from ..ops.attention import attention_varlen, rope_attention
+from ..ops.block import dense_block
 from ..ops.functional import gather_cached, head_norm_ok, head_norm_rope_and_cache_, rope_and_cache_
 from .config import ModelConfig
 
@@ -451,6 +452,12 @@ def layer_forward(cfg: ModelConfig, w: dict, x: torch.Tensor, inp: PackedInput, 
                                   f"({cfg.sliding_window}); windowed attention is not implemented, only the full-causal case")
     if cfg.family == "llama":
         lora = "_lora_scale" in w
+        if kv_sink is None and inp.sp_group is None and not lora and cfg.attn_type != "mla" and not cfg.sandwich_norm \
+                and "wgu" in w and "router" not in w and not w.get("_skip_mlp"):
+            pos, cos, sin = inp.rope_inputs(cfg, x.device)
+            y = dense_block(x, w, pos, cos, sin, inp.cu_seqlens, nq, nkv, d, cfg.rms_norm_eps)
+            if y is not None:
+                return y
         if lora:
             from . import lora as L
         h, x = ops.rmsnorm_residual(x, w["ln1"], cfg.rms_norm_eps)

@@ -252,3 +252,27 @@ def test_gemm2_grads(t, n, k):
         C.gemm2_grads(dy, w, x, out, acc, 1.0)
         assert torch.equal(out, dw)
         assert (acc.double() - ref).norm() <= n * 2.0 ** -27 * ref.norm() + 1e-6 * ref.norm()
+
+
+@pytest.mark.parametrize("model,lens", [("qwen2.5-0.5b", [3, 130]), ("qwen3-1.7b", [300, 1, 77]), ("llama3-8b", [40])])
+def test_dense_block_is_the_chain(model, lens, monkeypatch):
+    """The block as one function gives, bit for bit, what the chain of functions gives (its bias is added in the same place)."""
+    from polyrl_b200.models import get_model_config
+    from polyrl_b200.models import transformer as tf
+
+    cfg, t = get_model_config(model), sum(lens)
+    w = {n: _randn(*s, seed=i, scale=0.1 if len(s) == 1 else 0.02, shift=1.0 if n.startswith("ln") or n.endswith("norm") else 0.0).requires_grad_(True)
+         for i, (n, s) in enumerate(tf.layer_param_specs(cfg, 0))}
+    x, gy = _randn(t, cfg.hidden_size, seed=50).requires_grad_(True), _randn(t, cfg.hidden_size, seed=51)
+    cu = torch.tensor([0] + lens, dtype=torch.int32).cumsum(0).to(torch.int32).cuda()
+    inp = tf.PackedInput(torch.zeros(t, dtype=torch.long, device="cuda"), torch.cat([torch.arange(n) for n in lens]).cuda(), cu, max(lens))
+    y = tf.layer_forward(cfg, w, x, inp)
+    assert type(y.grad_fn).__name__.startswith("_DenseBlockFn")
+    got = [y, *torch.autograd.grad(y, [x, *w.values()], gy)]
+    monkeypatch.setattr(tf, "dense_block", lambda *a: None)
+    y = tf.layer_forward(cfg, w, x, inp)
+    for n, a, b in zip(["y", "x", *w], got, [y, *torch.autograd.grad(y, [x, *w.values()], gy)]):
+        assert torch.equal(a, b), n
+    w["wo"].requires_grad_(False)                        # a frozen weight: the chain, which leaves its gradient out
+    monkeypatch.undo()
+    assert not type(tf.layer_forward(cfg, w, x, inp).grad_fn).__name__.startswith("_DenseBlockFn")
