@@ -244,19 +244,21 @@ attn_bwd_keys_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     for (int w = blockIdx.x; item(w, t); w += gridDim.x) {
       const int key = t.k0 + r;
       // thread tid brings statistic tid >> 7 of query tid & 127, one tile ahead
-      auto fetch = [&](int it) {
-        const int h = t.hk * G + it / t.n_i, q = (t.i0 + it % t.n_i) * 128 + (tid & 127);
+      auto fetch = [&](int h, int tile) {
+        const int q = tile * 128 + (tid & 127);
         if (q >= t.lq) return 0.f;
-        const float2 st = p.stats[static_cast<int64_t>(h) * p.Tq + t.qs + q];
-        return tid >> 7 ? st.y : st.x;
+        return reinterpret_cast<const float*>(p.stats + static_cast<int64_t>(h) * p.Tq + t.qs + q)[tid >> 7];
       };
-      float ahead = t.iters > 0 ? fetch(0) : 0.f;
-      for (int it = 0; it < t.iters; ++it, ++n) {
-        const int q0 = (t.i0 + it % t.n_i) * 128;
+      const int tiles_end = t.i0 + t.n_i;
+      int tile = t.i0, h_next = t.hk * G, tile_next = t.i0;
+      float ahead = t.iters > 0 ? fetch(h_next, tile_next) : 0.f;
+      for (int it = 0; it < t.iters; ++it, ++n, tile = tile_next) {
+        const int q0 = tile * 128;
+        if (++tile_next == tiles_end) { tile_next = t.i0; ++h_next; }
         float* st = stat + (n & 1) * 256;
         st[tid] = ahead;
         asm volatile("bar.sync 1, 256;" ::: "memory");    // (a stage is overwritten two tiles later: everyone has passed the barrier between)
-        if (it + 1 < t.iters) ahead = fetch(it + 1);
+        if (it + 1 < t.iters) ahead = fetch(h_next, tile_next);
         const bool whole = q0 + 127 < t.lq && t.k0 + 127 < t.lk && (!p.causal || t.k0 + 127 <= q0 + t.off);
         // this thread's 64 queries that see its key: [seen_lo, seen_lo + seen_n)
         const int seen_lo = p.causal ? max(0, key - t.off - q0 - g * 64) : 0;
