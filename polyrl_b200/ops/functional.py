@@ -107,6 +107,11 @@ def _is_decode_shape(x2: torch.Tensor, w: torch.Tensor) -> bool:
     return (not torch.is_grad_enabled() or not (x2.requires_grad or w.requires_grad)) and x2.shape[0] <= _SKINNY_MAX_ROWS
 
 
+def _streams(w: torch.Tensor) -> bool:
+    """Weights as the stream kernel's tensor map takes them."""
+    return w.dim() == 2 and w.stride(1) == 1 and w.stride(0) % 8 == 0 and w.data_ptr() % 16 == 0
+
+
 def _use_skinny(x2: torch.Tensor, w: torch.Tensor) -> bool:
     if _cublas() or _decode_policy() != "skinny":
         return False
@@ -286,6 +291,13 @@ def linear_swiglu(x: torch.Tensor, wgu: torch.Tensor) -> torch.Tensor:
     if isinstance(wgu, Fp8Weight):
         return _linear_fp8(x, wgu, swiglu=True)
     if _is_kernel_tensor(x) and wgu.dtype == torch.bfloat16 and x.dim() == 2 and _use_skinny(x, wgu):
+        return skinny_linear(x, wgu, None, None, 1)
+    if _is_kernel_tensor(x) and wgu.dtype == torch.bfloat16 and x.dim() == 2 and _decode_policy() == "auto" and not _cublas() \
+            and _is_decode_shape(x, wgu) and 0 < x.shape[0] <= 128 and wgu.shape[0] <= 74 * 256 and wgu.shape[0] % 256 == 0 \
+            and x.shape[1] % 16 == 0 and x.data_ptr() % 16 == 0 and _streams(wgu):
+        # The tile kernel has one CTA per 256 weight rows: with fewer than half the SMs it cannot draw the weights fast enough.  The stream
+        # kernel splits the reduction over clusters.  [12288, 2048], 16 / 45 / 128 rows: 24.5 -> 16.5 / 18.1 / 23.5 us; at 256 rows, or
+        # with 28672 weight rows (112 CTAs: 53 against 60 us at 45 rows), the tile kernel is the faster one.
         return skinny_linear(x, wgu, None, None, 1)
     if _is_kernel_tensor(x) and wgu.dtype == torch.bfloat16 and not _cublas():
         return _LinearSwigluFn.apply(x, wgu)
