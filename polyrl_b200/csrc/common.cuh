@@ -347,6 +347,17 @@ __device__ __forceinline__ void wait_ge_sys(const uint32_t* p, uint32_t target) 
   }
 }
 
+// Kernels of a decode step are a few microseconds long, and two or three more pass between the last block of one and the first loads of the
+// next.  A kernel launched by launch_behind may start while the one before it on the stream still runs; every thread of it calls
+// grid_behind() before it reads or writes anything that another kernel touches.  That waits until the kernel before is complete, and only
+// then lets the next one start: whatever runs at the same time is the pair, and all kernels before the pair are complete.
+// Decode step of two 7B blocks and head, 45 sequences, fp8 weights: 504 -> 454 us; 8B bf16, 128 sequences: about 4%.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_behind() {
+  grid_wait();
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __device__ __forceinline__ int4 ld_nc_v4(const void* p) {
   int4 r;
   asm volatile("ld.global.nc.L1::no_allocate.v4.s32 {%0, %1, %2, %3}, [%4];"
@@ -415,6 +426,22 @@ __device__ __forceinline__ int find_row_tile(const int32_t* __restrict__ cu, int
 }
 
 }  // namespace prl
+
+// <<<grid, block, smem, stream>>> for kernels that call grid_behind()
+template <class... P, class... A>
+inline cudaError_t launch_behind(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... a) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(a)...);
+}
 
 // cuTensorMapEncodeTiled is a driver call and needs a context bound to the calling thread.  A fresh thread (an autograd worker
 // whose first op is one of our GEMMs on a cached buffer) has made no runtime call yet, so bind the primary context once.

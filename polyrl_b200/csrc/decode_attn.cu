@@ -55,6 +55,7 @@ paged_decode_kernel(const __nv_bfloat16* __restrict__ q, int64_t ldq,     // [nu
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gq = lane >> 2, qd = lane & 3;    // fragment row / quad index
 
+  grid_behind();
   const int len = seq_lens[seq];
   // visible keys: the last `window` and the first `keep_first`; their pages are numbered 0, 1, ... across the gap between the two
   const int first = max(0, len - window);
@@ -243,6 +244,7 @@ __global__ void decode_merge_kernel(const float* __restrict__ o_part, const floa
                                     const float* __restrict__ sink, __nv_bfloat16* __restrict__ out, int64_t ldo, int nq) {
   const int seq = blockIdx.x / nq, head = blockIdx.x % nq;
   const int64_t base = (static_cast<int64_t>(seq) * nq + head) * splits;
+  grid_behind();
   float mm = -INFINITY;
   for (int s = 0; s < splits; ++s) mm = fmaxf(mm, ml_part[(base + s) * 2]);
   float ll = 0.f;
@@ -324,19 +326,19 @@ extern "C" int prl_paged_decode(const void* q, int64_t ldq, const void* k_cache,
   static const int minb = [] { const char* e = getenv("POLYRL_DECODE_MINB"); return e ? atoi(e) : 3; }();
   if (d == 128) {
     auto kern = minb >= 4 ? paged_decode_kernel<128, 128, 1, 4> : paged_decode_kernel<128, 128, 1, 3>;
-    kern<<<grid, kAttnWarps * 32, 0, s>>>(
-        static_cast<const __nv_bfloat16*>(q), ldq, static_cast<const __nv_bfloat16*>(k_cache),
+    launch_behind(
+        kern, grid, kAttnWarps * 32, 0, s, static_cast<const __nv_bfloat16*>(q), ldq, static_cast<const __nv_bfloat16*>(k_cache),
         static_cast<const __nv_bfloat16*>(v_cache), block_table, ld_bt, seq_lens, nq, nkv, splits, scale_log2, window, keep_first, nullptr, o_part,
         ml_part, splits == 1 ? static_cast<__nv_bfloat16*>(out) : nullptr, ldo);
     if (splits > 1)
-      decode_merge_kernel<128><<<num_seqs * nq, 128, 0, s>>>(o_part, ml_part, splits, nullptr, static_cast<__nv_bfloat16*>(out), ldo, nq);
+      launch_behind(decode_merge_kernel<128>, num_seqs * nq, 128, 0, s, o_part, ml_part, splits, nullptr, static_cast<__nv_bfloat16*>(out), ldo, nq);
   } else if (d == 64) {
-    paged_decode_kernel<64, 64, 1, 3><<<grid, kAttnWarps * 32, 0, s>>>(
-        static_cast<const __nv_bfloat16*>(q), ldq, static_cast<const __nv_bfloat16*>(k_cache),
+    launch_behind(
+        paged_decode_kernel<64, 64, 1, 3>, grid, kAttnWarps * 32, 0, s, static_cast<const __nv_bfloat16*>(q), ldq, static_cast<const __nv_bfloat16*>(k_cache),
         static_cast<const __nv_bfloat16*>(v_cache), block_table, ld_bt, seq_lens, nq, nkv, splits, scale_log2, window, keep_first, nullptr, o_part,
         ml_part, splits == 1 ? static_cast<__nv_bfloat16*>(out) : nullptr, ldo);
     if (splits > 1)
-      decode_merge_kernel<64><<<num_seqs * nq, 64, 0, s>>>(o_part, ml_part, splits, nullptr, static_cast<__nv_bfloat16*>(out), ldo, nq);
+      launch_behind(decode_merge_kernel<64>, num_seqs * nq, 64, 0, s, o_part, ml_part, splits, nullptr, static_cast<__nv_bfloat16*>(out), ldo, nq);
   } else {
     return -31;
   }

@@ -120,6 +120,15 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
+  if (warp == 0 && lane == 0) {
+    // Behind the kernel before: its last blocks still run.  The first weights may come into L2 meanwhile, where a later write to them
+    // would still be seen; nothing is read into the SM yet.
+    for (int kb = kb0; kb < min(kb1, kb0 + stages); ++kb) {
+      tma_prefetch_l2_2d(&tmW, kb * BLOCK_K, row_g);
+      tma_prefetch_l2_2d(&tmW, kb * BLOCK_K, row_u);
+    }
+  }
+  grid_behind();
   if (warp == 0) {
     if (lane == 0) {
       int stage = 0; uint32_t phase = 0;
@@ -348,13 +357,15 @@ static int launch_stream(const void* X, const void* W, StreamParams p, int64_t l
   cfg.blockDim = dim3(kSgThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = p.S * NC;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   PRL_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tmW, tmX, p));
   return 0;
 }

@@ -11,6 +11,7 @@ namespace prl {
 
 constexpr int kNormThreads = 256;
 constexpr int kMaxVPT = 4;   // up to H = 256*8*4 = 8192
+constexpr int kStepRows = 256;   // rows of a decode step: launched behind the kernel before
 
 __device__ __forceinline__ float block_sum_256(float v, float* red) {
   v = warp_sum(v);
@@ -45,6 +46,7 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   __shared__ float red[2][THREADS / 32];
   const int nvec = H >> 3;
   int4 wv[VPT], xv[VPT];
+  grid_behind();
   auto load = [&](int row) {
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
@@ -103,6 +105,7 @@ add_rmsnorm_kernel(__nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restric
                    __nv_bfloat16* __restrict__ y, int T, int H, float eps) {
   __shared__ float red[8];
   const int nvec = H >> 3;
+  grid_behind();
   for (int row = blockIdx.x; row < T; row += gridDim.x) {
     __nv_bfloat16* xr = x + static_cast<int64_t>(row) * H;
     const __nv_bfloat16* rr = r + static_cast<int64_t>(row) * H;
@@ -371,6 +374,7 @@ __global__ void __launch_bounds__(256)
 quant_fp8_rowwise_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scale,
                          int T, int H) {
   __shared__ float red[8];
+  grid_behind();
   for (int row = blockIdx.x; row < T; row += gridDim.x) {
     const __nv_bfloat16* xr = x + static_cast<int64_t>(row) * H;
     float amax = 0.f;
@@ -432,8 +436,11 @@ extern "C" int prl_rmsnorm_fwd(const void* x, const void* w, void* y, float* rst
   norm_shape(H, [&](auto threads, auto vpt) {
     constexpr int kT = decltype(threads)::value;
     const int most = 148 * (2048 / kT / 2), grid = T < most ? T : most;       // 1024 threads an SM: two rows' loads in flight for each
-    rmsnorm_fwd_kernel<kT, decltype(vpt)::value><<<grid, kT, 0, s>>>(static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w),
-                                                                    static_cast<__nv_bfloat16*>(y), rstd, T, H, eps);
+    auto kern = rmsnorm_fwd_kernel<kT, decltype(vpt)::value>;
+    const auto* xb = static_cast<const __nv_bfloat16*>(x);
+    const auto* wb = static_cast<const __nv_bfloat16*>(w);
+    if (T <= kStepRows) launch_behind(kern, grid, kT, 0, s, xb, wb, static_cast<__nv_bfloat16*>(y), rstd, T, H, eps);
+    else kern<<<grid, kT, 0, s>>>(xb, wb, static_cast<__nv_bfloat16*>(y), rstd, T, H, eps);
   });
   PRL_CUDA_CHECK(cudaGetLastError());
   return 0;
@@ -442,8 +449,11 @@ extern "C" int prl_add_rmsnorm(void* x, const void* r, const void* w, void* y, i
   if (H % 8 != 0 || H > 8 * kNormThreads * kMaxVPT) return -20;
   if (T <= 0) return 0;
   const int grid = T < 148 * 8 ? T : 148 * 8;
-  add_rmsnorm_kernel<<<grid, kNormThreads, 0, s>>>(static_cast<__nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(r),
-                                                  static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(y), T, H, eps);
+  auto* xb = static_cast<__nv_bfloat16*>(x);
+  const auto* rb = static_cast<const __nv_bfloat16*>(r);
+  const auto* wb = static_cast<const __nv_bfloat16*>(w);
+  if (T <= kStepRows) launch_behind(add_rmsnorm_kernel, grid, kNormThreads, 0, s, xb, rb, wb, static_cast<__nv_bfloat16*>(y), T, H, eps);
+  else add_rmsnorm_kernel<<<grid, kNormThreads, 0, s>>>(xb, rb, wb, static_cast<__nv_bfloat16*>(y), T, H, eps);
   PRL_CUDA_CHECK(cudaGetLastError());
   return 0;
 }
@@ -506,8 +516,9 @@ extern "C" int prl_quant_fp8_rowwise(const void* x, void* q, float* scale, int T
   if (H % 8 != 0) return -22;
   if (T <= 0) return 0;
   const int grid = T < 148 * 8 ? T : 148 * 8;
-  quant_fp8_rowwise_kernel<<<grid, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q), scale,
-                                                T, H);
+  const auto* xb = static_cast<const __nv_bfloat16*>(x);
+  if (T <= kStepRows) launch_behind(quant_fp8_rowwise_kernel, grid, 256, 0, s, xb, static_cast<uint8_t*>(q), scale, T, H);
+  else quant_fp8_rowwise_kernel<<<grid, 256, 0, s>>>(xb, static_cast<uint8_t*>(q), scale, T, H);
   PRL_CUDA_CHECK(cudaGetLastError());
   return 0;
 }

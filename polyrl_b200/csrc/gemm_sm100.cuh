@@ -102,6 +102,7 @@ struct AccReader {
 // the TMA producer consults `Comm::wait_n_block` before touching the rows of B of an n-block.
 struct NoComm {
   struct Params {};
+  static constexpr bool kBehind = false;           // launched behind the kernel before it (launch_behind)
   static constexpr int kCommWarps = 0;
   __device__ __forceinline__ static void wait_n_block(const Params&, int /*n_blk*/) {}
   __device__ __forceinline__ static void run(const Params&, int /*tid*/) {}
@@ -161,6 +162,13 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if constexpr (Gate::kBehind) {                     // the first weights may come into L2 before the kernel before is complete
+    if (warp == 0 && lane == 0 && static_cast<int>(blockIdx.x) < total_work) {
+      const int nb = decode_work(blockIdx.x, num_m_blocks, num_n_blocks, n_splits, nb_per_split, sc).n_begin;
+      for (int kb = 0; kb < min(num_kb, kStages); ++kb) tma_prefetch_l2_2d(&tmB, kb * Cfg::BLOCK_K, nb * BN);
+    }
+    grid_behind();
+  }
 
   if (warp == 0) {
     // ================================ TMA producer ================================
@@ -336,8 +344,12 @@ int launch_gemm(const void* A, const void* B, int M, int N, int K, int64_t lda_b
   if (max_ctas > 0 && max_ctas < ctas) ctas = max_ctas;
   const int total = num_m_blocks * n_splits;
   if (total < ctas && !full_grid) ctas = total;
-  kern<<<ctas, kNumThreads + 32 * Gate::kCommWarps, Cfg::SMEM_BYTES, stream>>>(
-      tmA, tmB, ep, gp, M, N, K, num_m_blocks, num_n_blocks, n_splits, nb_per_split, sc);
+  if constexpr (Gate::kBehind)
+    PRL_CUDA_CHECK(launch_behind(kern, ctas, kNumThreads, Cfg::SMEM_BYTES, stream, tmA, tmB, ep, gp, M, N, K, num_m_blocks, num_n_blocks, n_splits,
+                                 nb_per_split, sc));
+  else
+    kern<<<ctas, kNumThreads + 32 * Gate::kCommWarps, Cfg::SMEM_BYTES, stream>>>(
+        tmA, tmB, ep, gp, M, N, K, num_m_blocks, num_n_blocks, n_splits, nb_per_split, sc);
   PRL_CUDA_CHECK(cudaGetLastError());
   return 0;
 }

@@ -259,6 +259,12 @@ extern "C" int prl_gemm_fp8(const void* A, const void* B, void* D, const float* 
   }
 }
 
+namespace prl {
+struct Behind : NoComm {
+  static constexpr bool kBehind = true;
+};
+}  // namespace prl
+
 // H = silu(A·Wg^T) * (A·Wu^T) with W_gu block-interleaved ([128 gate | 128 up] per 256 rows).
 extern "C" int prl_gemm_swiglu_bf16(const void* A, const void* Wgu, void* H, void* GU, int M, int N2, int K,
                                     int64_t lda, int64_t ldw, int64_t ldh, int64_t ldgu, float* ws, cudaStream_t stream) {
@@ -269,7 +275,7 @@ extern "C" int prl_gemm_swiglu_bf16(const void* A, const void* Wgu, void* H, voi
     return launch_gemm2<Cfg2, EpiSwiglu>(A, Wgu, nullptr, M, N2, K, lda * 2, ldw * 2, 0, sp, 0, stream, Sched{0, 1, 0}, ws);
   }
   using Cfg = GemmCfg<256, 2>;
-  return launch_gemm<Cfg, EpiSwiglu, NoGate, false>(A, Wgu, M, N2, K, lda * 2, ldw * 2, sp, NoGate::Params{}, 0, 0,
+  return launch_gemm<Cfg, EpiSwiglu, Behind, false>(A, Wgu, M, N2, K, lda * 2, ldw * 2, sp, Behind::Params{}, 0, 0,
                                                     stream);
 }
 

@@ -59,6 +59,7 @@ __device__ __forceinline__ float head_sum(float v) {
 template <int D, bool NORM>
 __global__ void __launch_bounds__(kQrThreads) qk_rope_kernel(QkRopeParams p) {
   constexpr int L = D / 16, HALF = D / 2;
+  grid_behind();
   const int heads = p.nq + p.nkv + (p.slots != nullptr ? p.nkv : 0);
   const int64_t item = (static_cast<int64_t>(blockIdx.x) * kQrThreads + threadIdx.x) / L;
   if (item >= static_cast<int64_t>(p.T) * heads) return;                  // (whole heads leave together)
@@ -217,8 +218,9 @@ template <int D>
 static void launch_qk_rope(const QkRopeParams& p, cudaStream_t s) {
   const int64_t heads = p.nq + p.nkv + (p.slots != nullptr ? p.nkv : 0), threads = p.T * heads * (D / 16);
   const unsigned grid = static_cast<unsigned>((threads + kQrThreads - 1) / kQrThreads);
-  if (p.qn != nullptr) qk_rope_kernel<D, true><<<grid, kQrThreads, 0, s>>>(p);
-  else qk_rope_kernel<D, false><<<grid, kQrThreads, 0, s>>>(p);
+  auto kern = p.qn != nullptr ? qk_rope_kernel<D, true> : qk_rope_kernel<D, false>;
+  if (p.T <= 256) launch_behind(kern, grid, kQrThreads, 0, s, p);       // a decode step
+  else kern<<<grid, kQrThreads, 0, s>>>(p);
 }
 
 }  // namespace prl

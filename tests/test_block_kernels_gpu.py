@@ -276,3 +276,31 @@ def test_dense_block_is_the_chain(model, lens, monkeypatch):
     w["wo"].requires_grad_(False)                        # a frozen weight: the chain, which leaves its gradient out
     monkeypatch.undo()
     assert not type(tf.layer_forward(cfg, w, x, inp).grad_fn).__name__.startswith("_DenseBlockFn")
+
+
+def test_decode_kernels_behind_each_other():
+    """Kernels of a decode step may start while the one before still runs: a chain in which each reads what the last one wrote, its buffers
+    freed and taken again on the way, gives the same values as with a wait after every kernel."""
+    from polyrl_b200.ops import ext
+
+    C, b, h, f = ext(), 45, 1024, 2048
+    wq = [OF.quantize_weight_fp8(_randn(*s, seed=i, scale=0.03)) for i, s in enumerate([(2 * f, h), (h, f)])]
+    norm = _randn(h, seed=5, scale=0.1, shift=1.0)
+
+    def chain(wait):
+        x = _randn(b, h, seed=9)
+        sync = torch.cuda.synchronize if wait else (lambda: None)
+        y = ops.rmsnorm(x, norm)
+        for _ in range(30):
+            sync()
+            g = OF._linear_fp8(y, wq[0], swiglu=True)
+            sync()
+            d = OF._linear_fp8(g, wq[1])
+            sync()
+            y = C.add_rmsnorm_(x, d, norm, 1e-6)
+        return x, y
+
+    with torch.no_grad():
+        want = chain(True)
+        for _ in range(5):
+            assert all(torch.equal(a, c) for a, c in zip(chain(False), want))
