@@ -447,6 +447,13 @@ def gather_cached(k_cache: torch.Tensor, v_cache: torch.Tensor, blk: torch.Tenso
 _CE_CHUNK = int(os.environ.get("POLYRL_CE_BWD_CHUNK", "16384"))
 
 
+def _ce_slice(rows: int) -> int:
+    """Vocabulary columns whose logit gradients are held at a time.  Up to 6144 rows two of the usual slices together are no larger than one
+    is at 12288 rows (400 MB), and longer reductions and fewer launches win: [2503, 896] x 151936 forward and backward 2277 -> 2163 us; four
+    together lose it again (2409), as the two products of a slice no longer share the chip well."""
+    return _CE_CHUNK if rows > 6144 or "POLYRL_CE_BWD_CHUNK" in os.environ else 2 * _CE_CHUNK
+
+
 class _LinearCEFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, hidden, weight, labels, inv_tau):
@@ -471,8 +478,9 @@ class _LinearCEFn(torch.autograd.Function):
         own = not _cublas() and h2.shape[1] % 8 == 0
         dh = (torch.empty if own else torch.zeros)(h2.shape, device=h2.device, dtype=torch.float32) if need_h else None
         dw = torch.empty_like(w) if need_w else None
-        for v0 in range(0, V, _CE_CHUNK):
-            v1 = min(V, v0 + _CE_CHUNK)
+        step = _ce_slice(h2.shape[0])
+        for v0 in range(0, V, step):
+            v1 = min(V, v0 + step)
             ws = w[v0:v1]
             dz = C.linear_ce_dz(h2, ws, lab, lse, ez, g_lp, g_ent, ctx.inv_tau, v0)
             if need_h and need_w and own and w.stride(1) == 1 and w.stride(0) % 8 == 0 and ws.data_ptr() % 16 == 0 and h2.data_ptr() % 16 == 0:
