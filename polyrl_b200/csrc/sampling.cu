@@ -175,6 +175,7 @@ sample_kernel(const T* __restrict__ logits, int64_t ld, int V, const float* __re
   __shared__ Part part[kSampleWarps];
   __shared__ Part of_cta[kSampleCtas];
   cg::cluster_group cluster = cg::this_cluster();
+  cluster_arrive();                     // waited for before the first store into another CTA: all CTAs of the cluster run by then
   const int rank = static_cast<int>(cluster.block_rank()), ctas = static_cast<int>(cluster.num_blocks());
   const int row = blockIdx.x / ctas;
   const Row r(logits + static_cast<int64_t>(row) * ld, V);
@@ -221,6 +222,7 @@ sample_kernel(const T* __restrict__ logits, int64_t ld, int V, const float* __re
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
   if (l == 0) part[w] = Part{best, m, s};
   __syncthreads();
+  cluster_wait();
   if (threadIdx.x == 0) {
     Part t = part[0];
     for (int i = 1; i < static_cast<int>(blockDim.x >> 5); ++i) {
@@ -273,6 +275,7 @@ sample_topk_topp_kernel(const T* __restrict__ logits, int64_t ld, int V, const f
   __shared__ uint32_t s_bin, bar;
   __shared__ double s_rest;
   cg::cluster_group cluster = cg::this_cluster();
+  cluster_arrive();                                       // as above
   const int rank = static_cast<int>(cluster.block_rank()), ctas = static_cast<int>(cluster.num_blocks());
   const int row = blockIdx.x / ctas, tid = threadIdx.x, w = tid >> 5, l = tid & 31;
   const Row r(logits + static_cast<int64_t>(row) * ld, V);
@@ -311,6 +314,7 @@ sample_topk_topp_kernel(const T* __restrict__ logits, int64_t ld, int V, const f
   if (l == 0) part[w].mass = m;
   if (tid == 0) bar = order_key(-INFINITY);
   __syncthreads();
+  cluster_wait();
   if (tid < ctas) {
     float t = part[0].mass;
     for (int i = 1; i < kSampleWarps; ++i) t = fmaxf(t, part[i].mass);

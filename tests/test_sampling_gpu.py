@@ -71,3 +71,11 @@ def test_choice_and_log_prob(C, dtype, b, v, offset, top_k, top_p):
         # the kernel's fast logarithm is 4e-7 off near one, where noise of up to log(2^24) comes from: 4e-7 e^11 relative for the
         # best of 65 K, so a choice may differ only where two keys are that close
         assert float(key.max() - key[k]) < 0.05
+
+
+@pytest.mark.parametrize("b,v,offset", [(1, 2, 0), (2, 5, 1), (16, 17, 0), (18, 40, 3)])
+@pytest.mark.parametrize("top_k,top_p", [(-1, 1.0), (3, 0.9)])
+def test_rows_with_less_than_a_granule_a_block(C, b, v, offset, top_k, top_p):
+    """Rows so short that most CTAs of a row's cluster have nothing to read and hand their part over at once."""
+    for _ in range(20):
+        test_choice_and_log_prob(C, torch.bfloat16, b, v, offset, top_k, top_p)
