@@ -127,11 +127,12 @@ __device__ __forceinline__ void offer_granule(Pick& best, float bar, const float
       }
   }
 }
-// The CTA's best key so far (as an order key), which every warp raises; a late read only prunes less.
+// The CTA's best key so far (as an order key), which every warp raises; a late read only prunes less.  Lanes may read different values while
+// other warps raise it, so the warp agrees on the largest: callers branch on the result around collectives of the whole warp.
 __device__ __forceinline__ float raise_bar(uint32_t* bar, const Pick& best) {
-  const uint32_t k = __reduce_max_sync(0xffffffffu, order_key(best.key)), b = *const_cast<volatile uint32_t*>(bar);
+  const uint32_t b = *const_cast<volatile uint32_t*>(bar), k = __reduce_max_sync(0xffffffffu, max(order_key(best.key), b));
   if (k > b && (threadIdx.x & 31) == 0) atomicMax(bar, k);
-  return from_order_key(k > b ? k : b);
+  return from_order_key(k);
 }
 
 __device__ __forceinline__ Pick warp_pick(Pick p) {

@@ -79,3 +79,23 @@ def test_rows_with_less_than_a_granule_a_block(C, b, v, offset, top_k, top_p):
     """Rows so short that most CTAs of a row's cluster have nothing to read and hand their part over at once."""
     for _ in range(20):
         test_choice_and_log_prob(C, torch.bfloat16, b, v, offset, top_k, top_p)
+
+
+@pytest.mark.parametrize("top_k,top_p", [(-1, 1.0), (50, 0.9)])
+def test_stretches_without_a_candidate(C, top_k, top_p):
+    """Whole warps and whole turns of a CTA see masked logits only, others of the same row do not."""
+    b, v = 5, 40000
+    torch.manual_seed(v)
+    for turn in range(20):
+        z = torch.randn(b, v, device="cuda")
+        z.masked_fill_((torch.rand(b, -(-v // 256), device="cuda") < (0.5, 0.97)[turn & 1]).repeat_interleave(256, 1)[:, :v], -math.inf)
+        z[:, turn * 1999] = 1.0
+        z = z.bfloat16()
+        seeds = torch.randint(0, 2 ** 62, (b,), device="cuda")
+        t = torch.full((b,), 0.8, device="cuda")
+        tok, lp = C.sample(z, t, seeds, False, False) if top_k < 0 else C.sample_topk_topp(z, t, seeds, False, top_k, top_p, False)
+        raw = z.gather(1, tok[:, None])[:, 0]
+        assert torch.isfinite(raw).all() and torch.isfinite(lp).all()
+        if top_k < 0:
+            want = (z.double() / 0.8).log_softmax(-1).gather(1, tok[:, None])[:, 0]
+            assert ((lp - want).abs() <= 1e-5 * want.abs().clamp_min(1)).all()       # fp32 sums, as above
