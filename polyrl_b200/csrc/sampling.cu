@@ -31,7 +31,8 @@ __device__ __forceinline__ uint32_t noise_hash(uint64_t seed, uint32_t row, uint
   return x;
 }
 __device__ __forceinline__ float gumbel_of(uint32_t x) {
-  const float u = (static_cast<float>((x ^ (x >> 16)) >> 8) + 0.5f) * (1.0f / 16777216.0f);
+  // (the largest number of 24 bits and a half would round to 2^24: infinite noise, which wins over any logit)
+  const float u = (static_cast<float>(min((x ^ (x >> 16)) >> 8, 0xfffffeu)) + 0.5f) * (1.0f / 16777216.0f);
   return -__logf(-__logf(u));
 }
 // Hashes below this give noise that is certainly less than `need`.  The 24 bits must reach 2^24 exp(-exp(-need)), less a margin of 256

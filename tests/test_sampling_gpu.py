@@ -99,3 +99,40 @@ def test_stretches_without_a_candidate(C, top_k, top_p):
         if top_k < 0:
             want = (z.double() / 0.8).log_softmax(-1).gather(1, tok[:, None])[:, 0]
             assert ((lp - want).abs() <= 1e-5 * want.abs().clamp_min(1)).all()       # fp32 sums, as above
+
+
+def _unhash(h):
+    """x with _hash(x) == h: every step of the mixer has an inverse."""
+    m = 0xFFFFFFFF
+    x = h ^ (h >> 16)
+    x = (x * pow(0x846CA68B, -1, 1 << 32)) & m
+    x = x ^ (x >> 15) ^ (x >> 30)
+    x = (x * pow(0x7FEB352D, -1, 1 << 32)) & m
+    return x ^ (x >> 16)
+
+
+def _seed_for(bits, col, low):
+    """A seed whose noise for element ``col`` of row 0 is made from the given 24 bits."""
+    high = _unhash(bits << 8 | 0x5A) ^ _hash(_hash((col + 0x9E3779B9) & 0xFFFFFFFF) ^ low)
+    s = high << 32 | low
+    return s - (1 << 64) if s >> 63 else s
+
+
+@pytest.mark.parametrize("bits", [0, 1, 12345678, 0xFFFFF0, 0xFFFFFD, 0xFFFFFE, 0xFFFFFF])
+@pytest.mark.parametrize("top_k", [-1, 2])
+def test_noise_at_its_ends(C, bits, top_k):
+    """Two elements, the first with noise from given bits, against the noise in 64 bits: it wins with a logit that is 1 more than needed and
+    loses with one that is 1 less.  Over all 2^24 values the noise is at most 0.84 from that, at the last three: there u is rounded to a
+    multiple of 2^-23 and the fast logarithm of it is off by 0.4 of its value."""
+    for low in (1, 77, 0xDEADBEEF):
+        seed = _seed_for(bits, 0, low)
+        other = _hash(_hash((1 + 0x9E3779B9) & 0xFFFFFFFF) ^ low)
+        other = _hash(other ^ ((seed >> 32) & 0xFFFFFFFF)) >> 8
+        assert _hash(_hash(_hash(0x9E3779B9) ^ low) ^ ((seed >> 32) & 0xFFFFFFFF)) >> 8 == bits
+        first, second = (-math.log(-math.log((b + 0.5) / 2 ** 24)) for b in (bits, other))
+        for more in (1.0, -1.0):
+            z = torch.tensor([[second - first + more, 0.0, -math.inf]], device="cuda")
+            s, t = torch.tensor([seed], device="cuda"), torch.ones(1, device="cuda")
+            tok, lp = C.sample(z, t, s, False, False) if top_k < 0 else C.sample_topk_topp(z, t, s, False, top_k, 1.0, False)
+            assert int(tok) == (0 if more > 0 else 1), (bits, low, more)
+            assert abs(float(lp) - float(z.double().log_softmax(-1)[0, int(tok)])) < 1e-4
