@@ -388,6 +388,7 @@ sample_topk_topp_kernel(const T* __restrict__ logits, int64_t ld, int V, const f
       __syncthreads();
       prefix = (prefix << (hi - lo)) | s_bin;
       want = s_rest;
+      if (want <= 0.) return prefix << lo;
       share = false;
       hi = lo;
     }

@@ -136,3 +136,26 @@ def test_noise_at_its_ends(C, bits, top_k):
             tok, lp = C.sample(z, t, s, False, False) if top_k < 0 else C.sample_topk_topp(z, t, s, False, top_k, 1.0, False)
             assert int(tok) == (0 if more > 0 else 1), (bits, low, more)
             assert abs(float(lp) - float(z.double().log_softmax(-1)[0, int(tok)])) < 1e-4
+
+
+def _noise_of(seed, col):
+    """Noise of one element of row 0, in 64 bits."""
+    n = _hash(_hash((col + 0x9E3779B9) & 0xFFFFFFFF) ^ (seed & 0xFFFFFFFF))
+    return -math.log(-math.log(((_hash(n ^ (seed >> 32 & 0xFFFFFFFF)) >> 8) + 0.5) / 2 ** 24))
+
+
+def _seeds_for(col, most):
+    """Seeds that give element ``col`` the largest noise (16.5) and element 0 at most ``most``."""
+    return [s for s in (_seed_for(0xFFFFFE, col, low) for low in range(1, 4000)) if _noise_of(s, 0) < most][:8]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_nucleus_of_everything(C, dtype):
+    """The largest top_p below one, and weights 1 and three of 0.7 * 2^-23: sums of 24 bits round each of the three up, and the mass asked for
+    is then more than what the later digits of the keys find.  All of the row is kept, the elements at the low end of a digit among them."""
+    z = torch.full((1, 4096), -math.inf, device="cuda")
+    z[0, 0], z[0, 1:4] = 25.5, 2.0                          # 23.5 ln 2 = 16.29 apart
+    z, scale = z.to(dtype), torch.full((1,), math.log(2.0), device="cuda")
+    for seed in _seeds_for(1, 0.1):
+        tok, _ = C.sample_topk_topp(z, scale, torch.tensor([seed], device="cuda"), False, -1, 1 - 2.0 ** -24, True)
+        assert int(tok) == 1
