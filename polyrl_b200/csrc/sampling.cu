@@ -253,12 +253,26 @@ sample_kernel(const T* __restrict__ logits, int64_t ld, int V, const float* __re
 // 3rdparty/verl/verl/trainer/config/rollout/rollout.yaml).
 //
 // Logits share a few exponents, so a histogram with shared-memory atomics runs one element after the other.  Here every thread owns a
-// column of 64 bins in shared memory ([bin][thread]: no bank conflict, no atomic), the columns are summed in a fixed order, then the CTAs'
-// sums over the cluster: the cut does not depend on timing (tensor-parallel engine ranks must sample identically).  Every pass reads the
-// row again, from L2: kept in registers (40 a thread at 152 K logits) or shared memory it would cost the third CTA of an SM.
-// [47, 151936] bf16, top_p 0.95: 46 us; with 64-bit atomics on 256 bins, one CTA per row and scalar loads it was 1808.
+// column of 64 counts or 32 masses in shared memory ([bin][thread]: no bank conflict, no atomic), then the CTAs' sums meet over the cluster.
+// Masses are whole numbers of 2^-40, so a digit's bins add up to the bin of the digit before, in any order, and the cut does not depend on
+// timing (tensor-parallel engine ranks must sample identically).  Every pass reads the row again, from L2: kept in registers (40 a thread
+// at 152 K logits) or shared memory it would cost the third CTA of an SM.
+// [47, 151936] bf16, top_p 0.95: 61 us.  With fp32 masses, which allow 64 bins and three passes instead of four, it was 47, but the cut moved
+// where masses tie within 2^-24; with 64-bit atomics on 256 bins, one CTA per row and scalar loads it was 1808.
 // ------------------------------------------------------------------------------------------------------------------
-constexpr int kBins = 64;
+constexpr int kBins = 64;               // most bins
+constexpr float kMassUnits = 1099511627776.f;        // 2^40
+struct CountDigits {
+  using Sum = uint32_t;
+  static constexpr bool mass = false;
+  static constexpr int BITS = 6;
+};
+struct MassDigits {
+  using Sum = uint64_t;
+  static constexpr bool mass = true;
+  static constexpr int BITS = 5;
+};
+constexpr int kHistBytes = kSampleThreads * 256;     // 64 counts or 32 masses a thread
 
 template <typename T>
 __global__ void __launch_bounds__(kSampleThreads, 3)
@@ -268,14 +282,14 @@ sample_topk_topp_kernel(const T* __restrict__ logits, int64_t ld, int V, const f
   using Row = SampleRow<T>;
   constexpr int N = Row::N;
   constexpr int KEY_BITS = 8 * static_cast<int>(sizeof(T));
-  extern __shared__ float hist[];                         // [kBins][kSampleThreads]; counts are stored as integers
+  extern __shared__ uint64_t hist[];                      // a column of sums for every thread
   struct Part { Pick pick; float mass; };
   __shared__ Part part[kSampleWarps];
   __shared__ Part of_cta[kSampleCtas];
-  __shared__ double sums[2][kSampleCtas][kBins];          // every CTA holds all CTAs' sums; two passes alternate
+  __shared__ uint64_t sums[2][kSampleCtas][kBins];        // every CTA holds all CTAs' sums; two passes alternate
   __shared__ float cta_max[kSampleCtas];
   __shared__ uint32_t s_bin, bar;
-  __shared__ double s_rest;
+  __shared__ uint64_t s_rest;
   cg::cluster_group cluster = cg::this_cluster();
   cluster_arrive();                                       // as above
   const int rank = static_cast<int>(cluster.block_rank()), ctas = static_cast<int>(cluster.num_blocks());
@@ -327,76 +341,84 @@ sample_topk_topp_kernel(const T* __restrict__ logits, int64_t ld, int V, const f
   for (int i = 1; i < ctas; ++i) m = fmaxf(m, cta_max[i]);
 
   // Largest key whose elements and all above reach `want` (a share of the whole where `share`), among elements with key >= floor_key.
-  // `mass`: weights instead of counts.
+  // Counts, or with Mass weights in units of 2^-40.
   int pass_no = 0;
-  auto select = [&](bool mass, double want, bool share, uint32_t floor_key) -> uint32_t {
+  auto select = [&](auto kind, double want_in, bool share, uint32_t floor_key) -> uint32_t {
+    using Kind = decltype(kind);
+    using Sum = typename Kind::Sum;
+    constexpr int BITS = Kind::BITS, BINS = 1 << BITS, PER_LANE = BINS / 32;
+    Sum* sum = reinterpret_cast<Sum*>(hist);               // [BINS][kSampleThreads]
+    uint64_t want = static_cast<uint64_t>(want_in);
     uint32_t prefix = 0;
     for (int hi = KEY_BITS; hi > 0;) {
-      const int lo = hi > 6 ? hi - 6 : 0;
-      float* col = hist + tid;
+      const int lo = hi > BITS ? hi - BITS : 0;
 #pragma unroll 16
-      for (int b = 0; b < kBins; ++b) col[b * kSampleThreads] = 0.f;          // also the integer 0
+      for (int b = 0; b < BINS; ++b) sum[b * kSampleThreads + tid] = 0;
       each([&](const float (&f)[N], int) {
 #pragma unroll
         for (int j = 0; j < N; ++j) {
           const uint32_t key = key_of(f[j]);
           if (key < floor_key || (hi < KEY_BITS && (key >> hi) != prefix)) continue;
-          float* bin = col + ((key >> lo) & ((1u << (hi - lo)) - 1u)) * kSampleThreads;
-          if (mass) *bin += ex2((f[j] - m) * k2);
-          else *reinterpret_cast<uint32_t*>(bin) += 1u;
+          Sum& bin = sum[((key >> lo) & ((1u << (hi - lo)) - 1u)) * kSampleThreads + tid];
+          if constexpr (Kind::mass) bin += __float2ull_rz(ex2((f[j] - m) * k2) * kMassUnits);
+          else bin += 1;
         }
       });
       __syncthreads();
-      double(&all)[kSampleCtas][kBins] = sums[pass_no++ & 1];
-      for (int b = w; b < kBins; b += kSampleWarps) {
-        double t;
-        if (mass) {
-          float x = 0.f;
+      uint64_t(&all)[kSampleCtas][kBins] = sums[pass_no++ & 1];
+      for (int b = w; b < BINS; b += kSampleWarps) {
+        Sum t = 0;
 #pragma unroll
-          for (int c = 0; c < kSampleWarps; ++c) x += hist[b * kSampleThreads + c * 32 + l];
-          t = warp_sum(x);
+        for (int c = 0; c < kSampleWarps; ++c) t += sum[b * kSampleThreads + c * 32 + l];
+        if constexpr (Kind::mass) {
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
         } else {
-          uint32_t x = 0;
-#pragma unroll
-          for (int c = 0; c < kSampleWarps; ++c) x += reinterpret_cast<const uint32_t*>(hist)[b * kSampleThreads + c * 32 + l];
-          t = __reduce_add_sync(0xffffffffu, x);
+          t = __reduce_add_sync(0xffffffffu, t);
         }
         if (l < ctas) *cluster.map_shared_rank(&all[rank][b], l) = t;
       }
       cluster.sync();
-      if (w == 0) {                                        // lane l: bins 63 - 2 l and 62 - 2 l, from the top down
-        double a = 0., b = 0.;
-        for (int c = 0; c < ctas; ++c) { a += all[c][kBins - 1 - 2 * l]; b += all[c][kBins - 2 - 2 * l]; }
-        double up = a + b;                                 // inclusive sum over the lanes up to this one
+      if (w == 0) {                                        // lane l: the bins from BINS - 1 - PER_LANE l on, from the top down
+        uint64_t of[PER_LANE] = {}, up = 0;
+        for (int c = 0; c < ctas; ++c)
+#pragma unroll
+          for (int i = 0; i < PER_LANE; ++i) of[i] += all[c][BINS - 1 - PER_LANE * l - i];
+#pragma unroll
+        for (int i = 0; i < PER_LANE; ++i) up += of[i];
+        uint64_t mine = up;                                // up: inclusive sum over the lanes up to this one
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-          const double t = __shfl_up_sync(0xffffffffu, up, o);
+          const uint64_t t = __shfl_up_sync(0xffffffffu, up, o);
           if (l >= o) up += t;
         }
-        if (share) want *= __shfl_sync(0xffffffffu, up, 31);
-        double above = __shfl_up_sync(0xffffffffu, up, 1);
-        if (l == 0) above = 0.;
+        if (share) {
+          want = static_cast<uint64_t>(want_in * static_cast<double>(__shfl_sync(0xffffffffu, up, 31)));
+          if (want == 0) want = 1;
+        }
         const uint32_t hit = __ballot_sync(0xffffffffu, up >= want);
         if (hit == 0) {
-          if (l == 0) { s_bin = 0; s_rest = 0.; }          // rounding left the sum short: everything with this prefix
+          if (l == 0) { s_bin = 0; s_rest = 0; }           // no mass at all: everything
         } else if (l == __ffs(hit) - 1) {
-          const bool second = above + a < want;
-          s_bin = static_cast<uint32_t>(kBins - 1 - 2 * l - (second ? 1 : 0));
-          s_rest = want - above - (second ? a : 0.);
+          uint64_t rest = want - (up - mine);
+          int i = 0;
+          for (; i < PER_LANE - 1 && of[i] < rest; ++i) rest -= of[i];
+          s_bin = static_cast<uint32_t>(BINS - 1 - PER_LANE * l - i);
+          s_rest = rest;
         }
       }
       __syncthreads();
       prefix = (prefix << (hi - lo)) | s_bin;
       want = s_rest;
-      if (want <= 0.) return prefix << lo;
+      if (want == 0) return prefix << lo;
       share = false;
       hi = lo;
     }
     return prefix;
   };
 
-  const uint32_t k_key = top_k > 0 && top_k < V ? select(false, static_cast<double>(top_k), false, 0) : 0;
-  const uint32_t p_key = !greedy && top_p < 1.f && top_p > 0.f ? select(true, static_cast<double>(top_p), true, k_key) : 0;
+  const uint32_t k_key = top_k > 0 && top_k < V ? select(CountDigits{}, static_cast<double>(top_k), false, 0) : 0;
+  const uint32_t p_key = !greedy && top_p < 1.f && top_p > 0.f ? select(MassDigits{}, static_cast<double>(top_p), true, k_key) : 0;
   const uint32_t cut = k_key > p_key ? k_key : p_key;
 
   // ---- Gumbel-max over the kept set + its mass
@@ -461,7 +483,7 @@ int launch_rows(K kernel, int B, int ctas, int smem, cudaStream_t s, Args... arg
 template <typename T>
 int launch_topk_topp(const void* logits, int64_t ld, int B, int V, const float* temp, int inverse, const uint64_t* seeds, int greedy_all,
                      int top_k, float top_p, int64_t* out_tok, float* out_lp, cudaStream_t s) {
-  constexpr int smem = kBins * kSampleThreads * static_cast<int>(sizeof(float));
+  constexpr int smem = kHistBytes;
   PRL_CUDA_CHECK(cudaFuncSetAttribute(sample_topk_topp_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   return launch_rows(sample_topk_topp_kernel<T>, B, row_ctas(B, 3), smem, s, static_cast<const T*>(logits), ld, V, temp, inverse, seeds,
                      greedy_all, top_k, top_p, out_tok, out_lp);

@@ -159,3 +159,17 @@ def test_nucleus_of_everything(C, dtype):
     for seed in _seeds_for(1, 0.1):
         tok, _ = C.sample_topk_topp(z, scale, torch.tensor([seed], device="cuda"), False, -1, 1 - 2.0 ** -24, True)
         assert int(tok) == 1
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("small,kept", [(4, False), (5, True)])
+def test_nucleus_mass_is_exact(C, dtype, small, kept):
+    """Weights of powers of two: one of 1, 2048 of 2^-20 and a few of 2^-26 beside the first.  The largest top_p below one leaves out
+    2^-24 (1 + 2^-9 + ...) at most: four of the smallest, not five.  A sum of 24 bits that starts from 1 loses every one of them."""
+    z = torch.full((1, 4096), -math.inf, device="cuda")
+    z[0, 0], z[0, 1:1 + small], z[0, 1024:3072] = 60.0, 34.0, 40.0            # 26 ln 2 = 18.02 apart
+    z, scale, seeds = z.to(dtype), torch.full((1,), math.log(2.0), device="cuda"), _seeds_for(1, -1.7)
+    assert len(seeds) == 8
+    for seed in seeds:
+        tok, _ = C.sample_topk_topp(z, scale, torch.tensor([seed], device="cuda"), False, -1, 1 - 2.0 ** -24, True)
+        assert (int(tok) == 1) == kept
