@@ -647,10 +647,13 @@ def sample_tokens(logits: torch.Tensor, temperature: torch.Tensor | float = 1.0,
         if seeds is None:
             seeds = torch.randint(0, 2 ** 62, (b,), device=logits.device, dtype=torch.int64)
         seeds = seeds.contiguous()
-        # temperatures as the engine holds them go to the kernel, which inverts them; any other form becomes inverse temperatures here
+        # temperatures as the engine holds them go to the kernel, which inverts them; any other form becomes inverse temperatures here: one
+        # for all rows, or an element a row in memory order, whatever the shape
         inverse = temperature.dtype != torch.float32 or temperature.shape != (b,) or not temperature.is_contiguous()
-        scales = torch.where(temperature > 0, 1.0 / temperature.clamp_min(1e-6), torch.zeros_like(temperature)).float().expand(b).contiguous() \
-            if inverse else temperature
+        scales = temperature
+        if inverse:
+            scales = torch.where(temperature > 0, 1.0 / temperature.clamp_min(1e-6), torch.zeros_like(temperature)).float().reshape(-1)
+            scales = (scales.expand(b) if scales.numel() == 1 else scales[:b]).contiguous()
         if simple:
             return tuple(_C().sample(logits, scales, seeds, bool(greedy), inverse))
         # top-k / top-p: radix-select kernel (no sort); log-prob under the renormalised kept set

@@ -173,3 +173,23 @@ def test_nucleus_mass_is_exact(C, dtype, small, kept):
     for seed in seeds:
         tok, _ = C.sample_topk_topp(z, scale, torch.tensor([seed], device="cuda"), False, -1, 1 - 2.0 ** -24, True)
         assert (int(tok) == 1) == kept
+
+
+@pytest.mark.parametrize("top_k,top_p", [(-1, 1.0), (20, 0.9)])
+def test_forms_of_temperatures(C, top_k, top_p):
+    """Temperatures of any shape with an element a row, or one for all, give what a plain vector gives."""
+    from polyrl_b200 import ops
+
+    b, v = 6, 5000
+    torch.manual_seed(0)
+    z, seeds = torch.randn(b, v, device="cuda").mul_(3).bfloat16(), torch.randint(0, 2 ** 62, (b,), device="cuda")
+    t = torch.tensor([0.7, 1.0, 0.0, 1.3, 0.5, 2.0], device="cuda")
+    sample = lambda temp: ops.sample_tokens(z, temp, seeds, top_k=top_k, top_p=top_p)      # noqa: E731
+    want = sample(t)
+    for form in (t[:, None], t[None], t.double(), t.repeat(2), torch.stack([t, t], 1)[:, 0], t.view(2, 3)):
+        assert all(torch.equal(a, c) for a, c in zip(sample(form), want))
+    want = sample(torch.full((b,), 0.7, device="cuda"))
+    for form in (0.7, torch.tensor(0.7, device="cuda"), torch.tensor([[0.7]], device="cuda")):
+        assert all(torch.equal(a, c) for a, c in zip(sample(form), want))
+    with pytest.raises(RuntimeError):
+        sample(t[:4])
