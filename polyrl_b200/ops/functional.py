@@ -432,7 +432,8 @@ def head_norm_rope_and_cache_(qkv, pos, cos, sin, nq, nkv, d, q_norm, k_norm, ep
 
 
 def gather_cached(k_cache: torch.Tensor, v_cache: torch.Tensor, blk: torch.Tensor, off: torch.Tensor):
-    """Keys and values [T, nkv, d] at the places (page ``blk[t]``, row ``off[t]``) of caches [pages, nkv, page, d]."""
+    """Keys and values [T, nkv, d] at the places (page ``blk[t]``, row ``off[t]``) of caches [pages, nkv, page, d].  A place outside the
+    cache is an error: IndexError on the CPU, a failed assertion of the kernel on the GPU, as with indexing."""
     if all(_is_kernel_tensor(c) and c.dim() == 4 and c.is_contiguous() and c.shape[3] % 8 == 0 and c.data_ptr() % 16 == 0 for c in (k_cache, v_cache)) \
             and k_cache.shape == v_cache.shape and blk.shape == off.shape \
             and all(i.device == k_cache.device == v_cache.device and i.dtype == torch.int64 and i.dim() == 1 and i.is_contiguous() for i in (blk, off)) \
