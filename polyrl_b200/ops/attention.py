@@ -76,6 +76,7 @@ class _RopeAttnFn(torch.autograd.Function):
             C.qk_norm_rope_(qkv, pos, cos, sin, nq, nkv, d, q_norm, k_norm, eps, rot)
         else:
             C.rope_(qkv, pos, cos, sin, nq, nkv, d, 1.0, None, None, None, 16)
+            torch.autograd.graph.increment_version(qkv)          # (mark_dirty would make the rotated rows an output)
             rot = None
         q, k, v = _heads(qkv if rot is None else rot, qkv, nq, nkv, d)
         o, lse = C.attn_fwd(q, k, v, cu, cu, scale, True, True)
@@ -112,8 +113,9 @@ def rope_attention(qkv: torch.Tensor, pos: torch.Tensor, cos: torch.Tensor, sin:
                    cu_seqlens: torch.Tensor, q_norm: torch.Tensor | None = None, k_norm: torch.Tensor | None = None,
                    eps: float = 1e-6) -> torch.Tensor | None:
     """Causal attention [T, nq, d] over packed rows ``qkv`` [T, (nq + 2 nkv) * d] of a projection, its query and key heads normed (if
-    gains are given) and rotated first.  ``qkv`` is consumed: its contents afterwards are undefined.  None: these operands need the
-    general path (``apply_rope`` and ``attention_varlen``)."""
+    gains are given) and rotated first.  ``qkv`` is consumed: its contents afterwards are undefined, and autograd knows that they changed,
+    so a node that saved them refuses its backward.  None: these operands need the general path (``apply_rope`` and
+    ``attention_varlen``), as do a leaf and a view, whose change in place autograd has to see."""
     from .functional import head_norm_ok
 
     if not (qkv.dim() == 2 and qkv.is_contiguous() and qkv.shape[1] == (nq + 2 * nkv) * d and qkv.data_ptr() % 16 == 0 and cu_seqlens.is_cuda
@@ -122,6 +124,8 @@ def rope_attention(qkv: torch.Tensor, pos: torch.Tensor, cos: torch.Tensor, sin:
         return None
     q, k, v = _heads(qkv.detach(), qkv.detach(), nq, nkv, d)
     if not _own_ok(q, k, v) or (q_norm is not None and not head_norm_ok(qkv, cos, sin, d, q_norm, k_norm)):
+        return None
+    if q_norm is None and torch.is_grad_enabled() and qkv.requires_grad and (qkv.is_leaf or qkv._is_view()):
         return None
     cu, scale = cu_seqlens.to(torch.int32).contiguous(), d ** -0.5
     if torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (qkv, q_norm, k_norm)):
@@ -132,6 +136,8 @@ def rope_attention(qkv: torch.Tensor, pos: torch.Tensor, cos: torch.Tensor, sin:
         ext().qk_norm_rope_(qkv, pos, cos, sin, nq, nkv, d, q_norm, k_norm, eps)
     else:
         ext().rope_(qkv, pos, cos, sin, nq, nkv, d, 1.0, None, None, None, 16)
+    if torch.is_grad_enabled():
+        torch.autograd.graph.increment_version(qkv)
     return ext().attn_fwd(q, k, v, cu, cu, scale, True, False)[0]
 
 

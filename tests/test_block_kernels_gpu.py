@@ -124,6 +124,31 @@ def test_rope_attention(d, nq, nkv, lens, norm):
     assert rope_attention(qkv[:, : (nq + 2 * nkv) * d - 8], pos, cos, sin, nq, nkv, d, cu) is None        # not the rows it is made for
 
 
+def test_rope_attention_changes_its_rows_in_the_open():
+    """Without gains the rows are rotated in place: not a leaf's or a view's, and a node that saved them refuses its backward."""
+    from polyrl_b200.ops.attention import rope_attention
+
+    nq, nkv, d, t = 4, 2, 64, 70
+    cos, sin = (f.cuda() for f in OF.ref.rope_tables(128, d, 1e4))
+    pos, cu = torch.arange(t).cuda(), torch.tensor([0, t], dtype=torch.int32).cuda()
+    leaf = _randn(t, (nq + 2 * nkv) * d, seed=1).requires_grad_(True)
+    before = leaf.detach().clone()
+    call = lambda x: rope_attention(x, pos, cos, sin, nq, nkv, d, cu)          # noqa: E731
+    assert call(leaf) is None and call(leaf.view(t, -1)) is None and call((leaf * 1.0).view(t, -1)) is None
+    assert torch.equal(leaf, before)
+    rows = leaf * 1.0
+    saved = rows.sin()
+    out = call(rows)
+    assert out is not None and torch.isfinite(torch.autograd.grad(out.sum(), leaf, retain_graph=True)[0]).all()
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        torch.autograd.grad(saved.sum(), leaf)
+    plain, w = before.clone(), _randn(1, seed=2).requires_grad_(True)
+    saved = plain * w
+    assert call(plain) is not None
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        torch.autograd.grad(saved.sum(), w)
+
+
 @pytest.mark.parametrize("t,v,h", [(1, 264, 64), (128, 392, 64), (129, 392, 128), (300, 640, 64), (515, 5000, 896)])
 @pytest.mark.parametrize("tau", [1.0, 0.7])
 def test_linear_ce_edges(t, v, h, tau):
