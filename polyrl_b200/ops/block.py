@@ -42,26 +42,35 @@ class _DenseBlockFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, rstd1, h1, qkv, rot, o, lse, x1, rstd2, h2, gu, a, pos, cos, sin, cu, ln1, wqkv, bqkv, q_norm, k_norm, wo, ln2, wgu, wd = ctx.saved_tensors
+        # the names above are the last references, unless the graph is kept: activations are given up as soon as they are used, as the nodes
+        # of a chain would (at 16 K tokens of an 8B block gu, a and h2 are 1.5 GB)
+        ctx.maybe_clear_saved_tensors()
         nq, nkv, d, eps = ctx.dims
         C, t = _C(), x.shape[0]
         dy = _g2_operand(dy.contiguous())
         da, dwd = C.gemm2_grads(dy, wd, a, _sink_for(wd))
+        del a
         dgu = C.swiglu_bwd(gu, da)
-        del da
+        del gu, da
         dh2, dwgu = C.gemm2_grads(dgu, wgu, h2, _sink_for(wgu))
-        del dgu
+        del dgu, h2
         dx1, dln2 = C.rmsnorm_bwd(x1, ln2, dh2, rstd2, dy, True)
+        del x1, dh2, dy
         do, dwo = C.gemm2_grads(dx1, wo, o.view(t, nq * d), _sink_for(wo))
         g = torch.empty(qkv.shape, device=x.device, dtype=x.dtype)
         C.attn_bwd(*_heads(qkv if rot is None else rot, qkv, nq, nkv, d), o, do.view(t, nq, d), lse, cu, cu, d ** -0.5, True, g)
+        del o, do, lse
         dqn = dkn = None
         if rot is not None:
             dqn, dkn = C.qk_norm_rope_bwd_(g, qkv, pos, cos, sin, nq, nkv, d, q_norm, k_norm, eps)
         else:
             C.rope_(g, pos, cos, sin, nq, nkv, d, -1.0, None, None, None, 16)
+        del qkv, rot
         dh1, dwqkv = C.gemm2_grads(g, wqkv, h1, _sink_for(wqkv))
+        dbqkv = None if bqkv is None else g.sum(0)
+        del g, h1
         dx, dln1 = C.rmsnorm_bwd(x, ln1, dh1, rstd1, dx1, True)
-        return (dx, None, None, None, None, None, dln1, dwqkv, None if bqkv is None else g.sum(0), dqn, dkn, dwo, dln2, dwgu, dwd)
+        return (dx, None, None, None, None, None, dln1, dwqkv, dbqkv, dqn, dkn, dwo, dln2, dwgu, dwd)
 
 
 def _plain(w: torch.Tensor) -> bool:

@@ -303,6 +303,36 @@ def test_dense_block_is_the_chain(model, lens, monkeypatch):
     assert not type(tf.layer_forward(cfg, w, x, inp).grad_fn).__name__.startswith("_DenseBlockFn")
 
 
+@pytest.mark.parametrize("model", ["qwen3-1.7b", "llama3-8b"])
+def test_dense_block_gives_up_its_activations(model, monkeypatch):
+    """Memory at the peak of the backward pass is no more than with the chain of functions, whose nodes free theirs one by one; a graph that is
+    kept can be gone through again."""
+    from polyrl_b200.models import get_model_config
+    from polyrl_b200.models import transformer as tf
+
+    cfg, t = get_model_config(model), 4096
+    w = {n: _randn(*s, seed=i, scale=0.02, shift=1.0 if len(s) == 1 else 0.0).requires_grad_(True) for i, (n, s) in enumerate(tf.layer_param_specs(cfg, 0))}
+    x, gy = _randn(t, cfg.hidden_size, seed=50).requires_grad_(True), _randn(t, cfg.hidden_size, seed=51)
+    cu = torch.tensor([0, t // 2, t], dtype=torch.int32).cuda()
+    inp = tf.PackedInput(torch.zeros(t, dtype=torch.long, device="cuda"), torch.cat([torch.arange(t // 2)] * 2).cuda(), cu, t // 2)
+
+    def peak():
+        y = tf.layer_forward(cfg, w, x, inp)
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        torch.autograd.grad(y, [x, *w.values()], gy)
+        return torch.cuda.max_memory_allocated()
+
+    block = [peak(), peak()][1]
+    y = tf.layer_forward(cfg, w, x, inp)
+    first, again = (torch.autograd.grad(y, [x, *w.values()], gy, retain_graph=k) for k in (True, False))
+    assert all(torch.equal(a, b) for a, b in zip(first, again))
+    del first, again, y
+    monkeypatch.setattr(tf, "dense_block", lambda *a: None)
+    chain = [peak(), peak()][1]
+    assert block <= chain + (1 << 20), (block, chain)
+
+
 def test_decode_kernels_behind_each_other():
     """Kernels of a decode step may start while the one before still runs: a chain in which each reads what the last one wrote, its buffers
     freed and taken again on the way, gives the same values as with a wait after every kernel."""
