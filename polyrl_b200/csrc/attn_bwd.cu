@@ -542,15 +542,17 @@ attn_bwd_queries_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
 }
 
 // stats[h, t] = (lse in base 2, D = sum_d dO[t, h, d] * O[t, h, d]).  A warp takes 32 tokens of one head, D / 8 threads a row, with 16-byte
-// loads; what it writes is 256 contiguous bytes.
+// loads; what it writes is 256 contiguous bytes.  Rows that belong to no sequence get a zero gradient here.
 template <int D>
 __global__ void __launch_bounds__(256)
 attn_stats_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o, int64_t ldo, int64_t lddo,
-                  const float* __restrict__ lse, float2* __restrict__ stats, int Tq, int nq) {
+                  const float* __restrict__ lse, float2* __restrict__ stats, __nv_bfloat16* __restrict__ dq, int64_t lddq,
+                  const int32_t* __restrict__ cu_q, int B, int Tq, int nq) {
   constexpr int L = D / 8, R = 32 / L;
   const int lane = threadIdx.x & 31, l = lane % L, w = blockIdx.x * 8 + (threadIdx.x >> 5);
   const int h = w % nq, t0 = w / nq * 32;
   if (t0 >= Tq) return;
+  const int begin = cu_q[0], end = cu_q[B];
   float mine = 0.f;
 #pragma unroll 8
   for (int k = 0; k < 32 / R; ++k) {
@@ -566,6 +568,7 @@ attn_stats_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
         const float2 x = unpack_bf16(au[i]), y = unpack_bf16(bu[i]);
         s += x.x * y.x + x.y * y.y;
       }
+      if (t < begin || t >= end) st_v4(dq + static_cast<int64_t>(t) * lddq + h * D + l * 8, make_int4(0, 0, 0, 0));
     }
 #pragma unroll
     for (int f = L / 2; f > 0; f >>= 1) s += __shfl_xor_sync(0xffffffffu, s, f);
@@ -610,14 +613,19 @@ extern "C" int prl_attn_bwd(const void* q, const void* k, const void* v, const v
                             float* stats, void* dq, void* dk, void* dv, const int32_t* cu_q, const int32_t* cu_k, int B,
                             int Tq, int Tk, int nq, int nkv, int d, int64_t ldq, int64_t ldk, int64_t ldv, int64_t ldo, int64_t lddo,
                             int64_t lddq, int64_t lddkv, float sm_scale, int causal, int q_tiles, int k_tiles, cudaStream_t stream) {
-  if (Tq <= 0 || Tk <= 0 || B <= 0) return 0;
+  if (Tq <= 0) return 0;
   if (nq % nkv != 0 || (d != 64 && d != 128)) return -120;
+  if (Tk <= 0 || B <= 0) {                                 // no key is seen
+    PRL_CUDA_CHECK(cudaMemset2DAsync(dq, lddq * 2, 0, static_cast<size_t>(nq) * d * 2, Tq, stream));
+    return 0;
+  }
   const int64_t blocks = (static_cast<int64_t>((Tq + 31) / 32) * nq + 7) / 8;
   const auto* op = static_cast<const __nv_bfloat16*>(o);
   const auto* gp = static_cast<const __nv_bfloat16*>(d_o);
   auto* st = reinterpret_cast<float2*>(stats);
-  if (d == 64) attn_stats_kernel<64><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(op, gp, ldo, lddo, lse, st, Tq, nq);
-  else attn_stats_kernel<128><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(op, gp, ldo, lddo, lse, st, Tq, nq);
+  auto* dqp = static_cast<__nv_bfloat16*>(dq);
+  if (d == 64) attn_stats_kernel<64><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(op, gp, ldo, lddo, lse, st, dqp, lddq, cu_q, B, Tq, nq);
+  else attn_stats_kernel<128><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(op, gp, ldo, lddo, lse, st, dqp, lddq, cu_q, B, Tq, nq);
   PRL_CUDA_CHECK(cudaGetLastError());
   CUtensorMap tmQ, tmK, tmV, tmdO;
   if (af_tmap(&tmQ, q, Tq, static_cast<uint64_t>(nq) * d, ldq * 2, 128)) return -121;

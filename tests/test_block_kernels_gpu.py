@@ -259,6 +259,27 @@ def test_attention_backward_tiles(d, lq, lk, causal):
         assert (a.double() - b).norm() <= 2e-2 * b.norm() + 1e-3
 
 
+@pytest.mark.parametrize("d", [64, 128])
+def test_attention_backward_outside_sequences(d):
+    """Query rows that belong to no sequence, and queries without any key, have a zero gradient whatever lay in the memory before."""
+    from polyrl_b200.ops import ext
+
+    nq, nkv, t = 4, 2, 300
+    q, k, v, go = (_randn(t, h, d, seed=i) for i, h in enumerate((nq, nkv, nkv, nq)))
+    cu = torch.tensor([5, 150, 263], dtype=torch.int32).cuda()
+    o, lse = ext().attn_fwd(q, k, v, cu, cu, d ** -0.5, True, True)
+    for out in (None, torch.full((t, (nq + 2 * nkv) * d), float("nan"), device="cuda", dtype=torch.bfloat16)):
+        junk = torch.full((t, nq, d), float("nan"), device="cuda", dtype=torch.bfloat16)
+        del junk                                             # (its block is the one that the gradient takes)
+        dq = ext().attn_bwd(q, k, v, o.nan_to_num(), go, lse, cu, cu, d ** -0.5, True, out)[0]
+        assert not dq[:5].any() and not dq[263:].any() and torch.isfinite(dq).all() and dq[5:263].any()
+    junk = torch.full((t, nq, d), float("nan"), device="cuda", dtype=torch.bfloat16)
+    del junk
+    none = torch.zeros(3, dtype=torch.int32, device="cuda")
+    dq, dk, dv = ext().attn_bwd(q, k[:0], v[:0], o.nan_to_num(), go, lse, cu, none, d ** -0.5, True)
+    assert not dq.any() and torch.isfinite(dq).all() and dk.shape == dv.shape == (0, nkv, d)
+
+
 @pytest.mark.parametrize("t,n,k", [(8, 136, 136), (387, 1152, 896), (300, 4096, 520), (2503, 2048, 896), (520, 200, 2056), (1030, 6144, 1000)])
 def test_gemm2_grads(t, n, k):
     """Input and weight gradient of a linear layer in one launch: bf16 and accumulating fp32 input gradient, results of the separate
