@@ -52,13 +52,14 @@ __device__ __forceinline__ void mma_scores(uint32_t acc, const uint8_t* a, const
   for (int kk = 0; kk < D / 16; ++kk)
     umma_bf16_ss(acc, umma_desc_sw128_kmajor(a + (kk >> 2) * 16384) + 2 * (kk & 3), umma_desc_sw128_kmajor(b + (kk >> 2) * 16384) + 2 * (kk & 3), id, kk != 0);
 }
-// acc (+)= A B with A [128, 128] as bf16 in TMEM (columns 64 g .. 64 g + 31 hold columns 64 g .. 64 g + 63), B [128, D] read MN-major
+// acc (+)= A B over the `left` rows of B, with A [128, 128] as bf16 in TMEM (columns 64 g .. 64 g + 31 hold columns 64 g .. 64 g + 63),
+// B [128, D] read MN-major
 template <int D>
-__device__ __forceinline__ void mma_from_tmem(uint32_t acc, uint32_t a, const uint8_t* b, bool add) {
+__device__ __forceinline__ void mma_from_tmem(uint32_t acc, uint32_t a, const uint8_t* b, bool add, int left) {
   constexpr uint32_t id = umma_idesc_major(128, D, 1, 1, 0, 1);
-#pragma unroll
-  for (int kk = 0; kk < 8; ++kk)
+  for_row_steps(left, [&](int kk) {
     umma_bf16_ts(acc, a + (kk >> 2) * 64 + 8 * (kk & 3), umma_desc_sw128_mnmajor(b, 16384) + kk * 128, id, add || kk != 0);
+  });
 }
 // 32 fp32 columns of a warp's 32 TMEM rows -> bf16 rows in memory, through 2 KB of shared memory; row `lane` of the warp is valid if
 // lane < rows.  any = false: zeros.
@@ -195,44 +196,66 @@ attn_bwd_keys_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     constexpr uint32_t idKM = umma_idesc_major(128, D, 1, 1, 0, 1);               // A K-major, B MN-major
     for (int w = blockIdx.x; item(w, t); w += gridDim.x) {
       if (t.iters == 0) continue;
-      if (lane == 0) {
-        auto scores = [&](int m) {                        // S^T of pair m: P^T of the one before is consumed
-          mbar_wait(&q_full[m & 1], (m >> 1) & 1);
-          if (m > 0) mbar_wait(&dv_done[(m - 1) & 1], ((m - 1) >> 1) & 1);
-          tc_fence_after();
+      // All lanes wait, for they clear rows, and meet before lane 0 issues anything: a lane that were still asking for a phase when the next
+      // one is over would wait for good.
+      // rows of the item's it-th query tile that are its sequence's
+      auto left = [&](int it) { return min(t.lq - (t.i0 + it % t.n_i) * 128, 128); };
+      auto scores = [&](int m, int it) {                  // S^T of pair m: P^T of the one before is consumed
+        mbar_wait(&q_full[m & 1], (m >> 1) & 1);
+        if (left(it) & 15) clear_rows<D>(sQ + (m & 1) * T, left(it));
+        if (m > 0) mbar_wait(&dv_done[(m - 1) & 1], ((m - 1) >> 1) & 1);
+        tc_fence_after();
+        __syncwarp();
+        if (lane == 0) {
           mma_scores<D>(tS, sK, sQ + (m & 1) * T);
           umma_commit(s_full);
-        };
-        auto products = [&](int m) {                      // dP^T of pair m: that of the one before has been read (ds_full)
-          mbar_wait(&do_full[m & 1], (m >> 1) & 1);
-          tc_fence_after();
+        }
+      };
+      auto operand = [&](int m, int it) {                 // dO of pair m
+        mbar_wait(&do_full[m & 1], (m >> 1) & 1);
+        if (left(it) & 15) clear_rows<D>(sdO + (m & 1) * T, left(it));
+      };
+      auto products = [&](int m) {                        // dP^T of pair m: that of the one before has been read (ds_full)
+        tc_fence_after();
+        __syncwarp();
+        if (lane == 0) {
           mma_scores<D>(tdP, sV, sdO + (m & 1) * T);
           umma_commit(dp_full);
-        };
-        mbar_wait(k_full, i & 1);
-        scores(n);
-        mbar_wait(v_full, i & 1);
-        products(n);
-        for (int it = 0; it < t.iters; ++it, ++n) {
-          const int s = n & 1;
-          mbar_wait(p_full, n & 1);
-          if (it == 0 && i > 0) mbar_wait(acc_free, (i - 1) & 1);
-          tc_fence_after();
-          mma_from_tmem<D>(tdV, tS, sdO + s * T, it != 0);                        // dV += P^T dO
+        }
+      };
+      mbar_wait(k_full, i & 1);
+      scores(n, 0);
+      operand(n, 0);
+      mbar_wait(v_full, i & 1);
+      products(n);
+      for (int it = 0; it < t.iters; ++it, ++n) {
+        const int s = n & 1;
+        mbar_wait(p_full, n & 1);
+        if (it == 0 && i > 0) mbar_wait(acc_free, (i - 1) & 1);
+        tc_fence_after();
+        __syncwarp();
+        if (lane == 0) {
+          mma_from_tmem<D>(tdV, tS, sdO + s * T, it != 0, left(it));   // dV += P^T dO
           umma_commit(&dv_done[s]);
-          if (it + 1 < t.iters) scores(n + 1);
-          mbar_wait(ds_full, n & 1);
-          tc_fence_after();
-          if (it + 1 < t.iters) products(n + 1);
-#pragma unroll
-          for (int kk = 0; kk < 8; ++kk)                                          // dK += dS^T Q  (reduction over the 128 query rows)
+        }
+        if (it + 1 < t.iters) {
+          scores(n + 1, it + 1);
+          operand(n + 1, it + 1);
+        }
+        mbar_wait(ds_full, n & 1);
+        tc_fence_after();
+        if (it + 1 < t.iters) products(n + 1);
+        __syncwarp();
+        if (lane == 0) {
+          for_row_steps(left(it), [&](int kk) {                                   // dK += dS^T Q  (reduction over the query rows)
             umma_bf16_ss(tdK, umma_desc_sw128_kmajor(sdS + (kk >> 2) * 16384) + 2 * (kk & 3), umma_desc_sw128_mnmajor(sQ + s * T, 16384) + kk * 128, idKM,
                          (it | kk) != 0);
+          });
           umma_commit(&dk_done[s]);
         }
+        __syncwarp();
       }
       ++i;
-      __syncwarp();
     }
   } else {
     const int g = (warp - 2) >> 2;
@@ -437,41 +460,57 @@ attn_bwd_queries_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   } else if (warp == 1) {
     for (int w = blockIdx.x; item(w, t); w += gridDim.x) {
       if (t.nt == 0) continue;
-      if (lane == 0) {
-        auto scores = [&](int m) {                        // S of tile m, over dS of tile m - 2
-          const int s = m & 1;
-          mbar_wait(&k_full[s], (m >> 1) & 1);
-          if (m >= 2) mbar_wait(&dq_done[s], ((m - 2) >> 1) & 1);
-          tc_fence_after();
+      auto left = [&](int j) { return min(t.lk - j * 128, 128); };                // keys of tile j that are the sequence's
+      auto scores = [&](int m, int j) {                   // S of tile m, over dS of tile m - 2
+        const int s = m & 1;
+        mbar_wait(&k_full[s], (m >> 1) & 1);
+        if (left(j) & 15) clear_rows<D>(sK + s * T, left(j));
+        if (m >= 2) mbar_wait(&dq_done[s], ((m - 2) >> 1) & 1);
+        tc_fence_after();
+        __syncwarp();
+        if (lane == 0) {
           mma_scores<D>(tS + s * 128, sQ, sK + s * T);
           umma_commit(&s_full[s]);
-        };
-        auto products = [&](int m) {                      // dP of tile m: that of the one before has been read (ds_full)
-          const int s = m & 1;
-          mbar_wait(&v_full[s], (m >> 1) & 1);
-          tc_fence_after();
+        }
+      };
+      auto operand = [&](int m, int j) {                  // V of tile m
+        mbar_wait(&v_full[m & 1], (m >> 1) & 1);
+        if (left(j) & 15) clear_rows<D>(sV + (m & 1) * T, left(j));
+      };
+      auto products = [&](int m) {                        // dP of tile m: that of the one before has been read (ds_full)
+        const int s = m & 1;
+        tc_fence_after();
+        __syncwarp();
+        if (lane == 0) {
           mma_scores<D>(tdP, sdO, sV + s * T);
           umma_commit(dp_full);
           umma_commit(&v_done[s]);
-        };
-        mbar_wait(q_full, i & 1);
-        scores(n);
-        mbar_wait(do_full, i & 1);
-        products(n);
-        for (int j = 0; j < t.nt; ++j, ++n) {
-          const int s = n & 1;
-          if (j + 1 < t.nt) scores(n + 1);
-          mbar_wait(ds_full, n & 1);
-          tc_fence_after();
-          if (j + 1 < t.nt) products(n + 1);
-          if (j == 0 && i > 0) mbar_wait(acc_free, (i - 1) & 1);
-          tc_fence_after();
-          mma_from_tmem<D>(tdQ, tS + s * 128, sK + s * T, j != 0);                // dQ += dS K
+        }
+      };
+      mbar_wait(q_full, i & 1);
+      scores(n, 0);
+      operand(n, 0);
+      mbar_wait(do_full, i & 1);
+      products(n);
+      for (int j = 0; j < t.nt; ++j, ++n) {
+        const int s = n & 1;
+        if (j + 1 < t.nt) {
+          scores(n + 1, j + 1);
+          operand(n + 1, j + 1);
+        }
+        mbar_wait(ds_full, n & 1);
+        tc_fence_after();
+        if (j + 1 < t.nt) products(n + 1);
+        if (j == 0 && i > 0) mbar_wait(acc_free, (i - 1) & 1);
+        tc_fence_after();
+        __syncwarp();
+        if (lane == 0) {
+          mma_from_tmem<D>(tdQ, tS + s * 128, sK + s * T, j != 0, left(j));      // dQ += dS K
           umma_commit(&dq_done[s]);
         }
+        __syncwarp();
       }
       ++i;
-      __syncwarp();
     }
   } else {
     const int g = (warp - 2) >> 2;

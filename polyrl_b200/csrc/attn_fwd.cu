@@ -502,13 +502,16 @@ attn_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   } else if (warp == 1) {
     constexpr uint32_t idS = umma_idesc(128, 128, 1, 1);
     constexpr uint32_t idO = umma_idesc_major(128, DV, 1, 1, 0, 1);         // B = V consumed MN-major
+    // all lanes wait, for they clear rows, and meet before lane 0 issues anything: a lane that were still asking for a phase when the next one
+    // is over would wait for good
     for (int w = blockIdx.x; item(w, it); w += gridDim.x, ++i) {
-      if (lane == 0) {
-        mbar_wait(q_full, i & 1);
-        for (int j = 0; j < it.nt; ++j, ++n) {
-          mbar_wait(k_full, n & 1);
-          if (n > 0) mbar_wait(pv_done, (n - 1) & 1);
-          tc_fence_after();
+      mbar_wait(q_full, i & 1);
+      for (int j = 0; j < it.nt; ++j, ++n) {
+        mbar_wait(k_full, n & 1);
+        if (n > 0) mbar_wait(pv_done, (n - 1) & 1);
+        tc_fence_after();
+        __syncwarp();
+        if (lane == 0) {
 #pragma unroll
           for (int kk = 0; kk < DK / 16; ++kk) {
             const uint64_t da = umma_desc_sw128_kmajor(sQ + (kk >> 2) * 16384) + 2 * (kk & 3);
@@ -516,17 +519,22 @@ attn_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             umma_bf16_ss(tS, da, db, idS, kk != 0);
           }
           umma_commit(s_full);
-          mbar_wait(v_full, n & 1);
-          mbar_wait(p_full, n & 1);
-          if (j == 0 && i > 0) mbar_wait(o_free, (i - 1) & 1);
-          tc_fence_after();
-#pragma unroll
-          for (int kk = 0; kk < 8; ++kk)               // 16 keys: 8 columns of P
+        }
+        mbar_wait(v_full, n & 1);
+        const int left = min(it.lk - it.tile_of(j) * kAfBN, kAfBN);
+        if (left < 16 * row_steps(left)) clear_rows<DV>(sV, left);  // (while the softmax works)
+        mbar_wait(p_full, n & 1);
+        if (j == 0 && i > 0) mbar_wait(o_free, (i - 1) & 1);
+        tc_fence_after();
+        __syncwarp();
+        if (lane == 0) {
+          for_row_steps(left, [&](int kk) {               // 16 keys: 8 columns of P
             umma_bf16_ts(tO, tS + 8 * kk, umma_desc_sw128_mnmajor(sV, 16384) + kk * 128, idO, (j | kk) != 0);
+          });
           umma_commit(pv_done);
         }
+        __syncwarp();
       }
-      __syncwarp();
     }
   } else {
     const int quad = warp & 3;

@@ -401,6 +401,33 @@ __device__ __forceinline__ float2 unpack_bf16(uint32_t u) {
   return __bfloat1622float2(h);
 }
 
+// The last tile of a packed sequence holds rows of the next one, or of no sequence at all.  A product that sums over a tile's rows takes the
+// steps of 16 that hold the sequence's `left` rows, one at least ...
+__device__ __forceinline__ int row_steps(int left) { return left >= 128 ? 8 : (max(left, 1) + 15) >> 4; }
+// (in a loop of its own: with a condition around each of eight unrolled steps only the first one took effect)
+template <class F>
+__device__ __forceinline__ void for_row_steps(int left, F&& f) {
+  if (left >= 128) {
+#pragma unroll
+    for (int kk = 0; kk < 8; ++kk) f(kk);
+  } else {
+#pragma unroll 1
+    for (int kk = 0; kk < row_steps(left); ++kk) f(kk);
+  }
+}
+// ... and the rest of the last step is zeros: its weight is 0, but 0 times an infinity or NaN is not.  D bf16 columns in shared memory
+// (chunks of 64 columns, 128 bytes a row); by one whole warp that has waited for the tile's load.
+template <int D>
+__device__ __forceinline__ void clear_rows(uint8_t* tile, int left) {
+  const int lane = threadIdx.x & 31;
+  for (int r = max(left, 0) + (lane >> 3); r < 16 * row_steps(left); r += 4)
+#pragma unroll
+    for (int c = 0; c < D / 64; ++c)
+      asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(smem_u32(tile + c * 16384 + r * 128 + (lane & 7) * 16)), "r"(0) : "memory");
+  fence_proxy_async();
+  __syncwarp();
+}
+
 // Which 128-row tile of a packed batch is number `t`?  Tiles are counted sequence by sequence.  Called by one whole warp, which looks at
 // 32 sequences at a time.  Returns the sequence (-1: fewer tiles than t + 1) and the tile's first row.
 __device__ __forceinline__ int find_row_tile(const int32_t* __restrict__ cu, int B, int t, int* row0) {

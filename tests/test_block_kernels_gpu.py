@@ -280,6 +280,32 @@ def test_attention_backward_outside_sequences(d):
     assert not dq.any() and torch.isfinite(dq).all() and dk.shape == dv.shape == (0, nkv, d)
 
 
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("lq,lk,causal", [([100, 77, 300], [100, 77, 300], True), ([1, 1, 1], [1, 1, 1], True), ([50, 3, 129], [400, 130, 257], True), ([64, 200, 65], [33, 129, 127], False),
+                                          ([40, 9, 144], [144, 300, 40], True)])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_attention_keeps_sequences_apart(d, lq, lk, causal, bad):
+    """Values that are not finite, in the second of three packed sequences, leave outputs and gradients of the others as they are, bit for bit."""
+    from polyrl_b200.ops import ext
+
+    q, k, v, cu_q, cu_k = _packed(d, lq, lk, 0.0)
+    go = _randn(*q.shape, seed=4)
+
+    def run():
+        o, lse = ext().attn_fwd(q, k, v, cu_q, cu_k, d ** -0.5, causal, True)
+        grads = ext().attn_bwd(q, k, v, o, go, lse, cu_q, cu_k, d ** -0.5, causal)
+        n = len(lq)
+        split = [x.split(lq if x.shape[0] == sum(lq) else lk) for x in (o, *grads)] + [lse.split(lq, 1)]
+        return [[p[i].clone() for p in split] for i in range(n)]
+
+    want = run()
+    for x, lens in ((q, lq), (k, lk), (v, lk), (go, lq)):
+        x.split(lens)[1].fill_(bad)
+    got = run()
+    for i in (0, 2):
+        assert all(torch.equal(a, b) and not torch.isnan(a).any() for a, b in zip(got[i], want[i])), i
+
+
 @pytest.mark.parametrize("t,n,k", [(8, 136, 136), (387, 1152, 896), (300, 4096, 520), (2503, 2048, 896), (520, 200, 2056), (1030, 6144, 1000)])
 def test_gemm2_grads(t, n, k):
     """Input and weight gradient of a linear layer in one launch: bf16 and accumulating fp32 input gradient, results of the separate
