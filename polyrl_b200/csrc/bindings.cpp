@@ -684,6 +684,9 @@ void nvls_bcast_store(const at::Tensor& src, int64_t mc_dst, int64_t ctas) {
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm2_grads", &gemm2_grads, py::arg("dy"), py::arg("w"), py::arg("x"), py::arg("dw") = py::none(), py::arg("dx32") = py::none(),
         py::arg("beta") = 0.0);
+  // the plans behind the products: one launch for both gradients? last round of [M, K] x [N, K]^T cut along K?
+  m.def("gemm2_grads_joint", [](int64_t t, int64_t n, int64_t k) { return prl_gemm2_grads_joint(t, n, k) != 0; });
+  m.def("gemm2_is_cut", [](int64_t m, int64_t n, int64_t k) { return prl_gemm2_ws_floats(m, n, k) != 0; });
   m.def("gemm2_bf16", &gemm2_bf16, py::arg("a"), py::arg("b"), py::arg("a_mn") = false, py::arg("b_mn") = false,
         py::arg("residual") = py::none(), py::arg("out") = py::none(), py::arg("force_bn") = 0);
   m.def("gemm2_accum_f32_", &gemm2_accum_f32_);

@@ -168,15 +168,49 @@ def test_linear_ce_edges(t, v, h, tau):
         assert (a.double() - b).norm() <= tol * b.norm()
 
 
+@pytest.mark.parametrize("t,v,h,chunk", [(100, 1304, 128, 256), (515, 1304, 896, 256), (515, 1000, 896, 128), (150, 40008, 64, None), (6200, 17000, 64, None)])
+@pytest.mark.parametrize("frozen", ["", "x", "w"])
+def test_linear_ce_slices(t, v, h, chunk, frozen, monkeypatch):
+    """Several slices of the vocabulary in the backward pass: labels at their edges, a ragged last one, gradients of both operands or of one,
+    in one launch (515 rows) or two; the usual slices and, for short rows, shorter ones.  Bounds as above."""
+    if chunk is not None:
+        monkeypatch.setattr(OF, "_CE_CHUNK", chunk)
+    step = OF._ce_slice(t)
+    assert v > step
+    x, w = _randn(t, h, seed=1), _randn(v, h, seed=2, scale=0.1)
+    edges = [e for lo in range(0, v, step) for e in (lo, lo + 1, lo - 1) if 0 <= e < v] + [v - 1]
+    lab = torch.tensor([edges[i % len(edges)] for i in range(t)]).cuda()
+    glp, gent = _randn(t, seed=3, dtype=torch.float32), _randn(t, seed=4, dtype=torch.float32)
+
+    def grads(leaves, f, g):
+        keep = [p.requires_grad_(n != frozen) for p, n in zip(leaves, "xw")]
+        out = f(*keep)
+        return [*out, *torch.autograd.grad(out, [p for p in keep if p.requires_grad], g)]
+
+    def plain(x64, w64):
+        logp = (x64 @ w64.t() / 0.7).log_softmax(-1)
+        return logp.gather(1, lab[:, None])[:, 0], -(logp.exp() * logp).sum(-1)
+
+    want = grads([x.double(), w.double()], plain, [glp.double(), gent.double()])
+    before = ops.LAUNCHES.get("gemm2_grads", 0)
+    got = grads([x, w], lambda a, b: ops.linear_cross_entropy(a, b, lab, 0.7), [glp, gent])
+    assert ops.LAUNCHES.get("gemm2_grads", 0) - before == (-(-v // step) if not frozen else 0)
+    for a, b, tol in zip(got, want, (1e-5, 1e-5, 1e-2, 1e-2)):
+        assert (a.double() - b).norm() <= tol * b.norm()
+
+
 @pytest.mark.parametrize("m,n,k", [(300, 520, 8200), (257, 264, 4104), (2048, 2560, 16384), (129, 2816, 6000)])
 def test_gemm_cut_along_the_reduction(m, n, k):
     """Products whose last round of tiles is cut: all layouts, residual, fp32 accumulation, gate / up.  One rounding to bf16; the fp32 sums
     are k / 16 additions, each at most 2^-23 off."""
+    from polyrl_b200 import _C
     from polyrl_b200.ops import ext
 
     C = ext()
     a, b = _randn(m, k, seed=1), _randn(n, k, seed=2, scale=0.05)
     m8 = m // 8 * 8
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert _C.gemm2_is_cut(m, n, k) and _C.gemm2_is_cut(m8, n, k) and _C.gemm2_is_cut(m, n // 256 * 256, k)
     want = a.double() @ b.double().t()
 
     def close(got, ref):
@@ -306,17 +340,23 @@ def test_attention_keeps_sequences_apart(d, lq, lk, causal, bad):
         assert all(torch.equal(a, b) and not torch.isnan(a).any() for a, b in zip(got[i], want[i])), i
 
 
-@pytest.mark.parametrize("t,n,k", [(8, 136, 136), (387, 1152, 896), (300, 4096, 520), (2503, 2048, 896), (520, 200, 2056), (1030, 6144, 1000)])
-def test_gemm2_grads(t, n, k):
-    """Input and weight gradient of a linear layer in one launch: bf16 and accumulating fp32 input gradient, results of the separate
-    products bit for bit where those sum whole tiles, ragged edges in every dimension."""
+@pytest.mark.parametrize("t,n,k,joint", [(8, 136, 136, True), (387, 1152, 896, True), (300, 4096, 520, False), (2503, 2048, 896, True), (520, 200, 2056, True),
+                                         (1030, 6144, 1000, True), (515, 392, 896, True)])
+def test_gemm2_grads(t, n, k, joint):
+    """Input and weight gradient of a linear layer, in one launch where the plan says so (148 SMs): bf16 and accumulating fp32 input gradient,
+    results of the separate products bit for bit where those sum whole tiles, ragged edges in every dimension."""
+    from polyrl_b200 import _C
     from polyrl_b200.ops import ext
 
     C = ext()
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert _C.gemm2_grads_joint(t, n, k) == joint
     dy, w, x = _randn(t, n, seed=1), _randn(n, k, seed=2, scale=0.05), _randn(t, k, seed=3)
     dx, dw = C.gemm2_grads(dy, w, x)
-    for got, want in ((dx, dy.double() @ w.double()), (dw, dy.double().t() @ x.double())):
+    apart = C.gemm2_bf16(dy, w, False, True, None, None, 0), C.gemm2_bf16(dy, x, True, True, None, None, 0)
+    for got, want, one, cut in ((dx, dy.double() @ w.double(), apart[0], _C.gemm2_is_cut(t, k, n)), (dw, dy.double().t() @ x.double(), apart[1], _C.gemm2_is_cut(n, k, t))):
         assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4 * want.abs().max()).all()
+        assert cut or torch.equal(got, one)
     acc = _randn(t, k, seed=4, dtype=torch.float32)
     ref = acc.double() + dy.double() @ w.double()
     out = torch.empty(n + 8, k + 8, device="cuda", dtype=torch.bfloat16)[8:, 8:]
