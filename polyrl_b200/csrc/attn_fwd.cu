@@ -60,7 +60,6 @@ struct AttnFwdParams {
   const float* lam;            // two maps: [1] weight of the second
   float keep, eps;             // two maps: factor behind the norm, and what is added under its root
   int dv_out, shared_row;      // two maps: values of a head that are written (<= DV); both maps' keys in one row
-  long long* dbg;              // optional timeline buffer (kernel experiments)
 };
 
 template <int DK, int kAfD, int MAPS>
@@ -213,9 +212,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
     for (int i = 0; i < OW; ++i) O[i] = 0.f;
     const uint32_t sP0_u32 = smem_u32(sP) + g * 16384 + r * 128;
-    const bool rec = p.dbg != nullptr && blockIdx.x == gridDim.x / 2 && blockIdx.y == 0 && threadIdx.x == 64;
-    long long* dbg = p.dbg;
-    if (rec) dbg[0] = clock64();
     auto store = [&](__nv_bfloat16* dst, float f) {
 #pragma unroll
       for (int c = 0; c < OW; c += 8) {
@@ -247,7 +243,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const int s = j & 1;
       mbar_wait(&s_full[s], (j >> 1) & 1);
       tc_fence_after();
-      if (rec && j < 30) dbg[1 + 5 * j] = clock64();
       const uint32_t tS = tS0 + s * 128 + lane_base + g * 64;
       const int base = tile_of(j - map * nt) * kAfBN, col0 = base + g * 64;
       const bool need_mask = (base + kAfBN - 1 > kmax) || (base + kAfBN > lk) || base <= klo;
@@ -274,7 +269,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       s_mx[j & 1][g][r] = mx;
       asm volatile("bar.sync 1, 256;" ::: "memory");
       mx = fmaxf(mx, s_mx[j & 1][g ^ 1][r]);
-      if (rec && j < 30) dbg[2 + 5 * j] = clock64();
       const float m_new = fmaxf(m_run, mx);
       const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
       const float alpha = (m_run == -INFINITY) ? 0.f : fast_exp2((m_run - m_use) * p.scale_log2);
@@ -313,21 +307,18 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                        : "memory");
         }
       }
-      if (rec && j < 30) dbg[3 + 5 * j] = clock64();
       fence_proxy_async();
       tc_fence_before();
       mbar_arrive(p_full(j));
       mbar_arrive(&s_empty[s]);
       l_run = l_run * alpha + lsum;
       m_run = m_new;
-      if (rec && j < 30) dbg[4 + 5 * j] = clock64();
       if constexpr (PST == 2) {
         if (j > map * nt) take(j - 1, alpha_before);
         alpha_before = alpha;
       } else {
         take(j, alpha);
       }
-      if (rec && j < 30) dbg[5 + 5 * j] = clock64();
     }
     if constexpr (PST == 2) take((map + 1) * nt - 1, alpha_before);
     // total row sum = the two groups' partial sums (same running max on both sides)
@@ -729,7 +720,7 @@ static int run_attn_rows(const void* q, const void* k, const void* v, const Attn
 // sink: fp32 [nq] or null.
 extern "C" int prl_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse, const int32_t* cu_q,
                             const int32_t* cu_k, int B, int Tq, int Tk, int nq, int nkv, int dk, int dv, int64_t ldq, int64_t ldk, int64_t ldv,
-                            int64_t ldo, float sm_scale, int causal, int max_tiles, const float* sink, int window, int keep_first, long long* dbg,
+                            int64_t ldo, float sm_scale, int causal, int max_tiles, const float* sink, int window, int keep_first,
                             cudaStream_t stream) {
   if (Tq <= 0 || B <= 0) return 0;
   if (nq % nkv != 0) return -110;
@@ -745,7 +736,6 @@ extern "C" int prl_attn_fwd(const void* q, const void* k, const void* v, void* o
   p.window = window > 0 ? min(window, kNoWindow) : kNoWindow;
   p.keep_first = window > 0 ? keep_first : 0;
   p.sink = sink;
-  p.dbg = dbg;
   if (dk == 64 && dv == 64) return run_attn_rows<64, 64>(q, k, v, p, Tk, ldq, ldk, ldv, max_tiles, stream);
   if (dk == 64 && dv == 128) return run_attn_rows<64, 128>(q, k, v, p, Tk, ldq, ldk, ldv, max_tiles, stream);
   if (dk == 128 && dv == 64) return run_attn_rows<128, 64>(q, k, v, p, Tk, ldq, ldk, ldv, max_tiles, stream);

@@ -8,7 +8,7 @@
 #include <vector>
 
 extern "C" {
-int prl_gemm2_bf16(const void*, const void*, void*, const void*, int, int, int, int64_t, int64_t, int64_t, int64_t, int, int, int, float*, cudaStream_t);
+int prl_gemm2_bf16(const void*, const void*, void*, const void*, int, int, int, int64_t, int64_t, int64_t, int, int, int, float*, cudaStream_t);
 int64_t prl_gemm2_ws_floats(int, int, int);
 int prl_gemm2_grads_joint(int, int, int);
 int prl_gemm2_grads(const void*, const void*, const void*, void*, float*, float, void*, int, int, int, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, cudaStream_t);
@@ -106,7 +106,7 @@ at::Tensor gemm2_bf16(const at::Tensor& a, const at::Tensor& b, bool a_mn, bool 
   }
   TORCH_CHECK(a.stride(0) >= a.size(1) && b.stride(0) >= b.size(1), "gemm2_bf16: row pitch shorter than the row");
   const at::Tensor ws = split_scratch(prl_gemm2_ws_floats(M, N, K), a);
-  const int rc = prl_gemm2_bf16(a.data_ptr(), b.data_ptr(), d.data_ptr(), r, M, N, K, a.stride(0), b.stride(0), d.stride(0), d.stride(0),
+  const int rc = prl_gemm2_bf16(a.data_ptr(), b.data_ptr(), d.data_ptr(), r, M, N, K, a.stride(0), b.stride(0), d.stride(0),
                                 a_mn ? 1 : 0, b_mn ? 1 : 0, static_cast<int>(force_bn), split_ptr(ws), cur_stream());
   TORCH_CHECK(rc == 0, "polyrl_b200 kernel 'gemm2_bf16' failed with code ", rc, " (M=", M, " N=", N, " K=", K, " a_mn=", a_mn,
               " b_mn=", b_mn, " lda=", a.stride(0), " ldb=", b.stride(0), " ldd=", d.stride(0), " a=", a.data_ptr(), " b=",

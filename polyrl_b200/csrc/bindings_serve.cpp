@@ -6,11 +6,11 @@
 #include "scheduler.hpp"
 
 extern "C" {
-int prl_gemm_bf16(const void*, const void*, void*, const void*, int, int, int, int64_t, int64_t, int64_t, int64_t, int, float*, cudaStream_t);
+int prl_gemm_bf16(const void*, const void*, void*, const void*, int, int, int, int64_t, int64_t, int64_t, int, float*, cudaStream_t);
 int64_t prl_gemm2_ws_floats(int, int, int);
 int prl_sample(const void*, int, int64_t, int, int, const float*, int, const uint64_t*, int, int64_t*, float*, cudaStream_t);
 int prl_sample_topk_topp(const void*, int, int64_t, int, int, const float*, int, const uint64_t*, int, int, float, int64_t*, float*, cudaStream_t);
-int prl_attn_fwd(const void*, const void*, const void*, void*, float*, const int32_t*, const int32_t*, int, int, int, int, int, int, int, int64_t, int64_t, int64_t, int64_t, float, int, int, const float*, int, int, long long*, cudaStream_t);
+int prl_attn_fwd(const void*, const void*, const void*, void*, float*, const int32_t*, const int32_t*, int, int, int, int, int, int, int, int64_t, int64_t, int64_t, int64_t, float, int, int, const float*, int, int, cudaStream_t);
 int prl_paged_decode_workspace_floats(int, int, int, int);
 int prl_paged_decode(const void*, int64_t, const void*, const void*, const int32_t*, int64_t, const int32_t*, int, int, int, int, float, int, int, int, float*, void*, int64_t, cudaStream_t);
 int prl_gemm_clamped_glu_bf16(const void*, const void*, void*, int, int, int, int64_t, int64_t, int64_t, float, float, cudaStream_t);
@@ -90,7 +90,7 @@ at::Tensor gemm_bf16(const at::Tensor& a, const at::Tensor& b, const c10::option
     r = residual->data_ptr();
   }
   const at::Tensor ws = split_scratch(M > 128 && force_bn == 0 ? prl_gemm2_ws_floats(M, N, K) : 0, a);
-  check(prl_gemm_bf16(a.data_ptr(), b.data_ptr(), d.data_ptr(), r, M, N, K, a.stride(0), b.stride(0), d.stride(0), d.stride(0),
+  check(prl_gemm_bf16(a.data_ptr(), b.data_ptr(), d.data_ptr(), r, M, N, K, a.stride(0), b.stride(0), d.stride(0),
                       static_cast<int>(force_bn), split_ptr(ws), cur_stream()), "gemm_bf16");
   return d;
 }
@@ -139,7 +139,7 @@ std::vector<at::Tensor> sample_topk_topp(const at::Tensor& logits, const c10::op
 
 std::vector<at::Tensor> attn_fwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& cu_q,
                                  const at::Tensor& cu_k, double sm_scale, bool causal, bool want_lse,
-                                 const c10::optional<at::Tensor>& dbg, const c10::optional<at::Tensor>& sink, int64_t window, int64_t keep_first) {
+                                 const c10::optional<at::Tensor>& sink, int64_t window, int64_t keep_first) {
   CHECK_BF16(q); CHECK_BF16(k); CHECK_BF16(v);
   const int64_t dk = q.size(-1), dv = v.size(-1);
   TORCH_CHECK(q.dim() == 3 && k.dim() == 3 && v.dim() == 3 && (dk == 64 || dk == 128 || dk == 192) && k.size(2) == dk && (dv == 128 || (dv == 64 && dk != 192)) &&
@@ -160,8 +160,7 @@ std::vector<at::Tensor> attn_fwd(const at::Tensor& q, const at::Tensor& k, const
   check(prl_attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), want_lse ? lse.data_ptr<float>() : nullptr,
                      cu_q.data_ptr<int>(), cu_k.data_ptr<int>(), B, Tq, Tk, nq, nkv, static_cast<int>(dk), static_cast<int>(dv), q.stride(0), k.stride(0), v.stride(0),
                      static_cast<int64_t>(nq) * dv, static_cast<float>(sm_scale), causal ? 1 : 0, Tq / 128 + B,
-                     sink.has_value() ? sink->data_ptr<float>() : nullptr, static_cast<int>(window), static_cast<int>(keep_first),
-                     dbg.has_value() ? reinterpret_cast<long long*>(dbg->data_ptr<int64_t>()) : nullptr, cur_stream()),
+                     sink.has_value() ? sink->data_ptr<float>() : nullptr, static_cast<int>(window), static_cast<int>(keep_first), cur_stream()),
         "attn_fwd");
   if (want_lse) return {o, lse};
   return {o};
@@ -1029,7 +1028,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_bf16", &gemm_bf16, py::arg("a"), py::arg("b"), py::arg("residual") = py::none(),
         py::arg("out") = py::none(), py::arg("force_bn") = 0);
   m.def("attn_fwd", &attn_fwd, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("cu_q"), py::arg("cu_k"), py::arg("sm_scale"),
-        py::arg("causal") = true, py::arg("want_lse") = true, py::arg("dbg") = py::none(), py::arg("sink") = py::none(), py::arg("window") = 0,
+        py::arg("causal") = true, py::arg("want_lse") = true, py::arg("sink") = py::none(), py::arg("window") = 0,
         py::arg("keep_first") = 0);
   m.def("paged_decode", &paged_decode, py::arg("q"), py::arg("k_cache"), py::arg("v_cache"), py::arg("block_table"),
         py::arg("seq_lens"), py::arg("nq"), py::arg("nkv"), py::arg("d"), py::arg("sm_scale"), py::arg("splits") = 1,

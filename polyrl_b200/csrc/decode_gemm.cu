@@ -4,7 +4,7 @@
 // tensor work is 37 % of peak at HBM speed and a 128x128x16 SS-mode `tcgen05.mma` costs ~140 clk whatever
 // the batch (the A-operand read from shared memory is exposed), so one SM can turn at most ~29 B/clk of
 // weights into MMAs while HBM delivers ~23 B/clk per SM.  A kernel that leaves SMs idle is therefore MMA
-// bound, not memory bound (round 1's 112-CTA gate/up kernel: 54 us against a 36 us HBM floor), and the
+// bound, not memory bound (a 112-CTA gate/up kernel: 54 us against a 36 us HBM floor), and the
 // activation multicast tried first changed nothing.  The design follows from that:
 //
 //   * swap-AB: UMMA M = 128 weight rows, UMMA N = padded batch; every CTA streams its own weight panel
@@ -20,7 +20,7 @@
 //     chunk back from shared memory.
 //   * epilogue: + bias | + residual | fp8 row/col scales | SwiGLU, 16-byte coalesced bf16 stores.
 //
-// Replaces the cuBLAS / sgl-kernel decode GEMMs of the reference stack (SURVEY §2.5b "Decode GEMMs";
+// Replaces the cuBLAS / sgl-kernel decode GEMMs of the reference stack (
 // 3rdparty/verl/verl/workers/rollout/sglang_rollout/sglang_rollout.py drives SGLang's library kernels).
 #include <cuda_runtime.h>
 #include <stdlib.h>
@@ -39,7 +39,7 @@ struct StreamParams {
   const float* x_scale;        // optional fp8: per batch row
   const float* w_scale;        // optional fp8: per weight row
   int64_t ldo;
-  int B, N, K, BP, S, kb_per_split, swiglu, tiles, dbg, nacc, pf;
+  int B, N, K, BP, S, kb_per_split, swiglu, tiles, nacc, pf;
 };
 
 __device__ __forceinline__ void st_shared_cluster_f32(uint32_t addr, float v) {
@@ -140,7 +140,6 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         tma_prefetch_l2_2d(&tmW, kb * BLOCK_K, row_u);
       }
       for (int kb = kb0; kb < kb1; ++kb) {
-        if ((p.dbg & 2) && kb - kb0 >= stages) break;              // experiment: MMA-only (ring loaded once)
         if (kb + pf < kb1) {
           tma_prefetch_l2_2d(&tmW, (kb + pf) * BLOCK_K, row_g);
           tma_prefetch_l2_2d(&tmW, (kb + pf) * BLOCK_K, row_u);
@@ -168,13 +167,8 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       const uint32_t idesc = FP8 ? umma_idesc(128 * NC, p.BP, 0, 0) : umma_idesc(128 * NC, p.BP, 1, 1);
       int stage = 0; uint32_t phase = 0;
       for (int kb = 0; kb < nkb; ++kb) {
-        if (!((p.dbg & 2) && kb >= stages)) mbar_wait(&full_bar[stage], phase);
+        mbar_wait(&full_bar[stage], phase);
         tc_fence_after();
-        if (!PAIR && (p.dbg & 1)) {                                // experiment: stream-only (no MMA)
-          mbar_arrive(&empty_bar[stage]);
-          if (++stage == stages) { stage = 0; phase ^= 1; }
-          continue;
-        }
         const uint64_t da = umma_desc_sw128_kmajor(smem_a + stage * A_BYTES);
         const uint64_t db = umma_desc_sw128_kmajor(smem_b + stage * b_bytes);
 #pragma unroll
@@ -189,11 +183,10 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
           }
         }
         if constexpr (PAIR) umma_commit_2sm(&empty_bar[stage], pair_mask);
-        else if (!(p.dbg & 2)) umma_commit(&empty_bar[stage]);
+        else umma_commit(&empty_bar[stage]);
         if (++stage == stages) { stage = 0; phase ^= 1; }
       }
       if constexpr (PAIR) umma_commit_2sm(acc_bar, pair_mask);
-      else if (p.dbg & 1) mbar_arrive(acc_bar);
       else umma_commit(acc_bar);
     }
   }
@@ -383,10 +376,6 @@ extern "C" int prl_stream_gemm(const void* X, const void* W, void* out, const vo
                                int dtype, int splits, int pair, cudaStream_t stream) {
   if (B <= 0 || B > 256) return -60;
   StreamParams p;
-  {
-    const char* e = getenv("PRL_STREAM_DBG");                       // kernel experiments only (scripts/dbg_stream_gemm.py)
-    p.dbg = e ? atoi(e) : 0;
-  }
   p.out = static_cast<__nv_bfloat16*>(out);
   p.res = static_cast<const __nv_bfloat16*>(res);
   p.bias = static_cast<const __nv_bfloat16*>(bias);

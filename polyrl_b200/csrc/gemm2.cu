@@ -8,9 +8,9 @@ namespace prl {
 
 template <int BN, bool A_MN, bool B_MN>
 static int run2(const void* A, const void* B, void* D, const void* R, int M, int N, int K, int64_t lda, int64_t ldb,
-                int64_t ldd, int64_t ldr, float* ws, cudaStream_t s) {
+                int64_t ldd, float* ws, cudaStream_t s) {
   using Cfg = Gemm2Cfg<BN, A_MN, B_MN, true>;
-  TmaStoreParams ep{static_cast<const __nv_bfloat16*>(R), ldr, static_cast<__nv_bfloat16*>(D), ldd};
+  TmaStoreParams ep{static_cast<const __nv_bfloat16*>(R), ldd, static_cast<__nv_bfloat16*>(D)};
   return launch_gemm2<Cfg, EpiTmaStore>(A, B, D, M, N, K, lda * 2, ldb * 2, ldd * 2, ep, 0, s, Sched{0, 1, 0}, ws);
 }
 
@@ -80,15 +80,15 @@ using namespace prl;
 // D[M,N] = sum_k A(m,k) B(n,k) (+R).  Pitches in ELEMENTS.
 //   a_mn = 0: A is [M,K] row-major;  a_mn = 1: A is [K,M] row-major (MN-major operand)
 //   b_mn = 0: B is [N,K] row-major;  b_mn = 1: B is [K,N] row-major
-// ldr: pitch of R, 0 for one row that is added to all (a bias).  ws: prl_gemm2_ws_floats(M, N, K) floats of scratch, or null.
+// R has the pitch of D.  ws: prl_gemm2_ws_floats(M, N, K) floats of scratch, or null.
 extern "C" int64_t prl_gemm2_ws_floats(int M, int N, int K) {
   return M > 0 && N > 128 && K > 0 ? plan_k_split(M, N, K).workers * 2ll * 256 * 256 : 0;
 }
 extern "C" int prl_gemm2_bf16(const void* A, const void* B, void* D, const void* R, int M, int N, int K, int64_t lda,
-                              int64_t ldb, int64_t ldd, int64_t ldr, int a_mn, int b_mn, int force_bn, float* ws, cudaStream_t stream) {
+                              int64_t ldb, int64_t ldd, int a_mn, int b_mn, int force_bn, float* ws, cudaStream_t stream) {
   const int bn = force_bn > 0 ? force_bn : pick_bn2(M, N);
   if (bn != 128 && bn != 256) return -10;
-#define PRL_G2(BN_, AM_, BM_) return run2<BN_, AM_, BM_>(A, B, D, R, M, N, K, lda, ldb, ldd, ldr, ws, stream)
+#define PRL_G2(BN_, AM_, BM_) return run2<BN_, AM_, BM_>(A, B, D, R, M, N, K, lda, ldb, ldd, ws, stream)
   if (bn == 256) {
     if (!a_mn && !b_mn) PRL_G2(256, false, false);
     if (!a_mn && b_mn) PRL_G2(256, false, true);

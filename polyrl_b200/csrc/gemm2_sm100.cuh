@@ -61,10 +61,9 @@ struct Gemm2Cfg {
 
 // TMA-store epilogue tag (handled inside the kernel, not a per-row functor).
 struct TmaStoreParams {
-  const __nv_bfloat16* R;   // optional residual [M, ldr]; ldr = 0: one row for all, a bias
-  int64_t ldr;
+  const __nv_bfloat16* R;              // optional residual, pitch as D
+  int64_t ldd;
   __nv_bfloat16* D = nullptr;          // the matrix that the TMA stores write, for tiles that are finished from their slots
-  int64_t ldd = 0;
 };
 struct EpiTmaStore {
   using Params = TmaStoreParams;
@@ -76,7 +75,7 @@ struct EpiTmaStore {
     if (col >= N) return;
     float4 t = sum(c);
     if (p.R != nullptr) {
-      const uint2 q = *reinterpret_cast<const uint2*>(p.R + static_cast<int64_t>(row) * p.ldr + col);
+      const uint2 q = *reinterpret_cast<const uint2*>(p.R + static_cast<int64_t>(row) * p.ldd + col);
       const float2 a = unpack_bf16(q.x), b = unpack_bf16(q.y);
       t.x += a.x; t.y += a.y; t.z += b.x; t.w += b.y;
     }
@@ -304,7 +303,7 @@ gemm2_sm100_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
               epi.apply(ep, r, col0);
             } else {
             if (ep.R != nullptr && row < M) {
-              const __nv_bfloat16* rp = ep.R + static_cast<int64_t>(row) * ep.ldr + col0;
+              const __nv_bfloat16* rp = ep.R + static_cast<int64_t>(row) * ep.ldd + col0;
 #pragma unroll
               for (int j = 0; j < 8; ++j) {
                 if (col0 + 8 * j < N) {

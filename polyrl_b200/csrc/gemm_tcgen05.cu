@@ -227,14 +227,13 @@ static int pick_bn(int M, int N) {
 using namespace prl;
 
 // D = A·B^T (+R).  A:[M,K] B:[N,K] bf16 row-major with pitches lda/ldb/ldd in ELEMENTS.
-extern "C" int prl_gemm2_bf16(const void*, const void*, void*, const void*, int, int, int, int64_t, int64_t, int64_t, int64_t, int, int,
+extern "C" int prl_gemm2_bf16(const void*, const void*, void*, const void*, int, int, int, int64_t, int64_t, int64_t, int, int,
                               int, float*, cudaStream_t);
 
 extern "C" int prl_gemm_bf16(const void* A, const void* B, void* D, const void* R, int M, int N, int K, int64_t lda,
-                             int64_t ldb, int64_t ldd, int64_t ldr, int force_bn, float* ws, cudaStream_t stream) {
+                             int64_t ldb, int64_t ldd, int force_bn, float* ws, cudaStream_t stream) {
   // more than one 128-row block of tokens: the CTA-pair kernel (256-row tiles, cta_group::2) is the faster mainloop
-  if (M > kBlockM && N > 128 && force_bn == 0) return prl_gemm2_bf16(A, B, D, R, M, N, K, lda, ldb, ldd, ldr, 0, 0, 0, ws, stream);
-  if (R != nullptr && ldr != ldd) return -14;          // a bias is the pair kernel's
+  if (M > kBlockM && N > 128 && force_bn == 0) return prl_gemm2_bf16(A, B, D, R, M, N, K, lda, ldb, ldd, 0, 0, 0, ws, stream);
   StoreParams sp{static_cast<__nv_bfloat16*>(D), static_cast<const __nv_bfloat16*>(R), ldd, nullptr, nullptr};
   const int bn = force_bn > 0 ? force_bn : pick_bn(M, N);
   switch (bn) {

@@ -623,7 +623,7 @@ def sink_varlen_ok(kw: int, vw: int) -> bool:
 def sink_attention_varlen(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_q: torch.Tensor, cu_k: torch.Tensor, scale: float,
                           sink: torch.Tensor | None) -> torch.Tensor:
     """Causal (bottom-right aligned) attention of packed spans, with a sink: the tcgen05 kernel, widths of ``sink_varlen_ok``, bf16."""
-    return _C().attn_fwd(q, k, v, cu_q, cu_k, scale, True, False, None, sink)[0]
+    return _C().attn_fwd(q, k, v, cu_q, cu_k, scale, True, False, sink)[0]
 
 
 # --------------------------------------------------------------------------------------------
@@ -695,7 +695,7 @@ def window_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor
 def window_attention_varlen(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_q: torch.Tensor, cu_k: torch.Tensor, scale: float, window: int,
                             keep_first: int) -> torch.Tensor:
     """Packed spans, bottom-right aligned: the tcgen05 kernel, width 64 or 128, bf16."""
-    return _C().attn_fwd(q, k, v, cu_q, cu_k, scale, True, False, None, None, window, keep_first)[0]
+    return _C().attn_fwd(q, k, v, cu_q, cu_k, scale, True, False, None, window, keep_first)[0]
 
 
 # --------------------------------------------------------------------------------------------
