@@ -70,8 +70,7 @@ def reference_arm(args) -> int:
     (python -m rlboost.verl_stream.trainer.main_stream) imports hydra / ray / omegaconf / tensordict / verl /
     sglang and spawns the Rust manager with `cargo run` — none of which exist on this image (no network)."""
     why = ("reference installs with --no-deps (baseline/_ref) but cannot run: its entry point needs ray, sglang==0.5.5, hydra-core, "
-           "omegaconf, tensordict, rpyc and a Rust toolchain (cargo run for the manager); none are installed/installable offline — "
-           "see baseline/install_attempt*.log, DESIGN.md section 5")
+           "omegaconf, tensordict, rpyc and a Rust toolchain (cargo run for the manager); none are installed/installable offline")
     if int(os.environ.get("RANK", 0)) == 0:
         print(json.dumps({"impl": "reference", "unavailable": why}), flush=True)
     return 0

@@ -1,4 +1,4 @@
-"""MoE decode on the GPU: engine log-probs of its own samples vs a full forward (run by scripts/gpu_round2_checks.sh, also with
+"""MoE decode on the GPU: engine log-probs of its own samples vs a full forward (also with
 POLYRL_MOE_STATIC_DECODE=1 = CUDA-graph decode over the static-shape expert path)."""
 import torch
 from polyrl_b200.models import transformer as tf
