@@ -7,7 +7,7 @@ PROCESSING_TOOLS / INTERACTING -> TERMINATED; request-level path of sglang_rollo
 scheduler owns every trajectory of the batch: finished turns are parsed on the host while the GPU keeps decoding
 the other sequences, tool calls run on a thread pool, and a trajectory re-enters the continuous batch as soon as
 its tool response is tokenised.  Tool / user tokens are part of ``responses`` with ``response_mask = 0`` (no loss,
-log-prob 0), exactly the layout the trainer expects (Appendix D of SURVEY.md).
+log-prob 0), exactly the layout the trainer expects.
 """
 from __future__ import annotations
 
@@ -338,7 +338,7 @@ class SingleTurnAgentLoop(MultiTurnRollout):
 
 def outputs_to_dataproto(outs: list[AgentLoopOutput], prompt_length: int, response_length: int, pad_id: int,
                          non_tensors: dict[str, Any] | None = None, model_cfg=None) -> DataProto:
-    """Left-pad prompts / right-pad responses into the trainer batch layout (keys of SURVEY.md Appendix D)."""
+    """Left-pad prompts / right-pad responses into the trainer batch layout."""
     b = len(outs)
     prompts = torch.full((b, prompt_length), pad_id, dtype=torch.long)
     p_mask = torch.zeros(b, prompt_length, dtype=torch.long)

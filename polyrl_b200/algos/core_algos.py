@@ -3,7 +3,7 @@ value loss and KL penalties.
 
 Capability parity with the reference's ``core_algos`` (3rdparty/verl/verl/trainer/ppo/core_algos.py:
 estimators :212-755, KL controllers :150-209, agg_loss :772-809, policy losses :887-1366, value loss
-:1370-1409, kl_penalty :1412-1473); formulas per SURVEY Appendix E.  Group statistics are vectorised
+:1370-1409, kl_penalty :1412-1473).  Group statistics are vectorised
 with ``torch.unique`` + ``index_add`` instead of per-sample Python dict loops.
 """
 from __future__ import annotations

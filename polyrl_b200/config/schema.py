@@ -1,4 +1,4 @@
-"""Typed configuration tree with the reference's key names (SURVEY §5.6), YAML loading and Hydra-style
+"""Typed configuration tree with the reference's key names, YAML loading and Hydra-style
 dotted overrides (``actor_rollout_ref.actor.optim.lr=1e-6``).  Hydra/OmegaConf are not available on the
 target image, so composition is implemented here: defaults from dataclasses < YAML file(s) < CLI
 overrides, then ``validate_config`` cross-field checks (reference: 3rdparty/verl/verl/utils/config.py:23-200,

@@ -11,7 +11,7 @@
 // gathered buffer is also what the backward pass re-uses (no second gather when it is kept).
 //
 // Baseline being replaced: torch FSDP all_gather_into_tensor + copy-out, then a cuBLAS GEMM
-// (3rdparty/verl/verl/workers/fsdp_workers.py:494-507; SURVEY §2.5c row 1).
+// (3rdparty/verl/verl/workers/fsdp_workers.py:494-507).
 #include "gemm_sm100.cuh"
 
 namespace prl {

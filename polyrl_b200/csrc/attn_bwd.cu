@@ -15,8 +15,9 @@
 // 64 KB a tile pair, had one stage of Q and dO and waited for each step in turn.
 // Both run one CTA an SM over many items: operands arrive through two stages, the next pair's scores are multiplied while the warps work
 // on this one, an item's first loads run under the end of the one before, and results leave through shared memory in whole 64-byte pieces.
-// 32 heads of 128 over 8, causal: 19 sequences of 647: 851 us before and after, 16 heads over 8, 9 sequences of 455: 132 -> 119 us a call; head
-// width 64 took a library (two 0.5B blocks, 387 tokens: 1870 -> 1365 us, most of it on the host).
+// 32 heads of 128 over 8, causal, 19 sequences of 647: as the one-kernel form when it was written, 637 us before and 623 with products that end
+// at the sequence's last row; 16 heads over 8, 9 sequences of 455: 132 -> 101 us a call; head width 64 took a library (two 0.5B blocks,
+// 387 tokens: 1870 -> 1365 us, most of it on the host).
 #include "common.cuh"
 
 namespace prl {

@@ -395,7 +395,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 //   warp 1  MMA issuer: S_n = Q K_n^T, then O += P_n V_n with P_n in TMEM, over the columns of S_n
 //   warps 2-5  softmax: thread = query row, so the row maximum and sum need no exchange; the 128 scores are read once and stay in
 //           registers; P goes back to TMEM as bf16
-// O stays in TMEM (fp32).  It is rescaled only when a row's maximum has grown by more than 2^8 since the last time: the probabilities
+// O stays in TMEM (fp32).  It is rescaled only when a row's maximum has grown by more than 2^8 since the last time (as published for the
+// Blackwell form of flash attention): the probabilities
 // are relative to that older maximum, at most 256, and lose nothing as bf16 and fp32 have the same exponent range.
 // A mask is one comparison an element with a place inside the tile, under a test that is the same for the whole tile (written as conditions
 // on keys and sequence lengths it took 4000 cycles a tile, twice the rest of the softmax).  Rows leave through shared memory, 64 bytes of

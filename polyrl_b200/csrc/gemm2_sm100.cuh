@@ -102,7 +102,7 @@ __device__ __forceinline__ float gelu_fast(float z) {
 }
 __device__ __forceinline__ float silu_fast(float z) { return __fdividef(z, 1.0f + __expf(fminf(-z, 80.f))); }
 
-// The last round of tiles, cut along the reduction.  `full` tiles go to the pairs whole; the k-blocks of the remaining `tiles` are dealt
+// The last round of tiles, cut along the reduction (as in "stream-K" decompositions).  `full` tiles go to the pairs whole; the k-blocks of the remaining `tiles` are dealt
 // out evenly, in order, to `workers` pairs, each of which takes a run of k-blocks of one tile or of the end of one and the start of the
 // next, and leaves its fp32 sums in a slot of `ws`.  split_finish_kernel adds a tile's slots in order and applies the epilogue.
 struct KSplit {

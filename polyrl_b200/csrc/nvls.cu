@@ -1,8 +1,7 @@
 // polyrl_b200 — NVLS: symmetric heap on the CUDA VMM API with an NVSwitch MULTICAST mapping, and the
 // `multimem.*` collectives that reduce inside the switch.
 //
-// Round 1's symmetric heap was cudaMalloc + legacy CUDA IPC, which cannot back a multicast object
-// (SURVEY §5.8).  Here every rank creates its share with cuMemCreate (exportable as a POSIX
+// A symmetric heap of cudaMalloc + legacy CUDA IPC cannot back a multicast object.  Here every rank creates its share with cuMemCreate (exportable as a POSIX
 // file descriptor), maps every peer's share for plain ld/st (same capability as before) AND binds its
 // share to one multicast object whose mapping `mc` addresses "the same offset on every GPU":
 //   multimem.ld_reduce [mc + off]   -> the switch reads all N copies and returns their sum (fp32 accumulate)

@@ -10,7 +10,7 @@
 //  * all-gather pull:    each rank pulls every peer's shard (rollout weight sync / ZeRO-3 unshard)
 //  * reduce-scatter pull fused with fp32 accumulate + grad-norm partial: the owner of a shard sums the
 //                        peers' bf16 gradients straight out of their HBM into its fp32 accumulator —
-//                        replaces NCCL reduce_scatter + cast/scale + norm (SURVEY §2.5c)
+//                        replaces NCCL reduce_scatter + cast/scale + norm
 #include "common.cuh"
 
 namespace prl {

@@ -10,8 +10,8 @@
 //   weight accumulate in two TMEM buffers of the same CTA and are combined lane-wise).
 // Outputs are written transposed back to [B, N] row-major with 64-byte coalesced segments.
 //
-// This is the rollout engine's replacement for the cuBLAS / sgl-kernel decode GEMMs of the reference stack
-// (SURVEY §2.5b "Decode GEMMs"); measured against cuBLAS in profiles/.
+// This is the rollout engine's replacement for the cuBLAS / sgl-kernel decode GEMMs of the reference stack;
+// measured against cuBLAS in profiles/.
 #include "common.cuh"
 
 namespace prl {

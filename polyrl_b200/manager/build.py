@@ -2,7 +2,7 @@
 
 Binaries are never committed: they are built from ``manager/src`` on first use and cached under ``manager/bin/`` (git-ignored)
 next to a stamp holding the hash of the sources + flags that produced them, so a checkout with arbitrary mtimes can never run a
-stale or foreign ELF (ADVICE r1)."""
+stale or foreign ELF."""
 from __future__ import annotations
 
 import hashlib
@@ -24,7 +24,7 @@ def _digest(paths: list[Path], flags: list[str]) -> str:
 
 def build_manager(force: bool = False, sanitize: str | None = None) -> Path | None:
     """``sanitize`` in {None, "thread", "address", "undefined"}: instrumented builds land next to the release binary as
-    ``rollout-manager-<sanitizer>`` (the reference's Rust manager has no race tooling, SURVEY 5.2; tests/test_manager.py runs
+    ``rollout-manager-<sanitizer>`` (the reference's Rust manager has no race tooling; tests/test_manager.py runs
     the scheduler / continuation / fault-injection scenarios under ThreadSanitizer)."""
     srcs = sorted(SRC.glob("*.cpp"))
     if not srcs:

@@ -1,5 +1,5 @@
-"""In-process fake rollout engine speaking the SGLang-compatible HTTP surface the manager relies on
-(SURVEY Appendix B): ``/generate`` (SSE, cumulative chunks), ``/health_generate``, ``/get_server_info``,
+"""In-process fake rollout engine speaking the SGLang-compatible HTTP surface the manager relies on:
+``/generate`` (SSE, cumulative chunks), ``/health_generate``, ``/get_server_info``,
 ``/abort_request``, ``/shutdown``, ``/update_weights_from_agent``.  Deterministic "model": next token =
 (sum(input_ids so far) * 31 + 7) % vocab — so a continuation resumed on another engine must reproduce
 exactly the tokens an uninterrupted run would have produced.  Fault injection: ``die_after_tokens`` closes

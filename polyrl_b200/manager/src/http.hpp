@@ -48,7 +48,7 @@ inline bool send_all(int fd, const std::string& s) { return send_all(fd, s.data(
 
 // Bounded pool of worker threads with small stacks.  Threads are created lazily up to `max_threads` and never exceed it; work
 // beyond that queues.  Used for request handlers (bounded by --http-workers) and for the blocking per-request engine streams
-// (bounded by --max-inflight-requests) — the round-1 manager spawned one detached thread per request instead.
+// (bounded by --max-inflight-requests) instead of one detached thread per request.
 class WorkerPool {
  public:
   explicit WorkerPool(size_t max_threads, size_t stack_bytes = 512 * 1024) : max_(max_threads ? max_threads : 1), stack_(stack_bytes) {}

@@ -1,13 +1,13 @@
 // polyrl_b200 rollout manager — native C++ re-implementation of the reference's Rust/tokio/axum service
-// (rollout-manager/src/{main,state,handlers,instance_manager}.rs).  Same 13 REST routes and JSON schemas
-// (SURVEY Appendix A), same scheduling semantics:
+// (rollout-manager/src/{main,state,handlers,instance_manager}.rs).  Same 13 REST routes and JSON schemas,
+// same scheduling semantics:
 //   * per-stats-tick admission quota + round-robin among engines whose queue is empty, otherwise park
 //   * token-level fault-tolerant continuation: on stream failure / abort keep the partial generation, evict
 //     the (remote) engine, append the generated tokens to the prompt, shrink max_new_tokens, re-dispatch (<=5x)
 //   * time-boxed generation on colocated ("local") engines, then abort-all and continue remotely
 //   * weight-version protocol (update_weight_version / get_receive_instances CAS / update_weights activate)
 //   * load-balance controller fed by /update_metrics
-// Differences (documented in DESIGN.md): the local window ends early when every request already finished
+// Differences: the local window ends early when every request already finished
 // (reference always sleeps the whole budget; opt back in with wait_full_local_window=true).
 #include <signal.h>
 #include <unistd.h>

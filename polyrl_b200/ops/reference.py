@@ -1,8 +1,8 @@
 """Plain-PyTorch reference implementations of every fused op (fp32 math).
 
 Used (a) as the CPU execution path so the whole framework runs under gloo without a GPU, and (b) as
-the numerical oracle for the sm_100a kernels in ``tests/``.  Math follows SURVEY Appendix E
-(reference: 3rdparty/verl/verl/utils/kernel/kernels.py:242-266,343-371,1237-1245).
+the numerical oracle for the sm_100a kernels in ``tests/``.  Math as in the reference
+( 3rdparty/verl/verl/utils/kernel/kernels.py:242-266,343-371,1237-1245).
 """
 from __future__ import annotations
 

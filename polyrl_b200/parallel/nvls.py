@@ -11,7 +11,7 @@ node.  If the driver / container has no multicast support the heap still works w
 the peer-pointer kernels.
 
 Reference: NVLS is reachable in the reference only through NCCL inside SGLang (``NCCL_NVLS_ENABLE``,
-3rdparty/verl/verl/workers/rollout/sglang_rollout/sglang_rollout.py:99); SURVEY §5.8 asks for the in-kernel form.
+3rdparty/verl/verl/workers/rollout/sglang_rollout/sglang_rollout.py:99); here kernels use it themselves.
 """
 from __future__ import annotations
 

@@ -1,7 +1,7 @@
 """Symmetric device heap over NVLink/NVSwitch: every rank allocates the same-sized buffer, exchanges CUDA
 IPC handles through the (gloo/NCCL) process group, and maps every peer's buffer, so kernels can issue
 plain ld/st (or TMA) on peer HBM.  This is the substrate for the in-kernel collectives (csrc/p2p.cu,
-csrc/ag_gemm.cu) that replace the reference's NCCL / TCP / shm paths (SURVEY §5.8).
+csrc/ag_gemm.cu) that replace the reference's NCCL / TCP / shm paths.
 
 Only ranks on one node (one NVSwitch domain) can share a heap; multi-node jobs fall back to NCCL.
 """

@@ -825,7 +825,7 @@ class Zero3Engine:
     def arm_norm_fold(self) -> None:
         """Call right before the LAST backward of a mini-batch: that micro-batch's reduce-scatter / accumulate kernels also
         accumulate sum(grad_acc^2) of the values they just produced, so ``step()`` needs no separate pass over the fp32
-        gradients (SURVEY 2.5b "grad clip: norm accumulated in RS kernel")."""
+        gradients."""
         if not (self.use_kernels and self.trainable) or self.replica_group is not None:
             return
         self.total_sumsq.zero_()

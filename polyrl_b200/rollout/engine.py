@@ -4,7 +4,7 @@ Replaces the patched SGLang server the reference launches per TP group
 (rlboost/verl_stream/workers/rollout/sglang_rollout/sglang_rollout_remote.py:103-182,
 rlboost/verl_stream/workers/rollout/sglang_rollout/sglang_http_async_engine.py:43-113).  The engine
 lives in the trainer process, so colocated weight hand-off is pointer aliasing (no CUDA-IPC
-serialisation, SURVEY §2.5c last rows) and ``release/resume_memory_occupation`` is dropping /
+serialisation) and ``release/resume_memory_occupation`` is dropping /
 re-creating the KV pool.
 
 Per step the scheduler either *prefills* newly admitted prompts (packed varlen forward that also fills
@@ -374,7 +374,7 @@ class RolloutEngine:
     @torch.no_grad()
     def _quantize_layers(self, layer_w: list[dict]) -> list[dict]:
         """bf16 -> (e4m3, row scale) for the four block projections; buffers are reused across syncs so captured decode
-        graphs stay valid (reference capability: fp8 rollout with bf16 update, BASELINE config 4)."""
+        graphs stay valid (reference capability: fp8 rollout with bf16 update)."""
         fresh = len(self._fp8_cache) != len(layer_w)
         if fresh:
             self._fp8_cache = [dict() for _ in layer_w]

@@ -1,5 +1,5 @@
 """HTTP front-end of the native rollout engine, wire-compatible with the SGLang endpoints the rollout
-manager and the reference trainer use (SURVEY Appendix B; reference patches:
+manager and the reference trainer use (reference patches:
 rlboost/sglang/patches.py:390-566, rlboost/verl_stream/workers/rollout/sglang_rollout/sglang_http_async_engine.py:155-299):
 
   POST /generate (stream => SSE ``data: {...}`` cumulative chunks, ``data: [DONE]``), GET /health_generate,

@@ -7,8 +7,8 @@ column-parallel (each rank owns nq/W query heads, nkv/W kv heads and F/W interme
 only holds its heads), O and down projections are row-parallel and need an all-reduce.  The reference stack
 issues that all-reduce as a separate NCCL / custom-all-reduce kernel after a cuBLAS GEMM; here the decode path
 uses ``skinny_gemm_tp``: the GEMM's epilogue pushes its partial tile into every peer's inbox with NVLink
-stores, signals per-tile flags and reduces in rank order — one kernel, no NCCL (SURVEY §2.5c "SGLang TP
-all-reduce x2 per layer per decode step").  Prefill (large M) uses the NCCL all-reduce.
+stores, signals per-tile flags and reduces in rank order — one kernel, no NCCL (the reference's SGLang
+all-reduces twice per layer per decode step).  Prefill (large M) uses the NCCL all-reduce.
 
 Lock-step: all TP ranks run identical engines on identical request streams with identical seeds; hidden states
 are bit-identical after the rank-ordered reduction, so sampling agrees without any host communication.  Rank 0

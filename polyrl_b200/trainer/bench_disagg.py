@@ -1,4 +1,4 @@
-"""``bench.py --mode disagg``: the flagship PolyRL deployment as a benchmark.
+"""``bench.py --mode disagg``: the flagship PolyRL deployment (Llama-3-8B PPO, half of the GPUs serve, half train) as a benchmark.
 
 N GPUs of one node, one process per GPU under torchrun: ranks [0, N/2) are ZeRO trainers, ranks [N/2, N) host native rollout
 engines (one TP engine of size min(4, N/2) per group) behind the C++ rollout manager that trainer rank 0 spawns.  Every step:

@@ -137,7 +137,7 @@ class StreamPPOTrainer:
         mini = a.actor.ppo_mini_batch_size * a.rollout.n
         b = list(range(mini, total + 1, mini))
         if not b or b[-1] != total:
-            b.append(total)           # clamp: the reference crashes when train_batch_size*n < mini (SURVEY App. E)
+            b.append(total)           # clamp: the reference crashes when train_batch_size*n < mini
         return b
 
     # ------------------------------------------------------------------ rollout stream

@@ -1,7 +1,7 @@
 """HBM planner: per-GPU memory of a colocated rollout + training job on 180 GB B200s and the layout decisions that follow
 (resident bf16 replica or per-layer gather, how many blocks keep their activations, whether optimizer state must be offloaded,
 KV-cache budget).  The same arithmetic drives ``Zero3Engine``'s ``resident`` / ``act_ckpt=auto`` choices at run time; this module
-makes it inspectable up front (Llama-3-70B PPO, TP-8 rollout / ZeRO-3 trainer, "8xB200 HBM sizing").
+makes it inspectable up front (for instance Llama-3-70B PPO on 8 GPUs: TP-8 rollout, ZeRO-3 trainer).
 
     python -m polyrl_b200.utils.hbm_sizing llama3-70b --gpus 8 --rollout-tp 8 --critic
 """

@@ -1,4 +1,4 @@
-"""Step metrics (names kept dashboard-compatible with the reference, SURVEY Appendix F):
+"""Step metrics (names kept dashboard-compatible with the reference):
 ``compute_data_metrics`` / ``compute_timing_metrics`` / ``compute_throughout_metrics`` / validation bootstrap
 (3rdparty/verl/verl/trainer/ppo/metric_utils.py:80-490) and ``reduce_metrics``."""
 from __future__ import annotations

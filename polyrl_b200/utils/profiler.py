@@ -1,5 +1,5 @@
 """Profiling hooks: torch.profiler / CUDA-profiler-API (nsys capture-range) / CUDA memory-history
-snapshots, NVTX-annotated timers.  Capability parity with verl's profiler package (SURVEY §5.1:
+snapshots, NVTX-annotated timers.  Capability parity with verl's profiler package (
 3rdparty/verl/verl/utils/profiler/{profile.py:26-371,nvtx_profile.py:85-200,performance.py:155-195})."""
 from __future__ import annotations
 
