@@ -1,5 +1,6 @@
-// polyrl_b200 — token sampling for the rollout engine: temperature + Gumbel-max categorical sampling (exact for top_k=-1 / top_p=1, the
-// GRPO default), top-k / top-p, or greedy, returning the token id AND its log-probability under the distribution that was sampled.
+// polyrl_b200 — token sampling for the rollout engine: temperature + Gumbel-max categorical sampling (noise of 24 bits an element; over the
+// whole row for top_k=-1 / top_p=1, the GRPO default), top-k / top-p, or greedy, returning the token id AND its log-probability under the
+// distribution that was sampled.
 //
 // Reference capability: SGLang sampler + `return_logprob` (meta_info.output_token_logprobs consumed at
 // rlboost/verl_stream/workers/rollout/sglang_rollout/sglang_rollout_remote.py:318-391).
