@@ -3,8 +3,8 @@
 // backward pass that emits d_logits for one vocab slice at a time.
 //
 // Capability parity: 3rdparty/verl/verl/utils/kernel/kernels.py:157-379 (Triton fwd mainloop +
-// epilogue) and :1124-1375 (d_logits split-N backward) / linear_cross_entropy.py:119.  Math per
-// SURVEY Appendix E: m = max z, S = sum exp(z-m), B = sum z·exp(z-m)/S, logprob = z_label - m - log S,
+// epilogue) and :1124-1375 (d_logits split-N backward) / linear_cross_entropy.py:119.
+// m = max z, S = sum exp(z-m), B = sum z·exp(z-m)/S, logprob = z_label - m - log S,
 // entropy = log S + m - B, z = h·W^T / tau.
 #include "gemm2_sm100.cuh"
 
@@ -213,7 +213,8 @@ using namespace prl;
 
 // How many runs of n-blocks a row's vocabulary is cut into: a run is one work item of an SM (pair), so with mb m-blocks the pass takes
 // ceil(mb runs / workers) rounds of ceil(nb / runs) tiles.  The cut with the fewest tiles in a row wins, the smaller one if equal.
-// (About two items a worker, whatever the remainder, left the last round nearly empty: 168 items on 74 pairs at 6005 x 128256, K 4096, 5540 us; now 144, 4170 us.)
+// About two items a worker, whatever the remainder, left the last round nearly empty: 168 items on 74 pairs at 6005 x 128256, K 4096, where
+// it is 144 now.  The whole call, with the two groups below: 5.88 -> 5.34 ms, both in turn.
 static int ce_runs(int T, int V) {
   const int mb = T > kBlockM ? (T + 255) / 256 : 1, nb = (V + 255) / 256;
   const int workers = T > kBlockM ? sm_count() / 2 : sm_count();

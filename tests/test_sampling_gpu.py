@@ -24,7 +24,7 @@ def _hash(x):
 
 def _noise(seed, row, v):
     n = _hash(_hash((torch.arange(v, device="cuda") + 0x9E3779B9 * (row + 1)) & 0xFFFFFFFF) ^ (seed & 0xFFFFFFFF))
-    u = ((_hash(n ^ (seed >> 32)) >> 8).float() + 0.5) * (1.0 / 16777216.0)
+    u = ((_hash(n ^ (seed >> 32)) >> 8).clamp(max=0xFFFFFE).float() + 0.5) * (1.0 / 16777216.0)      # (the last number would give u = 1)
     return -torch.log(-torch.log(u))
 
 
