@@ -107,6 +107,10 @@ def _is_decode_shape(x2: torch.Tensor, w: torch.Tensor) -> bool:
     return (not torch.is_grad_enabled() or not (x2.requires_grad or w.requires_grad)) and x2.shape[0] <= _SKINNY_MAX_ROWS
 
 
+def _stream_impl() -> bool:
+    return os.environ.get("POLYRL_DECODE_GEMM_IMPL", "stream") == "stream"
+
+
 def _streams(w: torch.Tensor) -> bool:
     """Weights as the stream kernel's tensor map takes them."""
     return w.dim() == 2 and w.stride(1) == 1 and w.stride(0) % 8 == 0 and w.data_ptr() % 16 == 0
@@ -119,21 +123,21 @@ def _use_skinny(x2: torch.Tensor, w: torch.Tensor) -> bool:
 
 
 def skinny_linear(x2: torch.Tensor, w: torch.Tensor, bias=None, residual=None, mode: int = 0, splits: int = 0) -> torch.Tensor:
-    """Own decode-shape GEMM: the round-2 stream GEMM (cluster split-K + DSMEM reduce-scatter, csrc/decode_gemm.cu); the round-1
+    """Own decode-shape GEMM: the stream GEMM (cluster split-K + DSMEM reduce-scatter, csrc/decode_gemm.cu); the older
     swap-AB kernel remains behind ``POLYRL_DECODE_GEMM_IMPL=skinny`` (it still backs the fused TP all-reduce epilogue)."""
     if x2.stride(-1) != 1 or x2.stride(0) % 8 != 0:
         x2 = x2.contiguous()
     if residual is not None and not residual.is_contiguous():
         residual = residual.contiguous()
     n_out = w.shape[0] // 2 if mode == 1 else w.shape[0]
-    if os.environ.get("POLYRL_DECODE_GEMM_IMPL", "stream") == "stream" and n_out % 8 == 0:
+    if _stream_impl() and n_out % 8 == 0:
         return _C().stream_gemm(x2, w, residual, bias, None, None, mode, splits, None, -1)
     ws, ctr = _skinny_buffers(x2.device)
     return _C().skinny_gemm(x2, w, residual, bias, None, None, ws, ctr, mode, splits)
 
 
 # --------------------------------------------------------------------------------------------
-# fp8 (e4m3, per-output-row scale) inference weights: rollout-side only (BASELINE config "fp8 rollout, bf16 update")
+# fp8 (e4m3, per-output-row scale) inference weights: rollout-side only (fp8 rollout, bf16 update)
 # --------------------------------------------------------------------------------------------
 class Fp8Weight:
     """``q`` [N, K] float8_e4m3fn + ``scale`` [N] fp32 (w ~= q * scale[:, None]).  Activations are quantised per token
@@ -175,7 +179,7 @@ def _linear_fp8(x: torch.Tensor, w: Fp8Weight, bias=None, residual=None, swiglu:
         if x.shape[0] <= _SKINNY_MAX_ROWS and n >= 128 and (not swiglu or n % 256 == 0):
             # stream GEMM: fp8 operands, fused scales / residual / SwiGLU, cluster split-K
             r = residual.contiguous() if residual is not None else None
-            if (n // 2 if swiglu else n) % 8 == 0 and os.environ.get("POLYRL_DECODE_GEMM_IMPL", "stream") == "stream":
+            if (n // 2 if swiglu else n) % 8 == 0 and _stream_impl():
                 return _C().stream_gemm(xq, w.q, r, bias, xs, w.scale, 1 if swiglu else 0, 0, None, 0)
             wsb, ctr = _skinny_buffers(x.device)
             return _C().skinny_gemm(xq, w.q, r, bias, xs, w.scale, wsb, ctr, 1 if swiglu else 0, 0)
@@ -294,10 +298,12 @@ def linear_swiglu(x: torch.Tensor, wgu: torch.Tensor) -> torch.Tensor:
         return skinny_linear(x, wgu, None, None, 1)
     if _is_kernel_tensor(x) and wgu.dtype == torch.bfloat16 and x.dim() == 2 and _decode_policy() == "auto" and not _cublas() \
             and _is_decode_shape(x, wgu) and 0 < x.shape[0] <= 128 and wgu.shape[0] <= 74 * 256 and wgu.shape[0] % 256 == 0 \
-            and x.shape[1] % 16 == 0 and x.data_ptr() % 16 == 0 and _streams(wgu):
+            and x.shape[1] % 16 == 0 and x.data_ptr() % 16 == 0 and _streams(wgu) and _stream_impl():
         # The tile kernel has one CTA per 256 weight rows: with fewer than half the SMs it cannot draw the weights fast enough.  The stream
-        # kernel splits the reduction over clusters.  [12288, 2048], 16 / 45 / 128 rows: 24.5 -> 16.5 / 18.1 / 23.5 us; at 256 rows, or
-        # with 28672 weight rows (112 CTAs: 53 against 60 us at 45 rows), the tile kernel is the faster one.
+        # kernel splits the reduction over clusters, while two of its CTAs fit the SMs for every 256 weight rows.  In a graph, tile and stream,
+        # 16 and 128 rows: [5632, 1024] 15.7 -> 7.2, 16.1 -> 12.0 us; [12288, 2048] 23.1 -> 15.6, 23.5 -> 23.1; [16384, 2560] 29.3 -> 19.1,
+        # 28.7 -> 26.2; [18944, 3584], the last one, 39.6 -> 25.9, 37.4 -> 34.3; [9728, 896] 15.7 -> 9.3, but 16.0 -> 17.0 at 128 rows.  Beyond
+        # the line it loses, [22016, 4096] 43.0 -> 54.1 and 43.9 -> 67.8; so it does at 256 rows.
         return skinny_linear(x, wgu, None, None, 1)
     if _is_kernel_tensor(x) and wgu.dtype == torch.bfloat16 and not _cublas():
         return _LinearSwigluFn.apply(x, wgu)
@@ -450,8 +456,10 @@ _CE_CHUNK = int(os.environ.get("POLYRL_CE_BWD_CHUNK", "16384"))
 
 def _ce_slice(rows: int) -> int:
     """Vocabulary columns whose logit gradients are held at a time.  Up to 6144 rows two of the usual slices together are no larger than one
-    is at 12288 rows (400 MB), and longer reductions and fewer launches win: [2503, 896] x 151936 forward and backward 2277 -> 2163 us; four
-    together lose it again (2409), as the two products of a slice no longer share the chip well."""
+    is at 12288 rows (400 MB), and longer reductions and fewer launches win.  Forward and backward with one and with two, 151936 x 896: 64 rows
+    730 and 469 us, 300 rows 864 and 631, 2503 rows 2426 and 2323, 6100 rows 6.22 and 5.61 ms; 128256 x 4096: 300 rows 1.71 and 1.66 ms, 2503
+    rows 8.84 and 8.56, 6100 rows 20.40 and 20.27; 151936 x 2048 at 6100 rows is the one size that loses, 12.32 and 12.36.  Four together were
+    slower than two at 2503 rows of 896, as the two products of a slice no longer share the chip well."""
     return _CE_CHUNK if rows > 6144 or "POLYRL_CE_BWD_CHUNK" in os.environ else 2 * _CE_CHUNK
 
 

@@ -420,6 +420,21 @@ def test_dense_block_gives_up_its_activations(model, monkeypatch):
     assert block <= chain + (1 << 20), (block, chain)
 
 
+@pytest.mark.parametrize("rows,impl,kernel", [(1, "stream", "stream_gemm"), (128, "stream", "stream_gemm"), (129, "stream", "gemm_swiglu"), (16, "skinny", "gemm_swiglu")])
+def test_gate_up_of_a_decode_step(rows, impl, kernel, monkeypatch):
+    """The stream kernel takes up to 128 rows where it is the chosen implementation, else the tile kernel; one rounding to bf16 of each
+    factor's fp32 sum of 512 products."""
+    monkeypatch.setenv("POLYRL_DECODE_GEMM_IMPL", impl)
+    x, w = _randn(rows, 512, seed=1), _randn(1024, 512, seed=2, scale=0.05)
+    before = ops.LAUNCHES.get(kernel, 0)
+    with torch.no_grad():
+        got = ops.linear_swiglu(x, w)
+    assert ops.LAUNCHES.get(kernel, 0) == before + 1
+    gu = (x.double() @ w.double().t()).view(rows, -1, 2, 128)
+    want = (torch.nn.functional.silu(gu[:, :, 0]) * gu[:, :, 1]).flatten(1)
+    assert ((got.double() - want).abs() <= 2.0 ** -7 * want.abs() + 1e-3).all()
+
+
 def test_decode_kernels_behind_each_other():
     """Kernels of a decode step may start while the one before still runs: a chain in which each reads what the last one wrote, its buffers
     freed and taken again on the way, gives the same values as with a wait after every kernel."""
